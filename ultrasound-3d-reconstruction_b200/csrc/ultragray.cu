@@ -61,7 +61,7 @@ struct Workspace {
                           //    sample, then (in place) its prefix along the ray
     float* t_far;         // P: product of the far factors of every instance settled at the sample
     float4* b_pos;        // P: backward: sample position, t
-    float4* b_coef;       // P: backward: dL/dT, T, dL/dnum, dL/dw (zero for skipped samples)
+    float4* b_coef;       // P: backward: dL/dT * T, dL/dnum, dL/dw, - (zero for skipped samples)
     float* b_suffix;      // P: backward: sum over the ray's samples y' >= y of dL/dT * T
     size_t bytes;
 };
@@ -537,6 +537,72 @@ far_prefix_kernel(int W, int H, const long long* __restrict__ header, const int*
     }
 }
 
+// What a (ray, Gaussian) pair of the checkpointed path needs per sample. The canonical point of
+// the ray at depth tc + u is xc + dg u (tc: the closest approach, xc the canonical point there),
+// so the profile of the transmission integral at a quadrature node is 2^((k2 u + k1) u + k0) and
+// the window's lower end is the constant 2 a0 = max(0, tc - wr) - tc: a sample costs three
+// 2-FMA polynomials instead of three canonical points. Working relative to tc also keeps the
+// digits that og + dg t loses when both terms are tens of canonical units.
+constexpr float kNegHalfLog2e = -0.72134752044448170f;  // -log2(e) / 2
+constexpr float kNegLog2e = -1.4426950408889634f;
+
+struct RayWindow {
+    float3 diff, is, xc, dg;  // ro - mu, 1/s, canonical closest point, canonical direction
+    float tc, a0, k2, k1, k0;
+};
+
+__device__ __forceinline__ RayWindow ray_window(const RayGeo& rg, const float3 mu, const float3 s, const float* R,
+                                                float wr) {
+    RayWindow w;
+    w.diff = v_sub(rg.o, mu);
+    w.is = make_float3(1.0f / s.x, 1.0f / s.y, 1.0f / s.z);
+    const float3 d = w.diff;
+    const float3 og = make_float3((R[0] * d.x + R[3] * d.y + R[6] * d.z) * w.is.x,
+                                  (R[1] * d.x + R[4] * d.y + R[7] * d.z) * w.is.y,
+                                  (R[2] * d.x + R[5] * d.y + R[8] * d.z) * w.is.z);
+    w.dg = make_float3((R[0] * rg.d.x + R[3] * rg.d.y + R[6] * rg.d.z) * w.is.x,
+                       (R[1] * rg.d.x + R[4] * rg.d.y + R[7] * rg.d.z) * w.is.y,
+                       (R[2] * rg.d.x + R[5] * rg.d.y + R[8] * rg.d.z) * w.is.z);
+    const float dg2 = v_dot(w.dg, w.dg);
+    w.tc = -v_dot(og, w.dg) / (dg2 + 1e-8f);
+    // xc through the world point of closest approach: the difference to mu is small there
+    const float3 c = v_add(d, v_mul(rg.d, w.tc));
+    w.xc = make_float3((R[0] * c.x + R[3] * c.y + R[6] * c.z) * w.is.x,
+                       (R[1] * c.x + R[4] * c.y + R[7] * c.z) * w.is.y,
+                       (R[2] * c.x + R[5] * c.y + R[8] * c.z) * w.is.z);
+    w.a0 = 0.5f * fmaxf(-w.tc, -wr);
+    w.k2 = kNegHalfLog2e * dg2;
+    w.k1 = 2.0f * kNegHalfLog2e * v_dot(w.xc, w.dg);
+    w.k0 = kNegHalfLog2e * v_dot(w.xc, w.xc);
+    return w;
+}
+
+// Quadrature of one sample at depth t (tc, a0, k2, k1, k0 of ray_window): node offsets u, profile
+// values f, half-width (0 when the window is empty), the integral.
+struct RayQuad {
+    float half, u0, u1, u2, f0, f1, f2, psi;
+};
+
+__device__ __forceinline__ RayQuad ray_quad(float t, float tc, float a0, float k2, float k1, float k0, float wr) {
+    RayQuad q;
+    const float a1 = fminf(t - tc, wr);
+    q.half = fmaxf(0.5f * a1 - a0, 0.0f);
+    q.u1 = 0.5f * a1 + a0;
+    q.u0 = q.half * -0.7745966692f + q.u1;
+    q.u2 = q.half * 0.7745966692f + q.u1;
+    q.f0 = exp2f((k2 * q.u0 + k1) * q.u0 + k0);
+    q.f1 = exp2f((k2 * q.u1 + k1) * q.u1 + k0);
+    q.f2 = exp2f((k2 * q.u2 + k1) * q.u2 + k0);
+    q.psi = q.half * (0.5555555556f * (q.f0 + q.f2) + 0.8888888889f * q.f1);
+    return q;
+}
+
+// Echo weight 2^(d^T P' d) with P' = -log2(e)/2 P, its off-diagonal entries doubled:
+// e = (P'00, P'01, P'02, P'11), f = (P'12, P'22).
+__device__ __forceinline__ float echo_weight(const float3 d, const float4 e, const float2 f) {
+    return exp2f((e.x * d.x + e.y * d.y + e.z * d.z) * d.x + (e.w * d.y + f.x * d.z) * d.y + f.y * d.z * d.z);
+}
+
 // Forward of a checkpointed ray: block (x, y) shades samples [FWD_SAMPLES y, ...) of ray x.
 // The ray's instances that are still inside their window somewhere in the tile, or echo in it,
 // are listed in list order (chunks of LIST_CAP), their records staged, and every sample
@@ -552,8 +618,11 @@ forward_ckpt_kernel(int W, int H, const int* __restrict__ ray_start, const int* 
                     const float* __restrict__ a_ele, const float* __restrict__ pert, const int* __restrict__ mono,
                     const float* __restrict__ t_pix, const float4* __restrict__ aux, const float* __restrict__ t_far,
                     float wr, float* __restrict__ image, float4* __restrict__ pixel_state) {
-    __shared__ float4 s_rec[LIST_CAP * REC_F4];
-    __shared__ float4 s_aux[LIST_CAP];
+    __shared__ float4 s_a[LIST_CAP];  // t_gauss, echo radius, first far sample, tau
+    __shared__ float4 s_b[LIST_CAP];  // tc, a0, k2, k1
+    __shared__ float4 s_c[LIST_CAP];  // k0, echo amplitude, P'12, P'22
+    __shared__ float4 s_d[LIST_CAP];  // mean, -
+    __shared__ float4 s_e[LIST_CAP];  // P'00, P'01, P'02, P'11
     constexpr int NW = FWD_SAMPLES / 32;
     __shared__ int s_list[LIST_CAP + SCAN_ROUND * FWD_SAMPLES];
     __shared__ int s_cnt[2][SCAN_ROUND * NW];  // kept instances per (chunk, warp), double-buffered
@@ -577,7 +646,7 @@ forward_ckpt_kernel(int W, int H, const int* __restrict__ ray_start, const int* 
         t_pixel = t[y];
         trans = t_far[(int64_t)x * H + y];
     }
-    float num = 0.0f, den = 0.0f, sacc = 0.0f;
+    float num = 0.0f, den = 0.0f;  // den is also the sum of weights that gamma takes
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
     int nl = 0, par = 0;  // listed instances (the same in every thread), s_cnt buffer
@@ -619,31 +688,39 @@ forward_ckpt_kernel(int W, int H, const int* __restrict__ ray_start, const int* 
         // stage and shade the listed instances (at most LIST_CAP at a time, in list order)
         for (int b0 = 0; b0 < nl; b0 += LIST_CAP) {
             const int nb = min(LIST_CAP, nl - b0);
-            for (int j = threadIdx.x; j < nb * REC_F4; j += blockDim.x) {
-                const int e = j / REC_F4, f = j - e * REC_F4;
-                s_rec[j] = rec[(int64_t)REC_F4 * sorted_gid[s0 + s_list[b0 + e]] + f];
+            for (int e = threadIdx.x; e < nb; e += blockDim.x) {
+                const int k = s0 + s_list[b0 + e];
+                const float4 a = aux[k];
+                Rec r;
+                load_rec(rec + (int64_t)REC_F4 * sorted_gid[k], r);
+                const RayWindow w = ray_window(rg, r.mu, r.s, r.R, wr);
+                s_a[e] = make_float4(a.x, a.y, a.w, r.tau);
+                s_b[e] = make_float4(w.tc, w.a0, w.k2, w.k1);
+                s_c[e] = make_float4(w.k0, r.sh.x + r.sh.y * rg.d.x + r.sh.z * rg.d.y + r.sh.w * rg.d.z,
+                                     2.0f * kNegHalfLog2e * r.P[5], kNegHalfLog2e * r.P[8]);
+                s_d[e] = make_float4(r.mu.x, r.mu.y, r.mu.z, 0.f);
+                s_e[e] = make_float4(kNegHalfLog2e * r.P[0], 2.0f * kNegHalfLog2e * r.P[1],
+                                     2.0f * kNegHalfLog2e * r.P[2], kNegHalfLog2e * r.P[4]);
             }
-            for (int e = threadIdx.x; e < nb; e += blockDim.x) s_aux[e] = aux[s0 + s_list[b0 + e]];
             __syncthreads();
             if (valid) {
                 for (int e = 0; e < nb; ++e) {
-                    const float4 a = s_aux[e];
-                    const float t_gauss = a.x;
-                    const bool need_t = t_gauss < t_pixel && y < __float_as_int(a.w);  // passed, not yet far
-                    const bool need_e = fabsf(t_gauss - t_pixel) <= a.y;
+                    const float4 a = s_a[e];
+                    const bool need_t = a.x < t_pixel && y < __float_as_int(a.z);  // passed, not yet far
+                    const bool need_e = fabsf(a.x - t_pixel) <= a.y;
                     if (!need_t && !need_e) continue;
-                    Rec r;
-                    load_rec(s_rec + e * REC_F4, r);
+                    const float4 c = s_c[e];
                     if (need_t) {
-                        const float psi = ray_integral(rg.o, rg.d, r.mu, r.s, r.R, t_pixel, wr);
-                        trans *= r.tau + (1.0f - r.tau) * __expf(-psi);
+                        const float4 b = s_b[e];
+                        const RayQuad q = ray_quad(t_pixel, b.x, b.y, b.z, b.w, c.x, wr);
+                        trans *= a.w + (1.0f - a.w) * exp2f(kNegLog2e * q.psi);
                     }
                     if (need_e) {
-                        const float wgt = gauss_weight(p, r.mu, r.P);
-                        const float I = r.sh.x + r.sh.y * rg.d.x + r.sh.z * rg.d.y + r.sh.w * rg.d.z;
-                        num += I * wgt;
+                        const float4 m = s_d[e];
+                        const float wgt = echo_weight(make_float3(p.x - m.x, p.y - m.y, p.z - m.z), s_e[e],
+                                                      make_float2(c.z, c.w));
+                        num += c.y * wgt;
                         den += wgt;
-                        sacc += wgt;
                     }
                 }
             }
@@ -654,12 +731,12 @@ forward_ckpt_kernel(int W, int H, const int* __restrict__ ray_start, const int* 
     if (!valid) return;
     float out = 0.0f;
     if (n > 0) {
-        const float gamma = 1.0f - __expf(-sacc);
+        const float gamma = 1.0f - __expf(-den);
         const float echo = num / (den + 1e-6f);
         out = trans * (gamma * echo);
     }
     image[(int64_t)y * W + x] = out;
-    pixel_state[(int64_t)x * H + y] = make_float4(trans, num, den, sacc);
+    pixel_state[(int64_t)x * H + y] = make_float4(trans, num, den, den);
 }
 
 // VJP of ray_integral w.r.t. the Gaussian (mean, scales, rotation), the quadrature nodes held
@@ -763,48 +840,8 @@ __device__ __forceinline__ void instance_epilogue(const RayGeo& rg, const Rec& r
     out[3] = dq;
 }
 
-// One instance's transmission term at a sample inside its window, and its echo term.
-__device__ __forceinline__ void near_terms(const RayGeo& rg, const Rec& r, float wr, const float4 pt, const float4 cf,
-                                           bool need_t, bool need_e, float dP[9], float dR[9], float ds[3],
-                                           float dmu[3], float& dtau_raw, float dsh[4]) {
-    const float t_pixel = pt.w;
-    if (need_t) {
-        const float psi = ray_integral(rg.o, rg.d, r.mu, r.s, r.R, t_pixel, wr);
-        const float exp_psi = __expf(-psi);
-        const float T_i = r.tau + (1.0f - r.tau) * exp_psi;
-        float dTi = 0.0f;
-        if (T_i > 1e-6f) dTi = cf.x * (cf.y / T_i);
-        dtau_raw += dTi * (1.0f - exp_psi) * (r.tau * (1.0f - r.tau));
-        const float dpsi = dTi * (1.0f - r.tau) * exp_psi * (-1.0f);
-        psi_vjp(rg, r, t_pixel, wr, dpsi, ds, dmu, dR);
-    }
-    if (need_e) {
-        const float3 p = make_float3(pt.x, pt.y, pt.z);
-        const float wgt = gauss_weight(p, r.mu, r.P);
-        const float I = r.sh.x + r.sh.y * rg.d.x + r.sh.z * rg.d.y + r.sh.w * rg.d.z;
-        const float a = cf.z * wgt;
-        dsh[0] += a;
-        dsh[1] += a * rg.d.x;
-        dsh[2] += a * rg.d.y;
-        dsh[3] += a * rg.d.z;
-        const float dw = (cf.z * I) + cf.w;
-        const float dQ = dw * wgt * (-0.5f);
-        const float dx = p.x - r.mu.x, dy = p.y - r.mu.y, dz = p.z - r.mu.z;
-        const float v0 = r.P[0] * dx + r.P[1] * dy + r.P[2] * dz;
-        const float v1 = r.P[3] * dx + r.P[4] * dy + r.P[5] * dz;
-        const float v2 = r.P[6] * dx + r.P[7] * dy + r.P[8] * dz;
-        dmu[0] += dQ * (-2.0f * v0);
-        dmu[1] += dQ * (-2.0f * v1);
-        dmu[2] += dQ * (-2.0f * v2);
-        const float ux = dQ * dx, uy = dQ * dy, uz = dQ * dz;
-        dP[0] += ux * dx; dP[1] += ux * dy; dP[2] += ux * dz;
-        dP[4] += uy * dy; dP[5] += uy * dz;
-        dP[8] += uz * dz;
-    }
-}
-
 // Backward of a checkpointed ray, per sample: the adjoint coefficients the per-sample path
-// stages (zero for samples whose |dL/dB| < 1e-6, which the reference skips), and the suffix sums
+// stages, dL/dT times T (zero for samples whose |dL/dB| < 1e-6, which the reference skips), and the suffix sums
 // along the ray of dL/dT * T (in double, fixed order; one warp per ray).
 __global__ void __launch_bounds__(32)
 ckpt_coef_kernel(int W, int H, const long long* __restrict__ header, const int* __restrict__ mono,
@@ -837,7 +874,7 @@ ckpt_coef_kernel(int W, int H, const long long* __restrict__ header, const int* 
             const float dden = de_raw * (-st.y / ((st.z + eps) * (st.z + eps)));
             const bool active = !(fabsf(gB) < 1e-6f);
             b_pos[pi] = make_float4(pp[0], pp[1], pp[2], t_pix[pi]);
-            b_coef[pi] = active ? make_float4(dT, st.x, dnum, dden + dS) : make_float4(0.f, 0.f, 0.f, 0.f);
+            b_coef[pi] = active ? make_float4(dT * st.x, dnum, dden + dS, 0.f) : make_float4(0.f, 0.f, 0.f, 0.f);
             v = active ? (double)dT * (double)st.x : 0.0;
         }
         // inclusive suffix within the chunk: lane l sums lanes l..31
@@ -852,16 +889,88 @@ ckpt_coef_kernel(int W, int H, const long long* __restrict__ header, const int* 
     }
 }
 
+// Sums over samples of one instance's backward. The integral's adjoint is linear in the canonical
+// point xc + dg u of a quadrature node, so with c the node's scalar adjoint only sum c, sum c u
+// and sum c u^2 are accumulated; the echo's in the weight adjoint times 1, d and d d^T.
+struct InstanceSums {
+    float s0, s1, s2, dtau, echo, u[3], m[6];
+};
+
+__device__ __forceinline__ void integral_sums(const RayQuad& q, float dpsi, InstanceSums& a) {
+    const float c = dpsi * q.half;
+    const float c0 = c * (0.5555555556f * q.f0), c1 = c * (0.8888888889f * q.f1), c2 = c * (0.5555555556f * q.f2);
+    const float d0 = c0 * q.u0, d1 = c1 * q.u1, d2 = c2 * q.u2;
+    a.s0 += c0 + c1 + c2;
+    a.s1 += d0 + d1 + d2;
+    a.s2 += d0 * q.u0 + d1 * q.u1 + d2 * q.u2;
+}
+
+// An instance's gradient from its sums (far_dT: the scalar adjoint of its far factor), chained
+// to dL/dR, dL/ds, dL/dmu and dL/dq.
+__device__ __forceinline__ void instance_finish(const RayGeo& rg, const Rec& r, const RayWindow& w, float wr,
+                                                float far_dT, InstanceSums& a, const float* __restrict__ quats, int g,
+                                                float4* __restrict__ out) {
+    if (far_dT != 0.0f) {
+        const RayQuad q = ray_quad(3.0e38f, w.tc, w.a0, w.k2, w.k1, w.k0, wr);
+        const float e = exp2f(kNegLog2e * q.psi);
+        a.dtau += far_dT * (1.0f - e);
+        integral_sums(q, -far_dT * (1.0f - r.tau) * e, a);
+    }
+    // integral_sums holds sum dpsi half w f (1, u, u^2); dpsi/d(canonical point) = -f times it
+    const float s0 = -a.s0, s1 = -a.s1, s2 = -a.s2;
+    const float xc[3] = {w.xc.x, w.xc.y, w.xc.z}, dg[3] = {w.dg.x, w.dg.y, w.dg.z}, is[3] = {w.is.x, w.is.y, w.is.z};
+    const float cv[3] = {w.diff.x + w.tc * rg.d.x, w.diff.y + w.tc * rg.d.y, w.diff.z + w.tc * rg.d.z};
+    const float rv[3] = {rg.d.x, rg.d.y, rg.d.z};
+    float dmu[3], ds[3], dR[9], gl[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float go = xc[k] * s0 + dg[k] * s1;  // dL/d(canonical point)
+        const float gd = xc[k] * s1 + dg[k] * s2;  // dL/d(canonical direction) about tc
+        ds[k] = -is[k] * (go * xc[k] + gd * dg[k]);
+        gl[k] = go * is[k];
+        const float hl = gd * is[k];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) dR[i * 3 + k] = gl[k] * cv[i] + hl * rv[i];
+    }
+    // echo: u = sum dQ d, m = sum dQ d d^T with dQ = dL/dQ of Q = d^T P d
+    const float m[9] = {a.m[0], a.m[1], a.m[2], a.m[1], a.m[3], a.m[4], a.m[2], a.m[4], a.m[5]};
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        dmu[i] = -(r.R[3 * i] * gl[0] + r.R[3 * i + 1] * gl[1] + r.R[3 * i + 2] * gl[2]) -
+                 2.0f * (r.P[3 * i] * a.u[0] + r.P[3 * i + 1] * a.u[1] + r.P[3 * i + 2] * a.u[2]);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float d = is[k] * is[k];
+        float t = 0.f;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const float mr = m[i * 3] * r.R[k] + m[i * 3 + 1] * r.R[3 + k] + m[i * 3 + 2] * r.R[6 + k];
+            dR[i * 3 + k] += 2.0f * mr * d;
+            t += r.R[i * 3 + k] * mr;
+        }
+        ds[k] -= 2.f * t * d * is[k];
+    }
+    const float4 q = make_float4(quats[4 * (int64_t)g], quats[4 * (int64_t)g + 1], quats[4 * (int64_t)g + 2],
+                                 quats[4 * (int64_t)g + 3]);
+    const float4 dq = quat_grad(q, dR);
+    out[0] = make_float4(dmu[0], dmu[1], dmu[2], a.dtau * (r.tau * (1.0f - r.tau)));
+    out[1] = make_float4(ds[0], ds[1], ds[2], a.echo);
+    out[2] = make_float4(a.echo * rg.d.x, a.echo * rg.d.y, a.echo * rg.d.z, 0.f);
+    out[3] = dq;
+}
+
 // Thread per instance of a checkpointed ray: the far part of its gradient from the suffix sum at
 // its first far sample, the samples inside its window [first sample past t_gauss, first far
 // sample) and its echo range |t - t_gauss| <= radius visited in sample order. The ray's
 // instances go out in chunks of CKPT_CHUNK; a block first finds each instance's sample range and
 // then hands the instances to its threads in order of that range's length (a counting sort on
 // CKPT_BINS classes), so that the lanes of a warp sweep similar numbers of samples. Which thread
-// computes an instance does not change its partial.
+// computes an instance does not change its partial. A chunk's instances are neighbours in depth,
+// so the samples it visits are staged in shared memory when they fit CKPT_SAMPLES.
 constexpr int CKPT_CHUNK = 512;
 constexpr int CKPT_BINS = 32;  // classes of 8 samples
-__global__ void __launch_bounds__(128)
+constexpr int CKPT_SAMPLES = 512;
+__global__ void __launch_bounds__(128, 5)
 backward_ckpt_kernel(int W, int H, const int* __restrict__ ray_start, const int* __restrict__ sorted_gid,
                      const int* __restrict__ sorted_inst, const long long* __restrict__ header,
                      const float4* __restrict__ rec, const float* __restrict__ quats, const float* __restrict__ ray_o,
@@ -869,10 +978,12 @@ backward_ckpt_kernel(int W, int H, const int* __restrict__ ray_start, const int*
                      const int* __restrict__ mono, const float* __restrict__ t_pix, const float4* __restrict__ aux,
                      const float4* __restrict__ b_pos, const float4* __restrict__ b_coef,
                      const float* __restrict__ b_suffix, float wr, float4* __restrict__ partial) {
+    __shared__ float4 s_pos[CKPT_SAMPLES], s_coef[CKPT_SAMPLES];
     __shared__ int s_key[CKPT_CHUNK];  // length class << 16 | rank within the class
     __shared__ int s_ord[CKPT_CHUNK];  // chunk positions ordered by class
     __shared__ int s_yt[CKPT_CHUNK], s_ya[CKPT_CHUNK], s_yb[CKPT_CHUNK];
     __shared__ int s_bin[CKPT_BINS];
+    __shared__ int s_lo, s_hi;  // samples the chunk visits
     if (header[H_FLAGS] != 0) return;
     const int x = blockIdx.x;
     if (!mono[x]) return;
@@ -884,7 +995,12 @@ backward_ckpt_kernel(int W, int H, const int* __restrict__ ray_start, const int*
         const int nc = min(CKPT_CHUNK, n - k0);
         __syncthreads();  // the previous chunk's arrays are read to the end
         if (threadIdx.x < CKPT_BINS) s_bin[threadIdx.x] = 0;
+        if (threadIdx.x == 0) {
+            s_lo = H;
+            s_hi = 0;
+        }
         __syncthreads();
+        int lo = H, hi = 0;
         for (int j = threadIdx.x; j < nc; j += blockDim.x) {
             const float4 a = aux[s0 + k0 + j];
             const float t_gauss = a.x, radius = a.y;
@@ -896,8 +1012,18 @@ backward_ckpt_kernel(int W, int H, const int* __restrict__ ray_start, const int*
             s_yt[j] = y_t;
             s_ya[j] = ya;
             s_yb[j] = yb;
+            if (ya < yb) {
+                lo = min(lo, ya);
+                hi = max(hi, yb);
+            }
             const int bin = min(CKPT_BINS - 1, max(yb - ya, 0) >> 3);
             s_key[j] = (bin << 16) | atomicAdd(&s_bin[bin], 1);
+        }
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        if ((threadIdx.x & 31) == 0) {
+            atomicMin(&s_lo, lo);
+            atomicMax(&s_hi, hi);
         }
         __syncthreads();
         if (threadIdx.x < 32) {  // exclusive scan of the class counts in one warp
@@ -909,6 +1035,14 @@ backward_ckpt_kernel(int W, int H, const int* __restrict__ ray_start, const int*
             }
             s_bin[threadIdx.x] = incl - v;
         }
+        lo = s_lo;
+        hi = s_hi;
+        const bool staged = hi - lo <= CKPT_SAMPLES;
+        if (staged)
+            for (int i = threadIdx.x; i < hi - lo; i += blockDim.x) {
+                s_pos[i] = b_pos[row + lo + i];
+                s_coef[i] = b_coef[row + lo + i];
+            }
         __syncthreads();
         for (int j = threadIdx.x; j < nc; j += blockDim.x) {
             const int key = s_key[j];
@@ -923,30 +1057,48 @@ backward_ckpt_kernel(int W, int H, const int* __restrict__ ray_start, const int*
             const float4 a = aux[s0 + k];
             const float t_gauss = a.x, radius = a.y;
             const int y_far = __float_as_int(a.w);
-            float dmu[3] = {0.f, 0.f, 0.f}, ds[3] = {0.f, 0.f, 0.f}, dR[9], dP[9], dtau_raw = 0.f;
-            float dsh[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int i = 0; i < 9; ++i) {
-                dR[i] = 0.f;
-                dP[i] = 0.f;
-            }
-            // the far factor, as the per-sample path evaluates it
-            const float psi = ray_integral(rg.o, rg.d, r.mu, r.s, r.R, 3.0e38f, wr);
-            const float far_exp = __expf(-psi);
-            const float far_T = r.tau + (1.0f - r.tau) * far_exp;
+            const RayWindow w = ray_window(rg, r.mu, r.s, r.R, wr);
+            const float amp = r.sh.x + r.sh.y * rg.d.x + r.sh.z * rg.d.y + r.sh.w * rg.d.z;
+            const float4 e = make_float4(kNegHalfLog2e * r.P[0], 2.0f * kNegHalfLog2e * r.P[1],
+                                         2.0f * kNegHalfLog2e * r.P[2], kNegHalfLog2e * r.P[4]);
+            const float2 f = make_float2(2.0f * kNegHalfLog2e * r.P[5], kNegHalfLog2e * r.P[8]);
+            const float tau = r.tau;
+            InstanceSums acc = {};
             const int y_t = s_yt[j], ya = s_ya[j], yb = s_yb[j];
-            for (int y = ya; y < yb; ++y) {
-                const float4 cf = b_coef[row + y];
-                if (cf.x == 0.0f && cf.z == 0.0f && cf.w == 0.0f) continue;  // skipped sample: every term is zero
-                const float4 pt = b_pos[row + y];
-                const bool need_t = y >= y_t && y < y_far;
-                const bool need_e = fabsf(t_gauss - pt.w) <= radius;
-                if (need_t || need_e) near_terms(rg, r, wr, pt, cf, need_t, need_e, dP, dR, ds, dmu, dtau_raw, dsh);
-            }
+            auto sweep = [&](const float4* pos, const float4* coef, int first) {
+                for (int y = ya; y < yb; ++y) {
+                    const float4 cf = coef[y - first];
+                    if (cf.x == 0.0f && cf.y == 0.0f && cf.z == 0.0f) continue;  // skipped sample: every term is zero
+                    const float4 pt = pos[y - first];
+                    if (y >= y_t && y < y_far) {
+                        const RayQuad qd = ray_quad(pt.w, w.tc, w.a0, w.k2, w.k1, w.k0, wr);
+                        const float ep = exp2f(kNegLog2e * qd.psi);
+                        const float Ti = tau + (1.0f - tau) * ep;
+                        const float dTi = Ti > 1e-6f ? cf.x / Ti : 0.0f;
+                        acc.dtau += dTi * (1.0f - ep);
+                        integral_sums(qd, -dTi * (1.0f - tau) * ep, acc);
+                    }
+                    if (fabsf(t_gauss - pt.w) <= radius) {
+                        const float3 d = make_float3(pt.x - r.mu.x, pt.y - r.mu.y, pt.z - r.mu.z);
+                        const float wgt = echo_weight(d, e, f);
+                        acc.echo += cf.y * wgt;
+                        const float dQ = (cf.y * amp + cf.z) * wgt * -0.5f;
+                        const float ux = dQ * d.x, uy = dQ * d.y, uz = dQ * d.z;
+                        acc.u[0] += ux; acc.u[1] += uy; acc.u[2] += uz;
+                        acc.m[0] += ux * d.x; acc.m[1] += ux * d.y; acc.m[2] += ux * d.z;
+                        acc.m[3] += uy * d.y; acc.m[4] += uy * d.z;
+                        acc.m[5] += uz * d.z;
+                    }
+                }
+            };
+            if (staged)
+                sweep(s_pos, s_coef, lo);
+            else
+                sweep(b_pos + row, b_coef + row, 0);
             float far_dT = 0.0f;
-            if (y_far < H && far_T > 1e-6f) far_dT = b_suffix[row + y_far] / far_T;
-            instance_epilogue(rg, r, wr, far_dT, far_exp, dP, dR, ds, dmu, dtau_raw, dsh, quats, g,
-                              partial + (int64_t)PARTIAL_F4 * sorted_inst[s0 + k]);
+            // the far factor as the forward's checkpoints hold it
+            if (y_far < H && a.z > 1e-6f) far_dT = b_suffix[row + y_far] / a.z;
+            instance_finish(rg, r, w, wr, far_dT, acc, quats, g, partial + (int64_t)PARTIAL_F4 * sorted_inst[s0 + k]);
         }
     }
 }
