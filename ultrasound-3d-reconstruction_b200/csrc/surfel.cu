@@ -215,7 +215,7 @@ __device__ __forceinline__ int sh_color(int g, int deg, int M, const float* mean
 
 struct Workspace {
     long long* header;
-    float4* rec;           // G x 5
+    float4* rec;           // G x 5; the last two floats hold the reach box
     float* depth;          // G (view depth, key bits)
     int4* rect;            // G tile rectangle [x0, y0, x1, y1)
     int* clamped;          // G (bits 0..2)
@@ -296,6 +296,37 @@ __global__ void init_kernel(int64_t T, int* __restrict__ tile_count, int* __rest
     tile_cursor[t] = 0;
 }
 
+// Pixel columns [x0, x1] and rows [y0, y1] that hold every pixel whose alpha with this surfel can
+// reach 1/255, as four 16-bit numbers: the box of {rho3d <= c} (the screen box of forward.cu:109-139
+// with the cutoff c = 2 ln(255 opacity) in the place of 9) together with the filter's disc
+// {rho2d <= c}, in double precision and half a pixel wider than that, which covers the float
+// rounding of the per-pixel test (about 1e-3 pixel). Everything when the box is unbounded (the
+// splat's plane passes the camera) or not finite; nothing when the opacity is below 1/255.
+__device__ __forceinline__ uint2 reach_box(const V3 T0, const V3 T1, const V3 T2, float px, float py, float opacity) {
+    const uint2 all = make_uint2(0x7fff8000u, 0x7fff8000u);  // low half: first, high half: last
+    if (opacity * 255.0f < 0.999f) return make_uint2(0x80007fffu, 0x80007fffu);
+    const double c = 2.0 * (double)logf(255.0f * opacity) * 1.0001 + 1e-3;
+    const double x0 = T0.x, x1 = T0.y, x2 = T0.z, y0 = T1.x, y1 = T1.y, y2 = T1.z, w0 = T2.x, w1 = T2.y, w2 = T2.z;
+    const double d = c * (w0 * w0 + w1 * w1) - w2 * w2;
+    if (!(d < -1e-6 * w2 * w2)) return all;
+    const double id = 1.0 / d;
+    const double ux = (c * (x0 * w0 + x1 * w1) - x2 * w2) * id, uy = (c * (y0 * w0 + y1 * w1) - y2 * w2) * id;
+    const double hx = sqrt(fmax(0.0, ux * ux - (c * (x0 * x0 + x1 * x1) - x2 * x2) * id));
+    const double hy = sqrt(fmax(0.0, uy * uy - (c * (y0 * y0 + y1 * y1) - y2 * y2) * id));
+    const double r = sqrt(c / FILTER_INV_SQUARE);
+    const double a = floor(fmin(ux - hx, px - r) - 0.5), b = ceil(fmax(ux + hx, px + r) + 0.5);
+    const double e = floor(fmin(uy - hy, py - r) - 0.5), f = ceil(fmax(uy + hy, py + r) + 0.5);
+    if (!(a <= b) || !(e <= f)) return all;  // not finite
+    auto half = [](double v) { return (unsigned)(int)fmin(fmax(v, -32768.0), 32767.0) & 0xffffu; };
+    return make_uint2(half(a) | (half(b) << 16), half(e) | (half(f) << 16));
+}
+
+// Whether a reach box meets columns [bx, bx + w) and rows [by, by + h).
+__device__ __forceinline__ bool reaches(unsigned xr, unsigned yr, int bx, int by, int w, int h) {
+    return (int)(short)(xr & 0xffffu) < bx + w && (int)(short)(xr >> 16) >= bx &&
+           (int)(short)(yr & 0xffffu) < by + h && (int)(short)(yr >> 16) >= by;
+}
+
 // Per Gaussian: near cull, homography, dual-visible normal, AABB radius, tile rectangle,
 // colour, render record, per-tile counts (forward.cu:141-246).
 __global__ void __launch_bounds__(256)
@@ -373,7 +404,8 @@ preprocess_kernel(Params p, int* __restrict__ radii, float4* __restrict__ rec, f
     o[1] = make_float4(T1.x, T1.y, T1.z, py);
     o[2] = make_float4(T2.x, T2.y, T2.z, p.opacities[g]);
     o[3] = make_float4(normal.x, normal.y, normal.z, rgb[0]);
-    o[4] = make_float4(rgb[1], rgb[2], 0.f, 0.f);
+    const uint2 box = reach_box(T0, T1, T2, px, py, p.opacities[g]);
+    o[4] = make_float4(rgb[1], rgb[2], __uint_as_float(box.x), __uint_as_float(box.y));
     rect_out[g] = make_int4(x0, y0, x1, y1);
     touched[g] = (x1 - x0) * (y1 - y0);
     (void)tile_count;  // counted per block by rect_count_kernel
@@ -430,17 +462,31 @@ __device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
+// A warp shades a block of 8 columns x 4 rows (warp w: column block w & 1, row block w >> 1).
+constexpr int BLK_W = 8, BLK_H = 4;
+__device__ __forceinline__ int block_x(int t) { return ((t >> 5) & 1) * BLK_W + (t & (BLK_W - 1)); }
+__device__ __forceinline__ int block_y(int t) { return (t >> 6) * BLK_H + ((t & 31) >> 3); }
+
+// One CTA per tile, one pixel per thread. Per staged batch every warp lists, by ballot and in order, the
+// surfels whose reach box meets its 8x4 pixels and composites only those: the others fail the alpha
+// test on all of them (decisions and sums are those of the whole list, and a contributor's number is
+// its place in the tile's list). The intersections of two listed surfels are evaluated together,
+// since what bounds the kernel is the dependent chain of the tile with the longest list (a clustered
+// scene of 200k surfels at 256x256: SMs 690k cycles busy on average, 2.07M at most). That
+// scene: US3D_GS_FWD
 __global__ void __launch_bounds__(BLOCK)
 forward_kernel(int W, int H, int gx, const int* __restrict__ tile_start, const int* __restrict__ sorted_gid,
                const long long* __restrict__ header, const float4* __restrict__ rec, const float* __restrict__ bg,
                float* __restrict__ out_color, float* __restrict__ out_others, float* __restrict__ accum,
                uint32_t* __restrict__ n_contrib) {
     __shared__ float4 s_rec[2][REC_F4][BLOCK];  // double-buffered staging
+    __shared__ unsigned char s_list[BLOCK / 32][BLOCK];
     if (header[H_FLAGS] != 0) return;
     const int tile = blockIdx.x;
     const int tx = tile % gx, ty = tile / gx;
-    const int lx = threadIdx.x % TILE, ly = threadIdx.x / TILE;
-    const uint32_t pxi = (uint32_t)(tx * TILE + lx), pyi = (uint32_t)(ty * TILE + ly);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int bx = tx * TILE + (warp & 1) * BLK_W, by = ty * TILE + (warp >> 1) * BLK_H;
+    const uint32_t pxi = (uint32_t)(tx * TILE + block_x(threadIdx.x)), pyi = (uint32_t)(ty * TILE + block_y(threadIdx.x));
     const bool inside = pxi < (uint32_t)W && pyi < (uint32_t)H;
     const float pxf = (float)pxi, pyf = (float)pyi;
     bool done = !inside;
@@ -448,7 +494,7 @@ forward_kernel(int W, int H, int gx, const int* __restrict__ tile_start, const i
     const int rounds = (n + BLOCK - 1) / BLOCK;
     int todo = n;
     float T = 1.0f;
-    uint32_t contributor = 0, last_contributor = 0;
+    uint32_t last_contributor = 0;
     float C[3] = {0.f, 0.f, 0.f};
     float N[3] = {0.f, 0.f, 0.f};
     float D = 0.f, M1 = 0.f, M2 = 0.f, distortion = 0.f, median_depth = 0.f, median_contributor = -1.f;
@@ -470,35 +516,50 @@ forward_kernel(int W, int H, int gx, const int* __restrict__ tile_start, const i
         cp_async_wait_all();  // this thread's copies of round i have landed
         if (__syncthreads_count(done) == BLOCK) break;  // ... and everyone's; no copy is in flight
         if (i + 1 < rounds) stage(i + 1);
+        if (__all_sync(0xffffffffu, done)) continue;
         const float4(*sr)[BLOCK] = s_rec[i & 1];
         const int nb = min(BLOCK, todo);
-        for (int j = 0; !done && j < nb; ++j) {
-            ++contributor;
-            const float4 r0 = sr[0][j], r1 = sr[1][j], r2 = sr[2][j];
-            Hit h;
-            if (!intersect(pxf, pyf, r0, r1, r2, h)) continue;
-            const float rho = fminf(h.rho3d, h.rho2d);
-            const float power = -0.5f * rho;
-            if (power > 0.0f) continue;
+        int nl = 0;
+        for (int jc = 0; jc < nb; jc += 32) {
+            const int jl = jc + lane;
+            const bool mine = jl < nb && reaches(__float_as_uint(sr[4][jl].z), __float_as_uint(sr[4][jl].w), bx, by,
+                                                 BLK_W, BLK_H);
+            const unsigned bits = __ballot_sync(0xffffffffu, mine);
+            if (mine) s_list[warp][nl + __popc(bits & ((1u << lane) - 1u))] = (unsigned char)jl;
+            nl += __popc(bits);
+        }
+        __syncwarp();
+        // alpha of surfel j at this pixel, 0 when the pair is skipped
+        auto alpha_of = [&](int j, float& depth) {
+            const float4 r2 = sr[2][j];
+            Hit h = {};
+            const bool ok = intersect(pxf, pyf, sr[0][j], sr[1][j], r2, h);
+            const float power = -0.5f * fminf(h.rho3d, h.rho2d);
             const float alpha = fminf(0.99f, r2.w * __expf(power));
-            if (alpha < 1.0f / 255.0f) continue;
+            depth = h.depth;
+            return ok && !(power > 0.0f) && !(alpha < 1.0f / 255.0f) ? alpha : 0.0f;
+        };
+        auto composite = [&](int j, float alpha, float depth) {
+            if (alpha == 0.0f || done) return;
             const float test_T = T * (1 - alpha);
             if (test_T < 0.0001f) {
                 done = true;
-                continue;
+                return;
             }
             const float w = alpha * T;
             const float A = 1 - T;
-            const float m = mscale * (1 - NEAR_N / h.depth);
+            const float m = mscale * (1 - NEAR_N / depth);
             distortion += (m * m * A + M2 - 2 * m * M1) * w;
-            D += h.depth * w;
+            D += depth * w;
             M1 += m * w;
             M2 += m * m * w;
+            last_contributor = (uint32_t)(i * BLOCK + j + 1);
             if (T > 0.5) {
-                median_depth = h.depth;
-                median_contributor = (float)contributor;
+                median_depth = depth;
+                median_contributor = (float)last_contributor;
             }
-            const float4 r3 = sr[3][j], r4 = sr[4][j];
+            const float4 r3 = sr[3][j];
+            const float2 r4 = *reinterpret_cast<const float2*>(&sr[4][j]);
             N[0] += r3.x * w;
             N[1] += r3.y * w;
             N[2] += r3.z * w;
@@ -506,7 +567,20 @@ forward_kernel(int W, int H, int gx, const int* __restrict__ tile_start, const i
             C[1] += r4.x * w;
             C[2] += r4.y * w;
             T = test_T;
-            last_contributor = contributor;
+        };
+        int e = 0;
+        for (; e + 2 <= nl; e += 2) {
+            const int ja = s_list[warp][e], jb = s_list[warp][e + 1];
+            float da, db;
+            const float aa = alpha_of(ja, da), ab = alpha_of(jb, db);
+            composite(ja, aa, da);
+            composite(jb, ab, db);
+        }
+        if (e < nl) {
+            const int ja = s_list[warp][e];
+            float da;
+            const float aa = alpha_of(ja, da);
+            composite(ja, aa, da);
         }
     }
     if (inside) {
@@ -532,46 +606,49 @@ forward_kernel(int W, int H, int gx, const int* __restrict__ tile_start, const i
 // Backward
 // ------------------------------------------------------------------------------------
 
-// Sum of v[0..23] over the 32 lanes of a warp, transposed: on return lanes with
-// (lane & 3) == 0 hold the totals of entries [3 (lane >> 2), 3 (lane >> 2) + 3) in o[0..2].
-__device__ __forceinline__ void warp_reduce24(const float (&v)[24], float (&o)[3]) {
+// Sums of va[0..17] and vb[0..17] over the 32 lanes of a warp, transposed: the first exchange gives
+// lanes 0-15 the terms of a and lanes 16-31 those of b, the next ones halve the terms that a lane
+// carries, 37 shuffles for both (27 for each alone). On return a lane holds the totals of
+// terms [base, base + count) of its instance in o[0..1], see PairSlot.
+__device__ __forceinline__ void warp_reduce_pair(const float (&va)[NGRAD], const float (&vb)[NGRAD], float (&o)[2]) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    float a[12];
-    const bool h16 = lane & 16;
+    const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4, h2 = lane & 2, h1 = lane & 1;
+    float x[18], y[10], z[6], w[4];
 #pragma unroll
-    for (int i = 0; i < 12; ++i) {
-        const float send = h16 ? v[i] : v[12 + i];
-        const float keep = h16 ? v[12 + i] : v[i];
-        a[i] = keep + __shfl_xor_sync(FULL, send, 16);
-    }
-    float b[6];
-    const bool h8 = lane & 8;
+    for (int i = 0; i < 18; ++i) x[i] = (h16 ? vb[i] : va[i]) + __shfl_xor_sync(FULL, h16 ? va[i] : vb[i], 16);
 #pragma unroll
-    for (int i = 0; i < 6; ++i) {
-        const float send = h8 ? a[i] : a[6 + i];
-        const float keep = h8 ? a[6 + i] : a[i];
-        b[i] = keep + __shfl_xor_sync(FULL, send, 8);
-    }
-    const bool h4 = lane & 4;
+    for (int i = 0; i < 9; ++i) y[i] = (h8 ? x[9 + i] : x[i]) + __shfl_xor_sync(FULL, h8 ? x[i] : x[9 + i], 8);
+    y[9] = 0.f;
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const float send = h4 ? b[i] : b[3 + i];
-        const float keep = h4 ? b[3 + i] : b[i];
-        o[i] = keep + __shfl_xor_sync(FULL, send, 4);
-    }
+    for (int i = 0; i < 5; ++i) z[i] = (h4 ? y[5 + i] : y[i]) + __shfl_xor_sync(FULL, h4 ? y[i] : y[5 + i], 4);
+    z[5] = 0.f;
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        o[i] += __shfl_xor_sync(FULL, o[i], 2);
-        o[i] += __shfl_xor_sync(FULL, o[i], 1);
-    }
+    for (int i = 0; i < 3; ++i) w[i] = (h2 ? z[3 + i] : z[i]) + __shfl_xor_sync(FULL, h2 ? z[i] : z[3 + i], 2);
+    w[3] = 0.f;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) o[i] = (h1 ? w[2 + i] : w[i]) + __shfl_xor_sync(FULL, h1 ? w[i] : w[2 + i], 1);
+}
+
+// The terms that a lane holds after warp_reduce_pair.
+struct PairSlot {
+    int base, count;
+};
+__device__ __forceinline__ PairSlot pair_slot(int lane) {
+    const int n8 = 9, n4 = (lane & 4) ? 4 : 5;
+    const int n2 = (lane & 2) ? max(n4 - 3, 0) : min(n4, 3);
+    const int n1 = (lane & 1) ? max(n2 - 2, 0) : min(n2, 2);
+    return PairSlot{((lane & 8) ? n8 : 0) + ((lane & 4) ? 5 : 0) + ((lane & 2) ? 3 : 0) + ((lane & 1) ? 2 : 0), n1};
 }
 
 // One CTA per tile, one pixel per thread, Gaussians replayed back to front
-// (backward.cu:103-404). Per staged Gaussian the block's 256 pixel contributions are summed
-// in a fixed order into the instance's 18-term partial:
+// (backward.cu:103-404). As in the forward, a warp holds 8x4 pixels and replays only the surfels whose
+// reach box meets them, two at a time: their intersections are independent, and their gradient terms
+// share one transposed warp reduction. Per staged Gaussian the sums of the warps that replayed it are
+// added in warp order into the instance's 18-term partial:
 //   [0..2] dL/dTu  [3..5] dL/dTv  [6..8] dL/dTw  [9..10] dL/dmean2D  [11..13] dL/dnormal
 //   [14] dL/dopacity  [15..17] dL/dcolor
+// Bound by the replay chain of the longest tile list. US3D_GS_BWD
 __global__ void __launch_bounds__(BLOCK)
 backward_kernel(int W, int H, int gx, const int* __restrict__ tile_start, const int* __restrict__ sorted_gid,
                 const int* __restrict__ sorted_inst, const long long* __restrict__ header,
@@ -581,15 +658,18 @@ backward_kernel(int W, int H, int gx, const int* __restrict__ tile_start, const 
     __shared__ float4 s_rec[2][REC_F4][BWD_BATCH];  // double-buffered staging
     __shared__ int s_inst[2][BWD_BATCH];
     __shared__ float s_red[BWD_BATCH][BLOCK / 32][NGRAD];
+    __shared__ unsigned s_who[BWD_BATCH];  // warps that wrote their sums
+    __shared__ unsigned char s_list[BLOCK / 32][BWD_BATCH];
     __shared__ int s_last;
     if (header[H_FLAGS] != 0) return;
     const int tile = blockIdx.x;
     const int tx = tile % gx, ty = tile / gx;
-    const int lx = threadIdx.x % TILE, ly = threadIdx.x / TILE;
-    const uint32_t pxi = (uint32_t)(tx * TILE + lx), pyi = (uint32_t)(ty * TILE + ly);
+    const uint32_t pxi = (uint32_t)(tx * TILE + block_x(threadIdx.x)), pyi = (uint32_t)(ty * TILE + block_y(threadIdx.x));
     const bool inside = pxi < (uint32_t)W && pyi < (uint32_t)H;
     const float pxf = (float)pxi, pyf = (float)pyi;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int bx = tx * TILE + (warp & 1) * BLK_W, by = ty * TILE + (warp >> 1) * BLK_H;
+    const PairSlot slot = pair_slot(lane);
     const int s0 = tile_start[tile], n = tile_start[tile + 1] - s0;
     const int64_t HW = (int64_t)H * W;
     const int64_t pix = (int64_t)W * pyi + pxi;
@@ -605,12 +685,12 @@ backward_kernel(int W, int H, int gx, const int* __restrict__ tile_start, const 
     if (last_contributor > 0) atomicMax(&s_last, last_contributor);
     __syncthreads();
     const int n_live = min(s_last, n);
+    const int warp_last = __reduce_max_sync(0xffffffffu, last_contributor);
     for (int k = n_live + threadIdx.x; k < n; k += BLOCK) {
         float4* out = partial + (int64_t)PARTIAL_F4 * sorted_inst[s0 + k];
 #pragma unroll
         for (int f = 0; f < PARTIAL_F4; ++f) out[f] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    uint32_t contributor = (uint32_t)n_live;
     const int median_contributor = inside ? (int)n_contrib[pix + HW] : 0;
     float dpix[3] = {0.f, 0.f, 0.f};
     float dd_depth = 0.f, dd_accum = 0.f, dd_reg = 0.f, dd_median = 0.f;
@@ -670,125 +750,129 @@ backward_kernel(int W, int H, int gx, const int* __restrict__ tile_start, const 
         }
         const float4(*sr)[BWD_BATCH] = s_rec[k & 1];
         const int* si = s_inst[k & 1];
-        for (int jj = 0; jj < nb; ++jj) {
-            float v[24];
+        if (threadIdx.x < BWD_BATCH) s_who[threadIdx.x] = 0u;
+        __syncthreads();
+        int nl = 0;
 #pragma unroll
-            for (int q = 0; q < 24; ++q) v[q] = 0.f;
-            bool contrib = false;
-            if (inside) {
-                --contributor;
-                if (contributor < (uint32_t)last_contributor) {
-                    const float4 r0 = sr[0][jj], r1 = sr[1][jj], r2 = sr[2][jj];
-                    Hit h;
-                    const bool hit = intersect(pxf, pyf, r0, r1, r2, h);
-                    float G = 0.f, alpha = 0.f;
-                    bool ok = hit;
-                    if (ok) {
-                        const float rho = fminf(h.rho3d, h.rho2d);
-                        const float power = -0.5f * rho;
-                        if (power > 0.0f) ok = false;
-                        if (ok) {
-                            G = __expf(power);
-                            alpha = fminf(0.99f, r2.w * G);
-                            if (alpha < 1.0f / 255.0f) ok = false;
-                        }
-                    }
-                    if (ok) {
-                        contrib = true;
-                        const float4 r3 = sr[3][jj], r4 = sr[4][jj];
-                        const float col[3] = {r3.w, r4.x, r4.y};
-                        const float nrm[3] = {r3.x, r3.y, r3.z};
-                        T = T / (1.f - alpha);
-                        const float wT = alpha * T;
-                        float dL_dalpha = 0.0f;
+        for (int jc = 0; jc < BWD_BATCH; jc += 32) {
+            const int jl = jc + lane;
+            // entry jl is contributor n_live - b0 - jl (counted from one): none of the warp's pixels
+            // has a contributor beyond warp_last
+            const bool mine = jl < nb && n_live - b0 - jl <= warp_last &&
+                              reaches(__float_as_uint(sr[4][jl].z), __float_as_uint(sr[4][jl].w), bx, by, BLK_W, BLK_H);
+            const unsigned bits = __ballot_sync(0xffffffffu, mine);
+            if (mine) s_list[warp][nl + __popc(bits & ((1u << lane) - 1u))] = (unsigned char)jl;
+            nl += __popc(bits);
+        }
+        __syncwarp();
+        // the pair (this pixel, entry jj): whether it contributes, and its weight
+        auto evaluate = [&](int jj, Hit& h, float& G, float& alpha) {
+            h = {};
+            const float4 r2 = sr[2][jj];
+            const bool hit = intersect(pxf, pyf, sr[0][jj], sr[1][jj], r2, h);
+            const float power = -0.5f * fminf(h.rho3d, h.rho2d);
+            G = __expf(power);
+            alpha = fminf(0.99f, r2.w * G);
+            return n_live - b0 - jj <= last_contributor && hit && !(power > 0.0f) && !(alpha < 1.0f / 255.0f);
+        };
+        // one step of the replay: the gradient terms of the pair
+        auto replay = [&](int jj, const Hit& h, float G, float alpha, float (&v)[NGRAD]) {
+            const float4 r2 = sr[2][jj], r3 = sr[3][jj];
+            const float2 r4 = *reinterpret_cast<const float2*>(&sr[4][jj]);
+            const float col[3] = {r3.w, r4.x, r4.y};
+            const float nrm[3] = {r3.x, r3.y, r3.z};
+            T = T / (1.f - alpha);
+            const float wT = alpha * T;
+            float dL_dalpha = 0.0f;
 #pragma unroll
-                        for (int ch = 0; ch < 3; ++ch) {
-                            accum_rec[ch] = last_alpha * last_color[ch] + (1.f - last_alpha) * accum_rec[ch];
-                            last_color[ch] = col[ch];
-                            dL_dalpha += (col[ch] - accum_rec[ch]) * dpix[ch];
-                            v[15 + ch] = wT * dpix[ch];
-                        }
-                        float dL_dz = 0.0f;
-                        const float c_d = h.depth;
-                        const float m_d = mscale * (1 - NEAR_N / c_d);
-                        const float dmd_dd = (FAR_N * NEAR_N) / ((FAR_N - NEAR_N) * c_d * c_d);
-                        if (contributor == (uint32_t)(median_contributor - 1)) dL_dz += dd_median;
-                        const float dL_dweight = (final_D2 + m_d * m_d * final_A - 2 * m_d * final_D) * dd_reg;
-                        dL_dalpha += dL_dweight - last_dL_dT;
-                        last_dL_dT = dL_dweight * alpha + (1 - alpha) * last_dL_dT;
-                        const float dL_dmd = 2.0f * (T * alpha) * (m_d * final_A - final_D) * dd_reg;
-                        dL_dz += dL_dmd * dmd_dd;
-                        accum_depth_rec = last_alpha * last_depth + (1.f - last_alpha) * accum_depth_rec;
-                        last_depth = c_d;
-                        dL_dalpha += (c_d - accum_depth_rec) * dd_depth;
-                        // the reference adds last_alpha * 1.0 in double precision
-                        accum_alpha_rec = (float)((double)last_alpha + (double)__fmul_rn(1.f - last_alpha, accum_alpha_rec));
-                        dL_dalpha += (1 - accum_alpha_rec) * dd_accum;
-#pragma unroll
-                        for (int ch = 0; ch < 3; ++ch) {
-                            accum_normal_rec[ch] = last_alpha * last_normal[ch] + (1.f - last_alpha) * accum_normal_rec[ch];
-                            last_normal[ch] = nrm[ch];
-                            dL_dalpha += (nrm[ch] - accum_normal_rec[ch]) * dd_normal[ch];
-                            v[11 + ch] = alpha * T * dd_normal[ch];
-                        }
-                        dL_dalpha *= T;
-                        last_alpha = alpha;
-                        dL_dalpha += (-T_final / (1.f - alpha)) * bg_dot_dpixel;
-                        const float dL_dG = r2.w * dL_dalpha;
-                        dL_dz += alpha * T * dd_depth;
-                        if (h.rho3d <= h.rho2d) {
-                            const float dsx = dL_dG * -G * h.sx + dL_dz * r2.x;
-                            const float dsy = dL_dG * -G * h.sy + dL_dz * r2.y;
-                            const float dsx_pz = dsx / h.p.z, dsy_pz = dsy / h.p.z;
-                            const V3 dL_dp = v3(dsx_pz, dsy_pz, -(dsx_pz * h.sx + dsy_pz * h.sy));
-                            const V3 dL_dk = vcross(h.l, dL_dp);
-                            const V3 dL_dl = vcross(dL_dp, h.k);
-                            v[0] = -dL_dk.x; v[1] = -dL_dk.y; v[2] = -dL_dk.z;
-                            v[3] = -dL_dl.x; v[4] = -dL_dl.y; v[5] = -dL_dl.z;
-                            v[6] = pxf * dL_dk.x + pyf * dL_dl.x + dL_dz * h.sx;
-                            v[7] = pxf * dL_dk.y + pyf * dL_dl.y + dL_dz * h.sy;
-                            v[8] = pxf * dL_dk.z + pyf * dL_dl.z + dL_dz * 1.0f;
-                        } else {
-                            const float dG_ddelx = -G * FILTER_INV_SQUARE * h.dx;
-                            const float dG_ddely = -G * FILTER_INV_SQUARE * h.dy;
-                            v[9] = dL_dG * dG_ddelx;
-                            v[10] = dL_dG * dG_ddely;
-                            v[6] = h.sx * dL_dz;
-                            v[7] = h.sy * dL_dz;
-                            v[8] = dL_dz;
-                        }
-                        v[14] = G * dL_dalpha;
-                    }
-                }
+            for (int ch = 0; ch < 3; ++ch) {
+                accum_rec[ch] = last_alpha * last_color[ch] + (1.f - last_alpha) * accum_rec[ch];
+                last_color[ch] = col[ch];
+                dL_dalpha += (col[ch] - accum_rec[ch]) * dpix[ch];
+                v[15 + ch] = wT * dpix[ch];
             }
-            if (__any_sync(0xffffffffu, contrib)) {
-                float o[3];
-                warp_reduce24(v, o);
-                const int base = 3 * (lane >> 2);
-                if ((lane & 3) == 0 && base < NGRAD) {
-                    s_red[jj][warp][base] = o[0];
-                    s_red[jj][warp][base + 1] = o[1];
-                    s_red[jj][warp][base + 2] = o[2];
-                }
-            } else if (lane < NGRAD) {
-                s_red[jj][warp][lane] = 0.f;
+            float dL_dz = 0.0f;
+            const float c_d = h.depth;
+            const float m_d = mscale * (1 - NEAR_N / c_d);
+            const float dmd_dd = (FAR_N * NEAR_N) / ((FAR_N - NEAR_N) * c_d * c_d);
+            if (n_live - b0 - jj == median_contributor) dL_dz += dd_median;
+            const float dL_dweight = (final_D2 + m_d * m_d * final_A - 2 * m_d * final_D) * dd_reg;
+            dL_dalpha += dL_dweight - last_dL_dT;
+            last_dL_dT = dL_dweight * alpha + (1 - alpha) * last_dL_dT;
+            const float dL_dmd = 2.0f * (T * alpha) * (m_d * final_A - final_D) * dd_reg;
+            dL_dz += dL_dmd * dmd_dd;
+            accum_depth_rec = last_alpha * last_depth + (1.f - last_alpha) * accum_depth_rec;
+            last_depth = c_d;
+            dL_dalpha += (c_d - accum_depth_rec) * dd_depth;
+            // the reference adds last_alpha * 1.0 in double precision
+            accum_alpha_rec = (float)((double)last_alpha + (double)__fmul_rn(1.f - last_alpha, accum_alpha_rec));
+            dL_dalpha += (1 - accum_alpha_rec) * dd_accum;
+#pragma unroll
+            for (int ch = 0; ch < 3; ++ch) {
+                accum_normal_rec[ch] = last_alpha * last_normal[ch] + (1.f - last_alpha) * accum_normal_rec[ch];
+                last_normal[ch] = nrm[ch];
+                dL_dalpha += (nrm[ch] - accum_normal_rec[ch]) * dd_normal[ch];
+                v[11 + ch] = alpha * T * dd_normal[ch];
+            }
+            dL_dalpha *= T;
+            last_alpha = alpha;
+            dL_dalpha += (-T_final / (1.f - alpha)) * bg_dot_dpixel;
+            const float dL_dG = r2.w * dL_dalpha;
+            dL_dz += alpha * T * dd_depth;
+            if (h.rho3d <= h.rho2d) {
+                const float dsx = dL_dG * -G * h.sx + dL_dz * r2.x;
+                const float dsy = dL_dG * -G * h.sy + dL_dz * r2.y;
+                const float dsx_pz = dsx / h.p.z, dsy_pz = dsy / h.p.z;
+                const V3 dL_dp = v3(dsx_pz, dsy_pz, -(dsx_pz * h.sx + dsy_pz * h.sy));
+                const V3 dL_dk = vcross(h.l, dL_dp);
+                const V3 dL_dl = vcross(dL_dp, h.k);
+                v[0] = -dL_dk.x; v[1] = -dL_dk.y; v[2] = -dL_dk.z;
+                v[3] = -dL_dl.x; v[4] = -dL_dl.y; v[5] = -dL_dl.z;
+                v[6] = pxf * dL_dk.x + pyf * dL_dl.x + dL_dz * h.sx;
+                v[7] = pxf * dL_dk.y + pyf * dL_dl.y + dL_dz * h.sy;
+                v[8] = pxf * dL_dk.z + pyf * dL_dl.z + dL_dz * 1.0f;
+            } else {
+                const float dG_ddelx = -G * FILTER_INV_SQUARE * h.dx;
+                const float dG_ddely = -G * FILTER_INV_SQUARE * h.dy;
+                v[9] = dL_dG * dG_ddelx;
+                v[10] = dL_dG * dG_ddely;
+                v[6] = h.sx * dL_dz;
+                v[7] = h.sy * dL_dz;
+                v[8] = dL_dz;
+            }
+            v[14] = G * dL_dalpha;
+        };
+        for (int e = 0; e < nl; e += 2) {
+            const int ja = s_list[warp][e], jb = e + 1 < nl ? s_list[warp][e + 1] : -1;
+            Hit ha, hb;
+            float Ga, Gb, aa, ab;
+            const bool ca = evaluate(ja, ha, Ga, aa);
+            bool cb = evaluate(jb >= 0 ? jb : ja, hb, Gb, ab);
+            cb = cb && jb >= 0;
+            const bool wa = __any_sync(0xffffffffu, ca), wb = __any_sync(0xffffffffu, cb);
+            if (!wa && !wb) continue;
+            float va[NGRAD], vb[NGRAD];
+#pragma unroll
+            for (int q = 0; q < NGRAD; ++q) va[q] = vb[q] = 0.f;
+            if (ca) replay(ja, ha, Ga, aa, va);
+            if (cb) replay(jb, hb, Gb, ab, vb);
+            float o[2];
+            warp_reduce_pair(va, vb, o);
+            const int jj = (lane & 16) ? jb : ja;
+            if ((lane & 16) ? wb : wa) {
+                if (slot.count > 0) s_red[jj][warp][slot.base] = o[0];
+                if (slot.count > 1) s_red[jj][warp][slot.base + 1] = o[1];
+                if ((lane & 15) == 0) atomicOr(&s_who[jj], 1u << warp);
             }
         }
         __syncthreads();
-        for (int jj = threadIdx.x; jj < nb; jj += BLOCK) {
-            float s[20];
-#pragma unroll
-            for (int q = 0; q < NGRAD; ++q) {
-                float a = s_red[jj][0][q];
-#pragma unroll
-                for (int w = 1; w < BLOCK / 32; ++w) a += s_red[jj][w][q];
-                s[q] = a;
-            }
-            s[18] = 0.f;
-            s[19] = 0.f;
-            float4* out = partial + (int64_t)PARTIAL_F4 * si[jj];
-#pragma unroll
-            for (int f = 0; f < PARTIAL_F4; ++f) out[f] = make_float4(s[4 * f], s[4 * f + 1], s[4 * f + 2], s[4 * f + 3]);
+        // term q of entry jj: the sums of the warps that replayed it, in warp order
+        for (int i = threadIdx.x; i < nb * 4 * PARTIAL_F4; i += BLOCK) {
+            const int jj = i / (4 * PARTIAL_F4), q = i - jj * (4 * PARTIAL_F4);
+            float a = 0.f;
+            if (q < NGRAD)
+                for (unsigned who = s_who[jj]; who != 0u; who &= who - 1u) a += s_red[jj][__ffs(who) - 1][q];
+            reinterpret_cast<float*>(partial + (int64_t)PARTIAL_F4 * si[jj])[q] = a;
         }
     }
 }
