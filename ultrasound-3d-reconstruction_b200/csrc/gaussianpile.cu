@@ -27,6 +27,7 @@
 #include "us3d_common.cuh"
 #include "scan.cuh"
 #include "binning.cuh"
+#include "stable_bins.cuh"
 
 namespace us3d {
 namespace gp {
@@ -58,7 +59,8 @@ struct Workspace {
     float4* bfp;        // G x 4, what the backward needs of the forward's footprint:
                         // (mu2_lat, mu2_ax, r_lat (< 0: no footprint), r_ax) (inv00, inv01, inv11, bno_const)
                         // (s2_00, s2_01, s2_11, 1 / det_norm) (mu_ele, 1 / denom_ele, dsigma_ele/dax, sigma_ele)
-    unsigned long long* keys;
+    StableScratch stable;    // small bucket grids (stable_bins)
+    unsigned long long* keys;  // the other ones: instances before the sort
     int* slot_inst;
     int* sorted_gid;
     int* sorted_inst;
@@ -80,8 +82,15 @@ static Workspace carve(void* base, int64_t G, int64_t T, int64_t cap) {
     w.bs_t = c.take<long long>((size_t)scan_num_blocks(T) + 1);
     w.cand = c.take<float4>((size_t)G * 3);
     w.bfp = c.take<float4>((size_t)G * 4);
-    w.keys = c.take<unsigned long long>((size_t)cap);
-    w.slot_inst = c.take<int>((size_t)cap);
+    if (stable_bins(G, T, false)) {
+        w.stable = stable_carve(c, G, T, true);
+        w.keys = nullptr;
+        w.slot_inst = nullptr;
+    } else {
+        w.stable = {};
+        w.keys = c.take<unsigned long long>((size_t)cap);
+        w.slot_inst = c.take<int>((size_t)cap);
+    }
     w.sorted_gid = c.take<int>((size_t)cap);
     w.sorted_inst = c.take<int>((size_t)cap);
     w.bytes = align_up(c.off, 256);
@@ -352,16 +361,6 @@ preprocess_kernel(int64_t G, int H, int W, int tile, int tiles_x, int tiles_y, f
         bfp[4 * g + 3] = make_float4(Ff.mu_ele, 1.f / denom_ele, dse_dax, Ff.sigma_ele);
     }
 }
-
-__global__ void check_kernel(long long* __restrict__ header, int64_t cap) {
-    const long long tg = header[H_SCAN_G], tt = header[H_SCAN_T];
-    long long flags = header[H_FLAGS];
-    if (tg != tt) flags |= FLAG_TABLE;
-    if (tg > cap || tg > 0x7fffffffLL) flags |= FLAG_OVERFLOW;
-    header[H_TOTAL] = tg;
-    header[H_FLAGS] = flags;
-}
-
 
 // ------------------------------------------------------------------------------------
 // Forward
@@ -1068,7 +1067,7 @@ __global__ void export_kernel(int T, const int* __restrict__ tile_start, const i
 using namespace us3d;
 using namespace us3d::gp;
 
-static bool g_gp_sort_attr[128];
+static BinAttr g_gp_sort_attr;
 
 static int gp_sizes(int H, int W, int tile, int* tx, int* ty) {
     US3D_CHECK_ARG(H > 0 && W > 0, "H/W must be positive");
@@ -1117,14 +1116,9 @@ extern "C" int us3d_gp_forward(void* workspace, size_t workspace_bytes, int64_t 
                                                   intensities, pose, grid_pack, focus_params, w.rects, w.dkey,
                                                   w.touched, w.tile_count, w.cand, w.bfp);
     US3D_CHECK_LAUNCH("gp preprocess");
-    US3D_CHECK_CUDA(launch_rect_count(n_gauss, tx, T, RectOf4{w.rects}, w.tile_count, stream));
-    US3D_CHECK_CUDA(exclusive_scan(w.touched, n_gauss, w.inst_offset, w.bs_g, w.header + H_SCAN_G, stream));
-    US3D_CHECK_CUDA(exclusive_scan(w.tile_count, T, w.tile_start, w.bs_t, w.header + H_SCAN_T, stream));
-    check_kernel<<<1, 1, 0, stream>>>(w.header, cap);
-    US3D_CHECK_CUDA(launch_rect_scatter(n_gauss, tx, T, RectOf4{w.rects}, w.dkey, w.inst_offset, w.tile_start,
-                                        w.tile_cursor, w.header, w.keys, w.slot_inst, stream));
-    US3D_CHECK_CUDA(launch_tile_sort(T, n_gauss, w.tile_start, w.header, w.keys, w.slot_inst, w.sorted_gid, w.sorted_inst,
-                                     g_gp_sort_attr, stream));
+    US3D_CHECK_CUDA(launch_bins(n_gauss, tx, T, RectOf4{w.rects}, sort_by_v ? w.dkey : nullptr, w.touched, w.stable, w.tile_count,
+                                w.tile_start, w.tile_cursor, w.inst_offset, w.bs_g, w.bs_t, w.header, cap, w.keys, w.slot_inst,
+                                w.sorted_gid, w.sorted_inst, g_gp_sort_attr, stream));
     // up to four threads per pixel (a whole-warp pixel block of at most 1024 threads); frames
     // with fewer than four tiles per SM split each tile over four blocks when it divides into
     // whole warps
@@ -1142,7 +1136,7 @@ extern "C" int us3d_gp_forward(void* workspace, size_t workspace_bytes, int64_t 
         split4 ? launch(forward_kernel<1, 4>, 1, 4) : launch(forward_kernel<1, 1>, 1, 1);
     US3D_CHECK_LAUNCH("gp forward");
     prof_end(prof, stream);
-    count_launches(1 + (n_gauss > 0) * 3 + 6 + 1 + tile_sort_launches(n_gauss) + 1);
+    count_launches(1 + (n_gauss > 0) + bins_launches(n_gauss, w.keys == nullptr, sort_by_v != 0) + 1);
     return US3D_OK;
 }
 

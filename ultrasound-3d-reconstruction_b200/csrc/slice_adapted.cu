@@ -17,6 +17,7 @@
 #include "us3d_common.cuh"
 #include "scan.cuh"
 #include "binning.cuh"
+#include "stable_bins.cuh"
 
 namespace us3d {
 namespace sa {
@@ -38,7 +39,8 @@ struct Workspace {
     int* tile_start;
     int* tile_cursor;
     long long* bs_t;
-    unsigned long long* keys;
+    StableScratch stable;    // small bucket grids (stable_bins)
+    unsigned long long* keys;  // the other ones: instances before the sort
     int* slot_inst;
     int* sorted_gid;
     int* sorted_inst;
@@ -63,8 +65,15 @@ static Workspace carve(void* base, int64_t N, int64_t T, int64_t cap) {
     w.tile_start = c.take<int>((size_t)T + 1);
     w.tile_cursor = c.take<int>((size_t)T);
     w.bs_t = c.take<long long>((size_t)scan_num_blocks(T) + 1);
-    w.keys = c.take<unsigned long long>((size_t)cap);
-    w.slot_inst = c.take<int>((size_t)cap);
+    if (stable_bins(N, T, false)) {
+        w.stable = stable_carve(c, N, T, false);
+        w.keys = nullptr;
+        w.slot_inst = nullptr;
+    } else {
+        w.stable = {};
+        w.keys = c.take<unsigned long long>((size_t)cap);
+        w.slot_inst = c.take<int>((size_t)cap);
+    }
     w.sorted_gid = c.take<int>((size_t)cap);
     w.sorted_inst = c.take<int>((size_t)cap);
     w.fwd_part = c.take<float4>(frame_split(T) > 1 ? (size_t)frame_split(T) * T * TILE * TILE : 0);
@@ -131,16 +140,6 @@ preprocess_kernel(int64_t N, int H, int W, int gw, int gh, float hw, float hh, f
     touched[g] = (x1 - x0) * (y1 - y0);
     (void)tile_count;  // counted per block by rect_count_kernel
 }
-
-__global__ void check_kernel(long long* __restrict__ header, int64_t cap) {
-    const long long tg = header[H_SCAN_G], tt = header[H_SCAN_T];
-    long long flags = header[H_FLAGS];
-    if (tg != tt) flags |= FLAG_TABLE;
-    if (tg > cap || tg > 0x7fffffffLL) flags |= FLAG_OVERFLOW;
-    header[H_TOTAL] = tg;
-    header[H_FLAGS] = flags;
-}
-
 
 // One block of 16x16 threads per tile and list range, staged Gaussians, per-pixel sums in
 // tile-list order (reference render.cu:354-426). With split > 1 the tile's list is cut into
@@ -511,7 +510,7 @@ dense_backward_kernel(int64_t P, int64_t N, const float2* __restrict__ pixels, c
 using namespace us3d;
 using namespace us3d::sa;
 
-static bool g_sa_sort_attr[128];
+static BinAttr g_sa_sort_attr;
 
 static int sa_check(int H, int W, float hw, float hh, float rs, int64_t N, int64_t cap) {
     US3D_CHECK_ARG(H > 0 && W > 0, "image dimensions must be positive");
@@ -555,14 +554,9 @@ extern "C" int us3d_sa_bounded_forward(void* workspace, size_t workspace_bytes, 
     if (n > 0)
         preprocess_kernel<<<gb, 256, 0, stream>>>(n, H, W, gw, gh, half_width, half_height, radius_sigma, m2, iv,
                                                   w.rects, w.bbox, w.touched, w.tile_count);
-    US3D_CHECK_CUDA(launch_rect_count(n, gw, T, RectOf4{w.rects}, w.tile_count, stream));
-    US3D_CHECK_CUDA(exclusive_scan(w.touched, n, w.inst_offset, w.bs_g, w.header + H_SCAN_G, stream));
-    US3D_CHECK_CUDA(exclusive_scan(w.tile_count, T, w.tile_start, w.bs_t, w.header + H_SCAN_T, stream));
-    check_kernel<<<1, 1, 0, stream>>>(w.header, cap);
-    US3D_CHECK_CUDA(launch_rect_scatter(n, gw, T, RectOf4{w.rects}, nullptr, w.inst_offset, w.tile_start,
-                                        w.tile_cursor, w.header, w.keys, w.slot_inst, stream));
-    US3D_CHECK_CUDA(launch_tile_sort(T, n, w.tile_start, w.header, w.keys, w.slot_inst, w.sorted_gid, w.sorted_inst,
-                                     g_sa_sort_attr, stream));
+    US3D_CHECK_CUDA(launch_bins(n, gw, T, RectOf4{w.rects}, nullptr, w.touched, w.stable, w.tile_count,
+                                w.tile_start, w.tile_cursor, w.inst_offset, w.bs_g, w.bs_t, w.header, cap, w.keys, w.slot_inst,
+                                w.sorted_gid, w.sorted_inst, g_sa_sort_attr, stream));
     const int split = frame_split(T);
     forward_kernel<<<(unsigned)(T * split), TILE * TILE, 0, stream>>>(
         split, H, W, gw, half_width, half_height, radius_sigma, m2, iv, weights, colors, w.tile_start, w.sorted_gid,
@@ -574,7 +568,7 @@ extern "C" int us3d_sa_bounded_forward(void* workspace, size_t workspace_bytes, 
         US3D_CHECK_LAUNCH("sa forward combine");
     }
     prof_end(prof, stream);
-    count_launches(1 + 3 * (n > 0) + 6 + 1 + tile_sort_launches(n) + 1 + (split > 1));
+    count_launches(1 + (n > 0) + bins_launches(n, w.keys == nullptr, false) + 1 + (split > 1));
     return US3D_OK;
 }
 

@@ -27,6 +27,7 @@
 #include "us3d_common.cuh"
 #include "scan.cuh"
 #include "binning.cuh"
+#include "stable_bins.cuh"
 #include "f32x2.cuh"
 
 namespace us3d {
@@ -50,7 +51,8 @@ struct Workspace {
     int* ray_cursor;    // W
     long long* bs_t;
     float4* rec;        // G x 7
-    unsigned long long* keys;
+    StableScratch stable;    // small bucket grids (stable_bins)
+    unsigned long long* keys;  // the other ones: instances before the sort
     int* slot_inst;
     int* sorted_gid;
     int* sorted_inst;
@@ -87,8 +89,15 @@ static Workspace carve(void* base, int64_t G, int64_t W, int64_t P, int64_t cap)
     w.ray_cursor = c.take<int>((size_t)W);
     w.bs_t = c.take<long long>((size_t)scan_num_blocks(W) + 1);
     w.rec = c.take<float4>((size_t)G * REC_F4);
-    w.keys = c.take<unsigned long long>((size_t)cap);
-    w.slot_inst = c.take<int>((size_t)cap);
+    if (stable_bins(G, W, true)) {
+        w.stable = stable_carve(c, G, W, true);
+        w.keys = nullptr;
+        w.slot_inst = nullptr;
+    } else {
+        w.stable = {};
+        w.keys = c.take<unsigned long long>((size_t)cap);
+        w.slot_inst = c.take<int>((size_t)cap);
+    }
     w.sorted_gid = c.take<int>((size_t)cap);
     w.sorted_inst = c.take<int>((size_t)cap);
     w.pixel_state = c.take<float4>((size_t)P);
@@ -298,16 +307,6 @@ preprocess_kernel(int64_t G, int W, float pixel_spacing, float col_off, float ne
     dkey[g] = f32_to_u32_sat(fmaxf(0.0f, pz) * 1000.0f);
     (void)ray_count;  // counted per block by rect_count_kernel
 }
-
-__global__ void check_kernel(long long* __restrict__ header, int64_t cap) {
-    const long long tg = header[H_SCAN_G], tt = header[H_SCAN_T];
-    long long flags = header[H_FLAGS];
-    if (tg != tt) flags |= FLAG_TABLE;
-    if (tg > cap || tg > 0x7fffffffLL) flags |= FLAG_OVERFLOW;
-    header[H_TOTAL] = tg;
-    header[H_FLAGS] = flags;
-}
-
 
 // ------------------------------------------------------------------------------------
 // Forward
@@ -1462,7 +1461,7 @@ reduce_kernel(int64_t G, const int* __restrict__ inst_offset, const long long* _
 }
 
 // Reference-format CSR of the ray binning (MapperForwardCUDA outputs, wrapper_mapper.cu:119-127).
-__global__ void export_kernel(int W, const int* __restrict__ ray_start, const unsigned long long* __restrict__ keys,
+__global__ void export_kernel(int W, const int* __restrict__ ray_start, const uint32_t* __restrict__ dkey,
                               const int* __restrict__ sorted_gid, int* __restrict__ counts, int* __restrict__ offsets,
                               int* __restrict__ indices, float* __restrict__ depths) {
     const int x = blockIdx.x;
@@ -1474,7 +1473,7 @@ __global__ void export_kernel(int W, const int* __restrict__ ray_start, const un
     }
     for (int s = s0 + threadIdx.x; s < s1; s += blockDim.x) {
         indices[s] = sorted_gid[s];
-        depths[s] = ((float)(uint32_t)(keys[s] >> 32)) * 0.001f;
+        depths[s] = ((float)dkey[sorted_gid[s]]) * 0.001f;
     }
 }
 
@@ -1484,7 +1483,7 @@ __global__ void export_kernel(int W, const int* __restrict__ ray_start, const un
 using namespace us3d;
 using namespace us3d::ugr;
 
-static bool g_ugr_sort_attr[128];
+static BinAttr g_ugr_sort_attr;
 
 // The transmittance checkpoints apply with a quadrature window (its far factor is constant) and
 // full transmission (the local-window mode bounds the product differently); forward and
@@ -1535,17 +1534,12 @@ extern "C" int us3d_ugr_forward(void* workspace, size_t workspace_bytes, int64_t
                                                   axis_lat, axis_ele, axis_ax, w.ray_range, w.dkey, w.touched,
                                                   w.ray_count, w.rec);
     US3D_CHECK_LAUNCH("ugr preprocess");
-    US3D_CHECK_CUDA(launch_rect_count(n_gauss, W, W, RangeOf2{w.ray_range}, w.ray_count, stream));
-    US3D_CHECK_CUDA(exclusive_scan(w.touched, n_gauss, w.inst_offset, w.bs_g, w.header + H_SCAN_G, stream));
-    US3D_CHECK_CUDA(exclusive_scan(w.ray_count, W, w.ray_start, w.bs_t, w.header + H_SCAN_T, stream));
-    check_kernel<<<1, 1, 0, stream>>>(w.header, cap);
-    US3D_CHECK_CUDA(launch_rect_scatter(n_gauss, W, W, RangeOf2{w.ray_range}, w.dkey, w.inst_offset, w.ray_start,
-                                        w.ray_cursor, w.header, w.keys, w.slot_inst, stream));
-    US3D_CHECK_CUDA(launch_tile_sort(W, n_gauss, w.ray_start, w.header, w.keys, w.slot_inst, w.sorted_gid, w.sorted_inst,
-                                     g_ugr_sort_attr, stream));
+    US3D_CHECK_CUDA(launch_bins(n_gauss, W, W, RangeOf2{w.ray_range}, w.dkey, w.touched, w.stable, w.ray_count,
+                                w.ray_start, w.ray_cursor, w.inst_offset, w.bs_g, w.bs_t, w.header, cap, w.keys, w.slot_inst,
+                                w.sorted_gid, w.sorted_inst, g_ugr_sort_attr, stream));
     const unsigned tiles_y = (unsigned)((H + FWD_SAMPLES - 1) / FWD_SAMPLES);
     const int* ckpt_rays = nullptr;
-    int launches = 1 + 3 * (n_gauss > 0) + 6 + 1 + tile_sort_launches(n_gauss) + 1;
+    int launches = 1 + (n_gauss > 0) + bins_launches(n_gauss, w.keys == nullptr, true) + 1;
     if (uses_checkpoints(H, quadrature_window_radius_mm, local_window_only)) {
         const unsigned by = per_ray_blocks(W);
         ray_depth_kernel<<<(unsigned)W, 256, 0, stream>>>(W, H, w.header, pixel_positions, ray_origins, ray_dirs,
@@ -1638,7 +1632,7 @@ extern "C" int us3d_ugr_export_csr(const void* workspace, int64_t n_gauss, int32
                                    float* out_sorted_depths, void* stream_) {
     US3D_CHECK_ARG(workspace && out_counts && out_offsets && W > 0, "bad argument");
     const Workspace w = carve(const_cast<void*>(workspace), n_gauss, W, (int64_t)W * H, cap);
-    export_kernel<<<(unsigned)W, 256, 0, (cudaStream_t)stream_>>>(W, w.ray_start, w.keys, w.sorted_gid, out_counts,
+    export_kernel<<<(unsigned)W, 256, 0, (cudaStream_t)stream_>>>(W, w.ray_start, w.dkey, w.sorted_gid, out_counts,
                                                                   out_offsets, out_indices, out_sorted_depths);
     US3D_CHECK_LAUNCH("ugr export");
     count_launches(1);
