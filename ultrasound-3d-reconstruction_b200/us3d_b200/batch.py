@@ -121,7 +121,7 @@ class GraphedTrainingStep:
 
 LAUNCH_SHAPES = [(b, t) for b in (128, 256, 512) for t in (128, 256)]
 BACKWARD_VARIANTS = (0, 1)  # one pixel per FP32 instruction / two pixels per packed FP32 pair
-FORWARD_VARIANTS = (0, 1)   # one pixel per thread / two pixels per thread in packed FP32 pairs
+FORWARD_VARIANTS = (0,)     # one kernel; set_forward_variant(1) is accepted and launches the same
 
 
 def get_forward_variant() -> int:
@@ -204,8 +204,6 @@ def autotune_launch(frames: UG.FrameTable, params, pixels: torch.Tensor, reps: i
         for variant in BACKWARD_VARIANTS:
             set_backward_variant(variant)
             for shape in LAUNCH_SHAPES:
-                if fvariant == 1 and shape[0] == 512:
-                    continue  # the packed forward stages at most 256 Gaussians (same as 256)
                 set_launch_config(*shape)
                 step()
                 torch.cuda.synchronize(pixels.device)
