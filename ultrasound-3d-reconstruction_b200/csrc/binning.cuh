@@ -517,10 +517,13 @@ tile_sort_huge_kernel(int64_t T, const int* __restrict__ tile_start, const long 
 constexpr int SORT_PACKED_THREADS = 256;
 constexpr int SORT_PACKED_MIN_BLOCKS = 7;
 
+// count, cursor (NULL: not checked): every bucket must have been filled exactly as counted; otherwise
+// later kernels see a flag.
 template <bool PACKED>
 static __global__ void __launch_bounds__(PACKED ? SORT_PACKED_THREADS : SORT_THREADS,
                                          PACKED ? SORT_PACKED_MIN_BLOCKS : SORT_MIN_BLOCKS)
-tile_sort_kernel(int64_t T, const int* __restrict__ tile_start, const long long* __restrict__ header,
+tile_sort_kernel(int64_t T, const int* __restrict__ tile_start, long long* header, const int* __restrict__ count,
+                 const int* __restrict__ cursor,
                  unsigned long long* __restrict__ keys, const int* __restrict__ slot_inst,
                  int* __restrict__ sorted_gid, int* __restrict__ sorted_inst,
                  const uint16_t* __restrict__ slot_mask, uint16_t* __restrict__ sorted_mask) {
@@ -530,6 +533,11 @@ tile_sort_kernel(int64_t T, const int* __restrict__ tile_start, const long long*
     if (t >= T || header[H_FLAGS] != 0) return;
     const int s0 = tile_start[t];
     const int n = tile_start[t + 1] - s0;
+    if (count != nullptr && cursor[t] != count[t]) {
+        if (threadIdx.x == 0)
+            atomicOr(reinterpret_cast<unsigned long long*>(header + H_FLAGS), (unsigned long long)FLAG_TABLE);
+        return;
+    }
     if (n <= 0) return;
     if (n <= SORT_SMEM_CAP) {
         if constexpr (PACKED)
@@ -639,19 +647,19 @@ static inline bool tile_sort_mid(int64_t n_elems) { return n_elems < SORT_PACK_G
 // shared-memory limit was raised (one array per translation unit, 128 devices). slot_mask /
 // sorted_mask may be NULL.
 static inline cudaError_t launch_tile_sort(int64_t T, int64_t n_elems, const int* tile_start,
-                                           const long long* header, unsigned long long* keys, const int* slot_inst,
+                                           long long* header, unsigned long long* keys, const int* slot_inst,
                                            int* sorted_gid, int* sorted_inst, bool* attr_done, cudaStream_t stream,
-                                           const uint16_t* slot_mask = nullptr,
-                                           uint16_t* sorted_mask = nullptr) {
+                                           const uint16_t* slot_mask = nullptr, uint16_t* sorted_mask = nullptr,
+                                           const int* count = nullptr, const int* cursor = nullptr) {
     if (T <= 0) return cudaSuccess;
     if (n_elems < SORT_PACK_G)
         tile_sort_kernel<true><<<(unsigned)T, SORT_PACKED_THREADS, 0, stream>>>(
-            T, tile_start, header, keys, slot_inst, sorted_gid, sorted_inst, slot_mask, sorted_mask);
+            T, tile_start, header, count, cursor, keys, slot_inst, sorted_gid, sorted_inst, slot_mask, sorted_mask);
     else
         tile_sort_kernel<false><<<(unsigned)T, SORT_THREADS, 0, stream>>>(
-            T, tile_start, header, keys, slot_inst, sorted_gid, sorted_inst, slot_mask, sorted_mask);
+            T, tile_start, header, count, cursor, keys, slot_inst, sorted_gid, sorted_inst, slot_mask, sorted_mask);
     cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess || n_elems <= SORT_SMEM_CAP) return e;  // a bucket holds an element once
     int dev = 0;
     e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -675,11 +683,12 @@ static inline cudaError_t launch_tile_sort(int64_t T, int64_t n_elems, const int
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
+    if (mid && n_elems <= SORT_MID_CAP) return cudaSuccess;
     const unsigned grid = (unsigned)(T < SORT_BIG_GRID ? T : SORT_BIG_GRID);
     tile_sort_big_kernel<<<grid, SORT_BIG_THREADS, tile_sort_big_smem_bytes(), stream>>>(
         T, tile_start, header, keys, slot_inst, sorted_gid, sorted_inst, slot_mask, sorted_mask, mid ? 1 : 0);
     e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+    if (e != cudaSuccess || n_elems <= SORT_BIG_CAP) return e;
     const unsigned hgrid = (unsigned)(T < SORT_HUGE_GRID ? T : SORT_HUGE_GRID);
     tile_sort_huge_kernel<<<hgrid, SORT_HUGE_THREADS, tile_sort_huge_smem_bytes(), stream>>>(
         T, tile_start, header, keys, slot_inst, sorted_gid, sorted_inst, slot_mask, sorted_mask,
@@ -688,6 +697,11 @@ static inline cudaError_t launch_tile_sort(int64_t T, int64_t n_elems, const int
 }
 
 // Kernel launches launch_tile_sort makes for T > 0 tiles over n_elems elements.
-static inline int tile_sort_launches(int64_t n_elems) { return 3 + (tile_sort_mid(n_elems) ? 1 : 0); }
+static inline int tile_sort_launches(int64_t n_elems) {
+    const bool mid = tile_sort_mid(n_elems);
+    if (n_elems <= SORT_SMEM_CAP) return 1;
+    if (mid && n_elems <= SORT_MID_CAP) return 2;
+    return 2 + (mid ? 1 : 0) + (n_elems > SORT_BIG_CAP ? 1 : 0);
+}
 
 }  // namespace us3d

@@ -1136,7 +1136,7 @@ extern "C" int us3d_gp_forward(void* workspace, size_t workspace_bytes, int64_t 
         split4 ? launch(forward_kernel<1, 4>, 1, 4) : launch(forward_kernel<1, 1>, 1, 1);
     US3D_CHECK_LAUNCH("gp forward");
     prof_end(prof, stream);
-    count_launches(1 + (n_gauss > 0) + bins_launches(n_gauss, w.keys == nullptr, sort_by_v != 0) + 1);
+    count_launches(1 + (n_gauss > 0) + bins_launches(n_gauss, T, w.keys == nullptr, sort_by_v != 0) + 1);
     return US3D_OK;
 }
 

@@ -568,7 +568,7 @@ extern "C" int us3d_sa_bounded_forward(void* workspace, size_t workspace_bytes, 
         US3D_CHECK_LAUNCH("sa forward combine");
     }
     prof_end(prof, stream);
-    count_launches(1 + (n > 0) + bins_launches(n, w.keys == nullptr, false) + 1 + (split > 1));
+    count_launches(1 + (n > 0) + bins_launches(n, T, w.keys == nullptr, false) + 1 + (split > 1));
     return US3D_OK;
 }
 

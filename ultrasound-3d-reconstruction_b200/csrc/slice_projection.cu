@@ -294,7 +294,7 @@ extern "C" int us3d_sa_project(void* workspace, size_t workspace_bytes, int64_t 
         compact_kernel<<<gb, 256, 0, stream>>>(p, (int)n_gauss, w.flags, w.offsets, out_means2d, out_inv2d,
                                                out_weights, out_colors, out_keep_idx, out_keep_mask);
     US3D_CHECK_LAUNCH("sa project");
-    count_launches(3 + 2 * (n_gauss > 0));
+    count_launches(scan_launches(n_gauss) + 2 * (n_gauss > 0));
     if (out_kept) {
         long long k = 0;
         US3D_CHECK_CUDA(cudaMemcpyAsync(&k, w.total, sizeof(k), cudaMemcpyDeviceToHost, stream));

@@ -354,15 +354,20 @@ static inline cudaError_t launch_chunk_fill(int64_t n, int gx, int64_t n_buckets
     return cudaGetLastError();
 }
 
-// Totals of the two scans agree (FLAG_TABLE otherwise) and fit the capacity (FLAG_OVERFLOW).
-static __global__ void bins_check_kernel(long long* __restrict__ header, int64_t cap) {
-    const long long tg = header[H_SCAN_G], tt = header[H_SCAN_T];
-    long long flags = header[H_FLAGS];
-    if (tg != tt) flags |= FLAG_TABLE;
-    if (tg > cap || tg > 0x7fffffffLL) flags |= FLAG_OVERFLOW;
-    header[H_TOTAL] = tg;
-    header[H_FLAGS] = flags;
-}
+// After the scan of the bucket counts: its total must be that of the elements' instances (FLAG_TABLE
+// otherwise) and fit the capacity (FLAG_OVERFLOW).
+struct BinsEnd {
+    long long* header;
+    int64_t cap;
+    __device__ __forceinline__ void operator()(long long tt) const {
+        const long long tg = header[H_SCAN_G];
+        long long flags = header[H_FLAGS];
+        if (tg != tt) flags |= FLAG_TABLE;
+        if (tg > cap || tg > 0x7fffffffLL) flags |= FLAG_OVERFLOW;
+        header[H_TOTAL] = tg;
+        header[H_FLAGS] = flags;
+    }
+};
 
 // Per-device flags of raised shared-memory limits (one object per translation unit).
 struct BinAttr {
@@ -389,9 +394,9 @@ static inline cudaError_t launch_bins(int64_t n, int gx, int64_t n_buckets, Rect
         e = launch_rect_count(n, gx, n_buckets, rect, count, stream);
     }
     if (e != cudaSuccess) return e;
-    e = exclusive_scan(count, n_buckets, start, bs_t, header + H_SCAN_T, stream);
+    e = exclusive_scan(count, n_buckets, start, bs_t, header + H_SCAN_T, stream, ScanLen{n_buckets},
+                       BinsEnd{header, cap});
     if (e != cudaSuccess) return e;
-    bins_check_kernel<<<1, 1, 0, stream>>>(header, cap);
     if (fill)
         return launch_chunk_fill(n, gx, n_buckets, rect, order, stable, inst_offset, start, header, sorted_gid,
                                  sorted_inst, attr.fill, stream);
@@ -401,9 +406,10 @@ static inline cudaError_t launch_bins(int64_t n, int gx, int64_t n_buckets, Rect
 }
 
 // Kernel launches launch_bins makes.
-static inline int bins_launches(int64_t n, bool fill, bool keyed) {
-    if (fill) return 3 + (keyed ? order_launches(n) : 0) + 2 + 3 + 1 + (n > 0);
-    return 3 + 2 * (n > 0) + 3 + 1 + tile_sort_launches(n);
+static inline int bins_launches(int64_t n, int64_t n_buckets, bool fill, bool keyed) {
+    const int scans = scan_launches(n) + scan_launches(n_buckets);
+    if (fill) return scans + (keyed ? order_launches(n) : 0) + 2 + (n > 0);
+    return scans + 2 * (n > 0) + tile_sort_launches(n);
 }
 
 }  // namespace us3d

@@ -1539,7 +1539,7 @@ extern "C" int us3d_ugr_forward(void* workspace, size_t workspace_bytes, int64_t
                                 w.sorted_gid, w.sorted_inst, g_ugr_sort_attr, stream));
     const unsigned tiles_y = (unsigned)((H + FWD_SAMPLES - 1) / FWD_SAMPLES);
     const int* ckpt_rays = nullptr;
-    int launches = 1 + (n_gauss > 0) + bins_launches(n_gauss, w.keys == nullptr, true) + 1;
+    int launches = 1 + (n_gauss > 0) + bins_launches(n_gauss, W, w.keys == nullptr, true) + 1;
     if (uses_checkpoints(H, quadrature_window_radius_mm, local_window_only)) {
         const unsigned by = per_ray_blocks(W);
         ray_depth_kernel<<<(unsigned)W, 256, 0, stream>>>(W, H, w.header, pixel_positions, ray_origins, ray_dirs,
