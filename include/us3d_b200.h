@@ -202,6 +202,37 @@ US3D_API int us3d_ug_backward(void* workspace, const us3d_slice_frame* frames_de
                      float* d_means, float* d_precision_tril, float* d_opacities,
                      float* d_intensities, void* stream);
 
+/* us3d_ug_backward with d_alpha and d_depth optional: NULL stands for zeros. */
+US3D_API int us3d_ug_backward_ex(void* workspace, const us3d_slice_frame* frames_dev, int32_t n_frames,
+                     int64_t n_tiles, int64_t n_pixels, int64_t n_gauss,
+                     int64_t instance_capacity, const float* pixel_positions, const float* d_image,
+                     const float* d_alpha, const float* d_depth, const float* saved_alpha,
+                     float chi2_threshold, float diag_beta, float bg_alpha,
+                     float bg_intensity, void* scratch, size_t scratch_bytes,
+                     float* d_means, float* d_precision_tril, float* d_opacities,
+                     float* d_intensities, void* stream);
+
+/* us3d_ug_bin_ex followed by us3d_ug_forward, returning the instance total, the number of (Gaussian, frame)
+ * pairs that survived the cull and the flags: waits for the binning on the host, not for the
+ * shading, which is queued meanwhile. With nonzero flags the outputs are not written. Refused under
+ * capture. */
+US3D_API int us3d_ug_bin_forward(void* workspace, size_t workspace_bytes, const us3d_slice_frame* frames_dev,
+                                 int32_t n_frames, int64_t n_tiles, int64_t n_pixels, int64_t n_gauss,
+                                 const float* means, const float* precision_tril, const float* opacities,
+                                 const float* intensities, float chi2_threshold, float diag_beta,
+                                 int32_t sort_by_depth, int64_t instance_capacity, const float* pixel_positions,
+                                 int32_t flags, float bg_alpha, float bg_intensity, float* out_image,
+                                 float* out_alpha, float* out_depth, int32_t* out_counts,
+                                 int64_t* total_instances, int64_t* total_tasks, int32_t* status_flags,
+                                 void* stream);
+
+/* Writes the table entry of a single frame (height x width, all Gaussians) whose origin and axes, three
+ * floats each, are on the device. */
+US3D_API int us3d_ug_frame_table(us3d_slice_frame* frame_dev, const float* origin, const float* axis_lat,
+                                 const float* axis_ax, const float* axis_ele, float lateral_spacing,
+                                 float axial_spacing, float axial_near, float lateral_col_offset,
+                                 int32_t height, int32_t width, void* stream);
+
 /*
  * Launch shapes of the UltraGauss shading kernels, process-wide (read at every launch; set
  * them before capturing a CUDA graph): Gaussians staged per forward batch (128, 256 or 512)
@@ -394,6 +425,15 @@ US3D_API int us3d_gp_forward(void* workspace, size_t workspace_bytes, int64_t n_
                              const float* focus_params, int32_t height, int32_t width, float lateral_spacing,
                              float axial_spacing, float axial_near, int32_t tile_size, float k_sigma,
                              int32_t sort_by_v, int64_t instance_capacity, float* out_image, void* stream);
+/* us3d_gp_forward, returning its instance total and flags as us3d_gp_read_status does: waits
+ * for the binning on the host, not for the shading, which is queued meanwhile. Refused under capture. */
+US3D_API int us3d_gp_forward_checked(void* workspace, size_t workspace_bytes, int64_t n_gauss, const float* means,
+                                     const float* scales, const float* quats, const float* opacities,
+                                     const float* intensities, const float* pose, const float* grid_pack,
+                                     const float* focus_params, int32_t height, int32_t width, float lateral_spacing,
+                                     float axial_spacing, float axial_near, int32_t tile_size, float k_sigma,
+                                     int32_t sort_by_v, int64_t instance_capacity, float* out_image,
+                                     int64_t* total_instances, int32_t* flags, void* stream);
 
 /* Instance total and flags of the last us3d_gp_forward (SYNCHRONISES `stream`). */
 US3D_API int us3d_gp_read_status(const void* workspace, int64_t* total_instances, int32_t* overflow,
@@ -447,6 +487,14 @@ US3D_API int us3d_sa_bounded_forward(void* workspace, size_t workspace_bytes, in
                                      const float* inv2d, const float* weights, const float* colors,
                                      float radius_sigma, int64_t instance_capacity, float* out_image,
                                      float* out_alpha, void* stream);
+/* us3d_sa_bounded_forward, returning its instance total and flags as us3d_sa_read_status does: waits
+ * for the binning on the host, not for the shading, which is queued meanwhile. Refused under capture. */
+US3D_API int us3d_sa_bounded_forward_checked(void* workspace, size_t workspace_bytes, int64_t n, int32_t height,
+                                             int32_t width, float half_width, float half_height, const float* means2d,
+                                             const float* inv2d, const float* weights, const float* colors,
+                                             float radius_sigma, int64_t instance_capacity, float* out_image,
+                                             float* out_alpha, int64_t* total_instances, int32_t* flags,
+                                             void* stream);
 US3D_API int us3d_sa_read_status(const void* workspace, int64_t* total_instances, int32_t* overflow,
                                  void* stream);
 /* Replaces bounded_backward (render.cu:923-1013): gradients w.r.t. means2d (N,2),
@@ -528,6 +576,18 @@ US3D_API int us3d_ugr_forward(void* workspace, size_t workspace_bytes, int64_t n
                               float quadrature_window_radius_mm, int32_t local_transmission_window_only,
                               float local_transmission_max_window_mm, int64_t instance_capacity,
                               float* out_image, void* stream);
+/* us3d_ugr_forward, returning its instance total and flags as us3d_ugr_read_status does: waits
+ * for the binning on the host, not for the shading, which is queued meanwhile. Refused under capture. */
+US3D_API int us3d_ugr_forward_checked(void* workspace, size_t workspace_bytes, int64_t n_gauss, const float* means,
+                                      const float* scales, const float* quats, const float* attenuations,
+                                      const float* sh_coeffs, const float* pixel_positions, const float* ray_origins,
+                                      const float* ray_dirs, const float* origin, const float* axis_lateral,
+                                      const float* axis_elevational, const float* axis_axial,
+                                      const float* ray_perturbations, int32_t width, int32_t height, float width_mm,
+                                      float near_mm, float lateral_col_offset, float elev_cutoff_mm, float k_sigma,
+                                      float quadrature_window_radius_mm, int32_t local_transmission_window_only,
+                                      float local_transmission_max_window_mm, int64_t instance_capacity,
+                                      float* out_image, int64_t* total_instances, int32_t* flags, void* stream);
 /* Synchronises `stream`: instance total and overflow flags of the last us3d_ugr_forward. */
 US3D_API int us3d_ugr_read_status(const void* workspace, int64_t* total_instances, int32_t* overflow,
                                   void* stream);
@@ -576,6 +636,16 @@ US3D_API int us3d_gs_forward(void* workspace, size_t workspace_bytes, int64_t n_
                              const float* projmatrix, const float* campos, int32_t prefiltered,
                              int64_t instance_capacity, float* out_color, float* out_others, int32_t* out_radii,
                              void* stream);
+/* us3d_gs_forward, returning its instance total and flags as us3d_gs_read_status does: waits
+ * for the binning on the host, not for the shading, which is queued meanwhile. Refused under capture. */
+US3D_API int us3d_gs_forward_checked(void* workspace, size_t workspace_bytes, int64_t n_gauss, int32_t sh_degree,
+                                     int32_t sh_coeffs, const float* background, int32_t width, int32_t height,
+                                     const float* means3D, const float* shs, const float* colors_precomp,
+                                     const float* opacities, const float* scales, float scale_modifier,
+                                     const float* rotations, const float* transmat_precomp, const float* viewmatrix,
+                                     const float* projmatrix, const float* campos, int32_t prefiltered,
+                                     int64_t instance_capacity, float* out_color, float* out_others,
+                                     int32_t* out_radii, int64_t* total_instances, int32_t* flags, void* stream);
 /* Synchronises `stream`: instance total and flags (1 overflow, 2 table, 4 prefiltered). */
 US3D_API int us3d_gs_read_status(const void* workspace, int64_t* total_instances, int32_t* flags, void* stream);
 /* Replaces RasterizeGaussiansBackwardCUDA (rasterize_points.cu:135-233). Gradient outputs

@@ -23,6 +23,18 @@ constexpr unsigned long long SORT_PAD_KEY = ~0ull;
 
 // Header words at the start of a binned workspace.
 enum { H_TOTAL = 0, H_FLAGS = 1, H_SCAN_G = 2, H_SCAN_T = 3, H_CAP = 4, H_G = 5, H_T = 6, H_P = 7, H_MODE = 8, H_NTASK = 9, H_WORDS = 16 };
+static_assert(H_WORDS == STATUS_WORDS, "a status read copies the whole header");
+
+// Waits for a forward call's status words.
+static inline int wait_status(StatusRead& status, int64_t* total, int32_t* flags, int64_t* n_tasks = nullptr) {
+    long long hdr[STATUS_WORDS];
+    const int st = status.wait(hdr);
+    if (st != US3D_OK) return st;
+    if (total) *total = hdr[H_TOTAL];
+    if (flags) *flags = (int32_t)hdr[H_FLAGS];
+    if (n_tasks) *n_tasks = hdr[H_NTASK];
+    return US3D_OK;
+}
 enum { FLAG_OVERFLOW = 1, FLAG_TABLE = 2 };
 
 static __device__ __forceinline__ void cswap(unsigned long long* k, int* v, int a, int b) {

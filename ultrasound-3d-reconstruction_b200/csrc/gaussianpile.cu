@@ -1089,12 +1089,12 @@ extern "C" size_t us3d_gp_backward_scratch_bytes(int64_t n_gauss, int64_t cap) {
     return (size_t)cap * PARTIAL_F4 * sizeof(float4) + (size_t)(n_gauss + 2) * 12 * sizeof(float) + 256;
 }
 
-extern "C" int us3d_gp_forward(void* workspace, size_t workspace_bytes, int64_t n_gauss, const float* means,
-                               const float* scales, const float* quats, const float* opacities,
-                               const float* intensities, const float* pose, const float* grid_pack,
-                               const float* focus_params, int32_t H, int32_t W, float lateral_spacing,
-                               float axial_spacing, float axial_near, int32_t tile_size, float k_sigma,
-                               int32_t sort_by_v, int64_t cap, float* out_image, void* stream_) {
+static int gp_forward_impl(void* workspace, size_t workspace_bytes, int64_t n_gauss, const float* means,
+                           const float* scales, const float* quats, const float* opacities, const float* intensities,
+                           const float* pose, const float* grid_pack, const float* focus_params, int32_t H, int32_t W,
+                           float lateral_spacing, float axial_spacing, float axial_near, int32_t tile_size,
+                           float k_sigma, int32_t sort_by_v, int64_t cap, float* out_image, StatusRead* status,
+                           void* stream_) {
     int tx, ty;
     int st = gp_sizes(H, W, tile_size, &tx, &ty);
     if (st != US3D_OK) return st;
@@ -1119,6 +1119,10 @@ extern "C" int us3d_gp_forward(void* workspace, size_t workspace_bytes, int64_t 
     US3D_CHECK_CUDA(launch_bins(n_gauss, tx, T, RectOf4{w.rects}, sort_by_v ? w.dkey : nullptr, w.touched, w.stable, w.tile_count,
                                 w.tile_start, w.tile_cursor, w.inst_offset, w.bs_g, w.bs_t, w.header, cap, w.keys, w.slot_inst,
                                 w.sorted_gid, w.sorted_inst, g_gp_sort_attr, stream));
+    if (status != nullptr) {
+        const int rc = status->record(w.header, stream);
+        if (rc != US3D_OK) return rc;
+    }
     // up to four threads per pixel (a whole-warp pixel block of at most 1024 threads); frames
     // with fewer than four tiles per SM split each tile over four blocks when it divides into
     // whole warps
@@ -1138,6 +1142,31 @@ extern "C" int us3d_gp_forward(void* workspace, size_t workspace_bytes, int64_t 
     prof_end(prof, stream);
     count_launches(1 + (n_gauss > 0) + bins_launches(n_gauss, T, w.keys == nullptr, sort_by_v != 0) + 1);
     return US3D_OK;
+}
+
+extern "C" int us3d_gp_forward(void* workspace, size_t workspace_bytes, int64_t n_gauss, const float* means,
+                               const float* scales, const float* quats, const float* opacities,
+                               const float* intensities, const float* pose, const float* grid_pack,
+                               const float* focus_params, int32_t H, int32_t W, float lateral_spacing,
+                               float axial_spacing, float axial_near, int32_t tile_size, float k_sigma,
+                               int32_t sort_by_v, int64_t cap, float* out_image, void* stream_) {
+    return gp_forward_impl(workspace, workspace_bytes, n_gauss, means, scales, quats, opacities, intensities, pose,
+                           grid_pack, focus_params, H, W, lateral_spacing, axial_spacing, axial_near, tile_size,
+                           k_sigma, sort_by_v, cap, out_image, nullptr, stream_);
+}
+
+extern "C" int us3d_gp_forward_checked(void* workspace, size_t workspace_bytes, int64_t n_gauss, const float* means,
+                                       const float* scales, const float* quats, const float* opacities,
+                                       const float* intensities, const float* pose, const float* grid_pack,
+                                       const float* focus_params, int32_t H, int32_t W, float lateral_spacing,
+                                       float axial_spacing, float axial_near, int32_t tile_size, float k_sigma,
+                                       int32_t sort_by_v, int64_t cap, float* out_image, int64_t* total,
+                                       int32_t* flags, void* stream_) {
+    StatusRead status;
+    const int st = gp_forward_impl(workspace, workspace_bytes, n_gauss, means, scales, quats, opacities, intensities,
+                                   pose, grid_pack, focus_params, H, W, lateral_spacing, axial_spacing, axial_near,
+                                   tile_size, k_sigma, sort_by_v, cap, out_image, &status, stream_);
+    return st != US3D_OK ? st : wait_status(status, total, flags);
 }
 
 extern "C" int us3d_gp_read_status(const void* workspace, int64_t* total, int32_t* flags, void* stream_) {

@@ -531,10 +531,10 @@ extern "C" size_t us3d_sa_backward_scratch_bytes(int64_t cap) {
     return cap < 0 ? 0 : (size_t)cap * PARTIAL_F4 * sizeof(float4);
 }
 
-extern "C" int us3d_sa_bounded_forward(void* workspace, size_t workspace_bytes, int64_t n, int32_t H, int32_t W,
-                                       float half_width, float half_height, const float* means2d, const float* inv2d,
-                                       const float* weights, const float* colors, float radius_sigma, int64_t cap,
-                                       float* out_image, float* out_alpha, void* stream_) {
+static int sa_bounded_forward_impl(void* workspace, size_t workspace_bytes, int64_t n, int32_t H, int32_t W,
+                                   float half_width, float half_height, const float* means2d, const float* inv2d,
+                                   const float* weights, const float* colors, float radius_sigma, int64_t cap,
+                                   float* out_image, float* out_alpha, StatusRead* status, void* stream_) {
     int st = sa_check(H, W, half_width, half_height, radius_sigma, n, cap);
     if (st != US3D_OK) return st;
     US3D_CHECK_ARG(workspace && out_image && out_alpha, "NULL pointer argument");
@@ -557,6 +557,10 @@ extern "C" int us3d_sa_bounded_forward(void* workspace, size_t workspace_bytes, 
     US3D_CHECK_CUDA(launch_bins(n, gw, T, RectOf4{w.rects}, nullptr, w.touched, w.stable, w.tile_count,
                                 w.tile_start, w.tile_cursor, w.inst_offset, w.bs_g, w.bs_t, w.header, cap, w.keys, w.slot_inst,
                                 w.sorted_gid, w.sorted_inst, g_sa_sort_attr, stream));
+    if (status != nullptr) {
+        const int rc = status->record(w.header, stream);
+        if (rc != US3D_OK) return rc;
+    }
     const int split = frame_split(T);
     forward_kernel<<<(unsigned)(T * split), TILE * TILE, 0, stream>>>(
         split, H, W, gw, half_width, half_height, radius_sigma, m2, iv, weights, colors, w.tile_start, w.sorted_gid,
@@ -570,6 +574,26 @@ extern "C" int us3d_sa_bounded_forward(void* workspace, size_t workspace_bytes, 
     prof_end(prof, stream);
     count_launches(1 + (n > 0) + bins_launches(n, T, w.keys == nullptr, false) + 1 + (split > 1));
     return US3D_OK;
+}
+
+extern "C" int us3d_sa_bounded_forward(void* workspace, size_t workspace_bytes, int64_t n, int32_t H, int32_t W,
+                                       float half_width, float half_height, const float* means2d, const float* inv2d,
+                                       const float* weights, const float* colors, float radius_sigma, int64_t cap,
+                                       float* out_image, float* out_alpha, void* stream_) {
+    return sa_bounded_forward_impl(workspace, workspace_bytes, n, H, W, half_width, half_height, means2d, inv2d,
+                                   weights, colors, radius_sigma, cap, out_image, out_alpha, nullptr, stream_);
+}
+
+extern "C" int us3d_sa_bounded_forward_checked(void* workspace, size_t workspace_bytes, int64_t n, int32_t H,
+                                               int32_t W, float half_width, float half_height, const float* means2d,
+                                               const float* inv2d, const float* weights, const float* colors,
+                                               float radius_sigma, int64_t cap, float* out_image, float* out_alpha,
+                                               int64_t* total, int32_t* flags, void* stream_) {
+    StatusRead status;
+    const int st = sa_bounded_forward_impl(workspace, workspace_bytes, n, H, W, half_width, half_height, means2d,
+                                           inv2d, weights, colors, radius_sigma, cap, out_image, out_alpha, &status,
+                                           stream_);
+    return st != US3D_OK ? st : wait_status(status, total, flags);
 }
 
 extern "C" int us3d_sa_read_status(const void* workspace, int64_t* total, int32_t* flags, void* stream_) {

@@ -33,6 +33,7 @@ extern "C" int us3d_set_device(int device) {
 // ---- launch counter and stage timing (benchmark instrumentation) ----
 #include <atomic>
 #include <mutex>
+#include <new>
 #include <string.h>
 #include <vector>
 
@@ -113,3 +114,89 @@ extern "C" int us3d_profile_collect(int* n_launches, double* total_ms) {
     p.used = 0;
     return US3D_OK;
 }
+
+// ---- status words read back to the host ----
+namespace us3d {
+
+namespace {
+struct StatusSlot {
+    long long* words;  // pinned
+    cudaEvent_t done;
+    int device;
+};
+constexpr int STATUS_SLOTS_KEPT = 32;  // idle slots kept; beyond that a returned slot is freed
+std::mutex g_slot_mu;
+StatusSlot* g_idle[STATUS_SLOTS_KEPT];
+int g_n_idle = 0;
+
+void free_slot(StatusSlot* s) {
+    if (s->done) cudaEventDestroy(s->done);
+    if (s->words) cudaFreeHost(s->words);
+    delete s;
+}
+
+cudaError_t acquire_slot(StatusSlot** out) {
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    {
+        std::lock_guard<std::mutex> lk(g_slot_mu);
+        for (int i = 0; i < g_n_idle; ++i)
+            if (g_idle[i]->device == device) {
+                *out = g_idle[i];
+                g_idle[i] = g_idle[--g_n_idle];
+                return cudaSuccess;
+            }
+    }
+    StatusSlot* s = new (std::nothrow) StatusSlot{nullptr, nullptr, device};
+    if (s == nullptr) return cudaErrorMemoryAllocation;
+    e = cudaHostAlloc(reinterpret_cast<void**>(&s->words), sizeof(long long) * STATUS_WORDS, cudaHostAllocPortable);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&s->done, cudaEventDisableTiming);
+    if (e != cudaSuccess) {
+        free_slot(s);
+        return e;
+    }
+    *out = s;
+    return cudaSuccess;
+}
+}  // namespace
+
+StatusRead::~StatusRead() {
+    StatusSlot* s = static_cast<StatusSlot*>(slot_);
+    if (s == nullptr) return;
+    if (pending_) cudaEventSynchronize(s->done);  // an error return in between: the copy may still be under way
+    {
+        std::lock_guard<std::mutex> lk(g_slot_mu);
+        if (g_n_idle < STATUS_SLOTS_KEPT) {
+            g_idle[g_n_idle++] = s;
+            return;
+        }
+    }
+    free_slot(s);
+}
+
+int StatusRead::record(const long long* words, cudaStream_t stream) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    US3D_CHECK_CUDA(cudaStreamIsCapturing(stream, &capture));
+    if (capture != cudaStreamCaptureStatusNone) {
+        set_error("the instance total cannot be read back while the stream is being captured");
+        return US3D_CUDA_ERROR;
+    }
+    StatusSlot* s = nullptr;
+    US3D_CHECK_CUDA(acquire_slot(&s));
+    slot_ = s;
+    pending_ = true;
+    US3D_CHECK_CUDA(cudaMemcpyAsync(s->words, words, sizeof(long long) * STATUS_WORDS, cudaMemcpyDeviceToHost, stream));
+    US3D_CHECK_CUDA(cudaEventRecord(s->done, stream));
+    return US3D_OK;
+}
+
+int StatusRead::wait(long long (&out)[STATUS_WORDS]) {
+    StatusSlot* s = static_cast<StatusSlot*>(slot_);
+    US3D_CHECK_CUDA(cudaEventSynchronize(s->done));
+    pending_ = false;
+    for (int i = 0; i < STATUS_WORDS; ++i) out[i] = s->words[i];
+    return US3D_OK;
+}
+
+}  // namespace us3d

@@ -1185,13 +1185,13 @@ static Params make_params(int64_t P, int32_t D, int32_t M, int32_t W, int32_t H,
     return p;
 }
 
-extern "C" int us3d_gs_forward(void* workspace, size_t workspace_bytes, int64_t n_gauss, int32_t sh_degree,
-                               int32_t sh_coeffs, const float* background, int32_t width, int32_t height,
-                               const float* means3D, const float* shs, const float* colors_precomp,
-                               const float* opacities, const float* scales, float scale_modifier,
-                               const float* rotations, const float* transmat_precomp, const float* viewmatrix,
-                               const float* projmatrix, const float* campos, int32_t prefiltered, int64_t cap,
-                               float* out_color, float* out_others, int32_t* out_radii, void* stream_) {
+static int gs_forward_impl(void* workspace, size_t workspace_bytes, int64_t n_gauss, int32_t sh_degree,
+                           int32_t sh_coeffs, const float* background, int32_t width, int32_t height,
+                           const float* means3D, const float* shs, const float* colors_precomp,
+                           const float* opacities, const float* scales, float scale_modifier, const float* rotations,
+                           const float* transmat_precomp, const float* viewmatrix, const float* projmatrix,
+                           const float* campos, int32_t prefiltered, int64_t cap, float* out_color, float* out_others,
+                           int32_t* out_radii, StatusRead* status, void* stream_) {
     US3D_CHECK_ARG(width > 0 && height > 0, "image_width/image_height must be positive");
     US3D_CHECK_ARG(n_gauss >= 0 && n_gauss <= 0x7fffffffLL, "n_gauss out of range");
     US3D_CHECK_ARG(cap >= 0 && cap <= 0x7fffffffLL, "instance capacity must be in [0, 2^31)");
@@ -1223,12 +1223,45 @@ extern "C" int us3d_gs_forward(void* workspace, size_t workspace_bytes, int64_t 
     US3D_CHECK_CUDA(launch_bins(n_gauss, p.gx, T, RectOf4{w.rect}, reinterpret_cast<const uint32_t*>(w.depth), w.touched, w.stable, w.tile_count,
                                 w.tile_start, w.tile_cursor, w.inst_offset, w.bs_g, w.bs_t, w.header, cap, w.keys, w.slot_inst,
                                 w.sorted_gid, w.sorted_inst, g_gs_sort_attr, stream));
+    if (status != nullptr) {
+        const int rc = status->record(w.header, stream);
+        if (rc != US3D_OK) return rc;
+    }
     forward_kernel<<<(unsigned)T, BLOCK, 0, stream>>>(width, height, p.gx, w.tile_start, w.sorted_gid, w.header, w.rec,
                                                       background, out_color, out_others, w.accum, w.n_contrib);
     US3D_CHECK_LAUNCH("gs forward");
     prof_end(prof, stream);
     count_launches(1 + (n_gauss > 0) + bins_launches(n_gauss, T, w.keys == nullptr, true) + 1);
     return US3D_OK;
+}
+
+extern "C" int us3d_gs_forward(void* workspace, size_t workspace_bytes, int64_t n_gauss, int32_t sh_degree,
+                               int32_t sh_coeffs, const float* background, int32_t width, int32_t height,
+                               const float* means3D, const float* shs, const float* colors_precomp,
+                               const float* opacities, const float* scales, float scale_modifier,
+                               const float* rotations, const float* transmat_precomp, const float* viewmatrix,
+                               const float* projmatrix, const float* campos, int32_t prefiltered, int64_t cap,
+                               float* out_color, float* out_others, int32_t* out_radii, void* stream_) {
+    return gs_forward_impl(workspace, workspace_bytes, n_gauss, sh_degree, sh_coeffs, background, width, height,
+                           means3D, shs, colors_precomp, opacities, scales, scale_modifier, rotations,
+                           transmat_precomp, viewmatrix, projmatrix, campos, prefiltered, cap, out_color, out_others,
+                           out_radii, nullptr, stream_);
+}
+
+extern "C" int us3d_gs_forward_checked(void* workspace, size_t workspace_bytes, int64_t n_gauss, int32_t sh_degree,
+                                       int32_t sh_coeffs, const float* background, int32_t width, int32_t height,
+                                       const float* means3D, const float* shs, const float* colors_precomp,
+                                       const float* opacities, const float* scales, float scale_modifier,
+                                       const float* rotations, const float* transmat_precomp, const float* viewmatrix,
+                                       const float* projmatrix, const float* campos, int32_t prefiltered, int64_t cap,
+                                       float* out_color, float* out_others, int32_t* out_radii, int64_t* total,
+                                       int32_t* flags, void* stream_) {
+    StatusRead status;
+    const int st = gs_forward_impl(workspace, workspace_bytes, n_gauss, sh_degree, sh_coeffs, background, width,
+                                   height, means3D, shs, colors_precomp, opacities, scales, scale_modifier, rotations,
+                                   transmat_precomp, viewmatrix, projmatrix, campos, prefiltered, cap, out_color,
+                                   out_others, out_radii, &status, stream_);
+    return st != US3D_OK ? st : wait_status(status, total, flags);
 }
 
 extern "C" int us3d_gs_read_status(const void* workspace, int64_t* total, int32_t* flags, void* stream_) {

@@ -954,8 +954,8 @@ backward_kernel(int64_t T, int64_t P, const us3d_slice_frame* __restrict__ frame
                 gD = 0.f;
             } else {
                 gI = d_image[p];
-                gA = d_alpha[p];
-                gD = d_depth[p];
+                gA = d_alpha ? d_alpha[p] : 0.f;
+                gD = d_depth ? d_depth[p] : 0.f;
             }
             const float dnum = gI * inv_alpha;
             const float dtot = gA - gI * num * inv_alpha * inv_alpha;
@@ -1320,8 +1320,8 @@ backward_packed_kernel(int64_t T, int64_t P, const us3d_slice_frame* __restrict_
                     gD = 0.f;
                 } else {
                     gI = d_image[p];
-                    gA = d_alpha[p];
-                    gD = d_depth[p];
+                    gA = d_alpha ? d_alpha[p] : 0.f;
+                    gD = d_depth ? d_depth[p] : 0.f;
                 }
                 const float inv_sa = 1.0f / fmaxf(sum_alpha, 1e-8f);
                 px[h] = pixels[3 * p];
@@ -1849,13 +1849,70 @@ extern "C" int us3d_ug_forward(void* workspace, const us3d_slice_frame* frames, 
     return US3D_OK;
 }
 
+extern "C" int us3d_ug_bin_forward(void* workspace, size_t workspace_bytes, const us3d_slice_frame* frames,
+                                   int32_t n_frames, int64_t n_tiles, int64_t n_pixels, int64_t n_gauss,
+                                   const float* means, const float* tril, const float* opac, const float* inten,
+                                   float chi2, float beta, int32_t sort_by_depth, int64_t cap, const float* pixels,
+                                   int32_t flags, float bg_alpha, float bg_intensity, float* out_image,
+                                   float* out_alpha, float* out_depth, int32_t* out_counts, int64_t* total,
+                                   int64_t* n_tasks, int32_t* status_flags, void* stream_) {
+    int st = us3d_ug_bin_ex(workspace, workspace_bytes, frames, n_frames, n_tiles, n_pixels, n_gauss, means, tril, opac,
+                            inten, chi2, beta, sort_by_depth, cap, pixels, flags, stream_);
+    if (st != US3D_OK) return st;
+    StatusRead status;
+    st = status.record(carve(workspace, n_gauss, n_tiles, n_pixels, cap).header, (cudaStream_t)stream_);
+    if (st != US3D_OK) return st;
+    st = us3d_ug_forward(workspace, frames, n_frames, n_tiles, n_pixels, n_gauss, cap, pixels, chi2, beta, bg_alpha,
+                         bg_intensity, out_image, out_alpha, out_depth, out_counts, stream_);
+    return st != US3D_OK ? st : wait_status(status, total, status_flags, n_tasks);
+}
+
+namespace us3d {
+namespace ug {
+__global__ void frame_table_kernel(us3d_slice_frame* frame, const float* __restrict__ o, const float* __restrict__ lat,
+                                   const float* __restrict__ ax, const float* __restrict__ ele, float dlat, float dax,
+                                   float near, float coloff, int H, int W) {
+    const int i = threadIdx.x;
+    if (i < 3) {
+        frame->origin[i] = o[i];
+        frame->axis_lat[i] = lat[i];
+        frame->axis_ax[i] = ax[i];
+        frame->axis_ele[i] = ele[i];
+    }
+    if (i == 3) {
+        frame->lateral_spacing = dlat;
+        frame->axial_spacing = dax;
+        frame->axial_near = near;
+        frame->lateral_col_offset = coloff;
+        frame->height = H;
+        frame->width = W;
+        frame->tiles_x = (W + TILE - 1) / TILE;
+        frame->tiles_y = (H + TILE - 1) / TILE;
+        frame->pixel_offset = frame->tile_offset = frame->gauss_offset = frame->gauss_count = 0;
+    }
+}
+}  // namespace ug
+}  // namespace us3d
+
+extern "C" int us3d_ug_frame_table(us3d_slice_frame* frame, const float* origin, const float* axis_lat,
+                                   const float* axis_ax, const float* axis_ele, float lateral_spacing,
+                                   float axial_spacing, float axial_near, float lateral_col_offset, int32_t height,
+                                   int32_t width, void* stream_) {
+    US3D_CHECK_ARG(frame && origin && axis_lat && axis_ax && axis_ele, "NULL pointer argument");
+    frame_table_kernel<<<1, 32, 0, (cudaStream_t)stream_>>>(frame, origin, axis_lat, axis_ax, axis_ele, lateral_spacing,
+                                                            axial_spacing, axial_near, lateral_col_offset, height, width);
+    US3D_CHECK_LAUNCH("ug frame table");
+    count_launches(1);
+    return US3D_OK;
+}
+
 static int ug_backward_impl(void* workspace, const us3d_slice_frame* frames, int32_t n_frames, int64_t n_tiles,
                             int64_t n_pixels, int64_t n_gauss, int64_t cap, const float* pixels,
                             const float* d_image, const float* d_alpha, const float* d_depth,
                             const float* loss_image, const float* loss_target, const float4* loss_coef,
                             const float* saved_alpha, float chi2, float beta, float bg_alpha, float bg_intensity,
                             void* scratch, size_t scratch_bytes, float* d_means, float* d_tril, float* d_opac,
-                            float* d_inten, cudaStream_t stream) {
+                            float* d_inten, bool need_all, cudaStream_t stream) {
     const bool fused = loss_coef != nullptr;
     int st = check_common(frames, n_frames, n_tiles, n_pixels, n_gauss);
     if (st != US3D_OK) return st;
@@ -1868,7 +1925,7 @@ static int ug_backward_impl(void* workspace, const us3d_slice_frame* frames, int
     if (fused)
         US3D_CHECK_ARG(n_pixels == 0 || (pixels && loss_image && loss_target && saved_alpha), "input pointer is NULL");
     else
-        US3D_CHECK_ARG(n_pixels == 0 || (pixels && d_image && d_alpha && d_depth && saved_alpha),
+        US3D_CHECK_ARG(n_pixels == 0 || (pixels && d_image && saved_alpha && (!need_all || (d_alpha && d_depth))),
                        "input pointer is NULL");
     const Workspace w = carve(workspace, n_gauss, n_tiles, n_pixels, cap);
     float4* partial = reinterpret_cast<float4*>(scratch);
@@ -1916,7 +1973,18 @@ extern "C" int us3d_ug_backward(void* workspace, const us3d_slice_frame* frames,
                                 float* d_tril, float* d_opac, float* d_inten, void* stream_) {
     return ug_backward_impl(workspace, frames, n_frames, n_tiles, n_pixels, n_gauss, cap, pixels, d_image, d_alpha,
                             d_depth, nullptr, nullptr, nullptr, saved_alpha, chi2, beta, bg_alpha, bg_intensity,
-                            scratch, scratch_bytes, d_means, d_tril, d_opac, d_inten, (cudaStream_t)stream_);
+                            scratch, scratch_bytes, d_means, d_tril, d_opac, d_inten, true, (cudaStream_t)stream_);
+}
+
+extern "C" int us3d_ug_backward_ex(void* workspace, const us3d_slice_frame* frames, int32_t n_frames, int64_t n_tiles,
+                                   int64_t n_pixels, int64_t n_gauss, int64_t cap, const float* pixels,
+                                   const float* d_image, const float* d_alpha, const float* d_depth,
+                                   const float* saved_alpha, float chi2, float beta, float bg_alpha,
+                                   float bg_intensity, void* scratch, size_t scratch_bytes, float* d_means,
+                                   float* d_tril, float* d_opac, float* d_inten, void* stream_) {
+    return ug_backward_impl(workspace, frames, n_frames, n_tiles, n_pixels, n_gauss, cap, pixels, d_image, d_alpha,
+                            d_depth, nullptr, nullptr, nullptr, saved_alpha, chi2, beta, bg_alpha, bg_intensity,
+                            scratch, scratch_bytes, d_means, d_tril, d_opac, d_inten, false, (cudaStream_t)stream_);
 }
 
 extern "C" int us3d_ug_backward_loss(void* workspace, const us3d_slice_frame* frames, int32_t n_frames,
@@ -1929,7 +1997,7 @@ extern "C" int us3d_ug_backward_loss(void* workspace, const us3d_slice_frame* fr
     US3D_CHECK_ARG((reinterpret_cast<uintptr_t>(loss_coef) & 15) == 0, "loss coefficients must be 16-byte aligned");
     return ug_backward_impl(workspace, frames, n_frames, n_tiles, n_pixels, n_gauss, cap, pixels, nullptr, nullptr,
                             nullptr, image, target, reinterpret_cast<const float4*>(loss_coef), saved_alpha, chi2,
-                            beta, bg_alpha, bg_intensity, scratch, scratch_bytes, d_means, d_tril, d_opac, d_inten,
+                            beta, bg_alpha, bg_intensity, scratch, scratch_bytes, d_means, d_tril, d_opac, d_inten, true,
                             (cudaStream_t)stream_);
 }
 

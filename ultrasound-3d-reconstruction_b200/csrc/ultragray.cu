@@ -1504,15 +1504,15 @@ extern "C" size_t us3d_ugr_backward_scratch_bytes(int64_t cap) {
     return cap < 0 ? 0 : (size_t)cap * PARTIAL_F4 * sizeof(float4);
 }
 
-extern "C" int us3d_ugr_forward(void* workspace, size_t workspace_bytes, int64_t n_gauss, const float* means,
-                                const float* scales, const float* quats, const float* attenuations,
-                                const float* sh_coeffs, const float* pixel_positions, const float* ray_origins,
-                                const float* ray_dirs, const float* origin, const float* axis_lat,
-                                const float* axis_ele, const float* axis_ax, const float* ray_perturbations,
-                                int32_t W, int32_t H, float width_mm, float near_mm, float lateral_col_offset,
-                                float elev_cutoff_mm, float k_sigma, float quadrature_window_radius_mm,
-                                int32_t local_window_only, float local_max_window_mm, int64_t cap,
-                                float* out_image, void* stream_) {
+static int ugr_forward_impl(void* workspace, size_t workspace_bytes, int64_t n_gauss, const float* means,
+                            const float* scales, const float* quats, const float* attenuations,
+                            const float* sh_coeffs, const float* pixel_positions, const float* ray_origins,
+                            const float* ray_dirs, const float* origin, const float* axis_lat, const float* axis_ele,
+                            const float* axis_ax, const float* ray_perturbations, int32_t W, int32_t H,
+                            float width_mm, float near_mm, float lateral_col_offset, float elev_cutoff_mm,
+                            float k_sigma, float quadrature_window_radius_mm, int32_t local_window_only,
+                            float local_max_window_mm, int64_t cap, float* out_image, StatusRead* status,
+                            void* stream_) {
     US3D_CHECK_ARG(W > 0 && H >= 0, "image_width/image_height must be positive");
     US3D_CHECK_ARG(width_mm > 0.f && k_sigma > 0.f, "width_mm and k_sigma must be > 0");
     US3D_CHECK_ARG(n_gauss >= 0 && n_gauss <= 0x7fffffffLL, "n_gauss out of range");
@@ -1537,6 +1537,10 @@ extern "C" int us3d_ugr_forward(void* workspace, size_t workspace_bytes, int64_t
     US3D_CHECK_CUDA(launch_bins(n_gauss, W, W, RangeOf2{w.ray_range}, w.dkey, w.touched, w.stable, w.ray_count,
                                 w.ray_start, w.ray_cursor, w.inst_offset, w.bs_g, w.bs_t, w.header, cap, w.keys, w.slot_inst,
                                 w.sorted_gid, w.sorted_inst, g_ugr_sort_attr, stream));
+    if (status != nullptr) {
+        const int rc = status->record(w.header, stream);
+        if (rc != US3D_OK) return rc;
+    }
     const unsigned tiles_y = (unsigned)((H + FWD_SAMPLES - 1) / FWD_SAMPLES);
     const int* ckpt_rays = nullptr;
     int launches = 1 + (n_gauss > 0) + bins_launches(n_gauss, W, w.keys == nullptr, true) + 1;
@@ -1566,6 +1570,41 @@ extern "C" int us3d_ugr_forward(void* workspace, size_t workspace_bytes, int64_t
     prof_end(prof, stream);
     count_launches(launches);
     return US3D_OK;
+}
+
+extern "C" int us3d_ugr_forward(void* workspace, size_t workspace_bytes, int64_t n_gauss, const float* means,
+                                const float* scales, const float* quats, const float* attenuations,
+                                const float* sh_coeffs, const float* pixel_positions, const float* ray_origins,
+                                const float* ray_dirs, const float* origin, const float* axis_lat,
+                                const float* axis_ele, const float* axis_ax, const float* ray_perturbations,
+                                int32_t W, int32_t H, float width_mm, float near_mm, float lateral_col_offset,
+                                float elev_cutoff_mm, float k_sigma, float quadrature_window_radius_mm,
+                                int32_t local_window_only, float local_max_window_mm, int64_t cap, float* out_image,
+                                void* stream_) {
+    return ugr_forward_impl(workspace, workspace_bytes, n_gauss, means, scales, quats, attenuations, sh_coeffs,
+                            pixel_positions, ray_origins, ray_dirs, origin, axis_lat, axis_ele, axis_ax,
+                            ray_perturbations, W, H, width_mm, near_mm, lateral_col_offset, elev_cutoff_mm, k_sigma,
+                            quadrature_window_radius_mm, local_window_only, local_max_window_mm, cap, out_image,
+                            nullptr, stream_);
+}
+
+extern "C" int us3d_ugr_forward_checked(void* workspace, size_t workspace_bytes, int64_t n_gauss, const float* means,
+                                        const float* scales, const float* quats, const float* attenuations,
+                                        const float* sh_coeffs, const float* pixel_positions,
+                                        const float* ray_origins, const float* ray_dirs, const float* origin,
+                                        const float* axis_lat, const float* axis_ele, const float* axis_ax,
+                                        const float* ray_perturbations, int32_t W, int32_t H, float width_mm,
+                                        float near_mm, float lateral_col_offset, float elev_cutoff_mm, float k_sigma,
+                                        float quadrature_window_radius_mm, int32_t local_window_only,
+                                        float local_max_window_mm, int64_t cap, float* out_image, int64_t* total,
+                                        int32_t* flags, void* stream_) {
+    StatusRead status;
+    const int st = ugr_forward_impl(workspace, workspace_bytes, n_gauss, means, scales, quats, attenuations,
+                                    sh_coeffs, pixel_positions, ray_origins, ray_dirs, origin, axis_lat, axis_ele,
+                                    axis_ax, ray_perturbations, W, H, width_mm, near_mm, lateral_col_offset,
+                                    elev_cutoff_mm, k_sigma, quadrature_window_radius_mm, local_window_only,
+                                    local_max_window_mm, cap, out_image, &status, stream_);
+    return st != US3D_OK ? st : wait_status(status, total, flags);
 }
 
 extern "C" int us3d_ugr_read_status(const void* workspace, int64_t* total, int32_t* flags, void* stream_) {

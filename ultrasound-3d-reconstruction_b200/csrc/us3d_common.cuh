@@ -22,6 +22,25 @@ void count_launches(int n);
 int prof_begin(const char* stage, cudaStream_t stream);
 void prof_end(int slot, cudaStream_t stream);
 
+// One call's copy of the words at the start of a workspace (instance total, flags) to the host. It is
+// queued behind the binning and waited for after the shading has been queued too, so that the host
+// neither leaves the GPU idle between the two nor waits for the shading. Pinned words and an event come
+// from a pool shared by all threads and streams (status.cu); the destructor gives them back.
+constexpr int STATUS_WORDS = 16;
+class StatusRead {
+public:
+    StatusRead() = default;
+    StatusRead(const StatusRead&) = delete;
+    StatusRead& operator=(const StatusRead&) = delete;
+    ~StatusRead();
+    int record(const long long* words, cudaStream_t stream);  // US3D_OK or an error (refused under capture)
+    int wait(long long (&out)[STATUS_WORDS]);
+
+private:
+    void* slot_ = nullptr;
+    bool pending_ = false;
+};
+
 #define US3D_CHECK_ARG(cond, ...)                 \
     do {                                          \
         if (!(cond)) {                            \

@@ -43,6 +43,9 @@ def _us_focus_params_vector(config: GaussianPlieRenderConfig, device: torch.devi
     vals[8] = 0.5  # det_gamma
     vals[9] = float(config.det_eps)
     vals[10] = max(float(config.opacity_cull_threshold), 1.0e-12)
+    if device.type == "cuda" and not torch.cuda.is_current_stream_capturing():
+        # from pinned memory: a copy from pageable memory waits for everything queued on the stream
+        return torch.tensor(vals, dtype=torch.float32, pin_memory=True).to(device, non_blocking=True)
     return torch.tensor(vals, dtype=torch.float32, device=device)
 
 
@@ -124,5 +127,5 @@ def render_gaussianpile_projected_slice(config: GaussianPlieRenderConfig, gauss_
     device = gauss_means.device
     return _GaussianPileProjectedSliceCudaFunction.apply(
         gauss_means, gauss_scales, gauss_quats, gauss_alphas, torch.ones_like(gauss_alphas), pose_probe_to_world,
-        slice_grid_geometry.to(device=device, dtype=torch.float32), _meta_vector(config, device),
+        slice_grid_geometry.to(device=device, dtype=torch.float32), _meta_vector(config, torch.device("cpu")),
         _us_focus_params_vector(config, device), shape_gradients)

@@ -78,11 +78,11 @@ class _RenderFunction(torch.autograd.Function):
         # Without a request for intermediates the tiles are culled to the Gaussians' in-slice
         # chi-square ellipses (identical image and gradients, no candidate counts).
         cull = holder is not None and not holder.get("want_counts", True) and n_pixels > 0
-        b = _ug.bin_gaussians(means, tril, opac, inten, frames, float(config.chi2_threshold),
-                              float(config.diag_beta), bool(config.mapper_sort_by_depth),
-                              slice_cull_pixels=pixels if cull else None)
-        image, alpha, depth, counts = _ug.forward(b, pixels, float(config.fixed_bg_alpha),
-                                                  float(config.fixed_bg_intensity))
+        b, image, alpha, depth, counts = _ug.bin_forward(
+            means, tril, opac, inten, frames, float(config.chi2_threshold), float(config.diag_beta),
+            bool(config.mapper_sort_by_depth), pixels, float(config.fixed_bg_alpha), float(config.fixed_bg_intensity),
+            cull, True)
+        ctx.set_materialize_grads(False)
         if counts is None:
             counts = torch.zeros(0, dtype=torch.int32, device=pixels.device)
         ctx.save_for_backward(pixels, alpha)
@@ -99,10 +99,11 @@ class _RenderFunction(torch.autograd.Function):
         del d_counts
         pixels, alpha = ctx.saved_tensors
         cfg = ctx.config
-        dm, dt, do, di = _ug.backward(
-            ctx.binning, pixels, d_image.contiguous().float(), d_alpha.contiguous().float(),
-            d_depth.contiguous().float(), alpha, float(cfg.fixed_bg_alpha), float(cfg.fixed_bg_intensity),
-        )
+        if d_image is None:
+            d_image = torch.zeros_like(alpha)
+        c = lambda t: None if t is None else t.contiguous().float()  # noqa: E731
+        dm, dt, do, di = _ug.backward(ctx.binning, pixels, c(d_image), c(d_alpha), c(d_depth), alpha,
+                                      float(cfg.fixed_bg_alpha), float(cfg.fixed_bg_intensity), absent_zero=True)
         if ctx.means_cols == 4:
             dm = torch.nn.functional.pad(dm, (0, 1))
         return None, dm, dt, do, di, None, None, None, None, None, None

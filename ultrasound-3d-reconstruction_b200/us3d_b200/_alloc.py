@@ -14,6 +14,11 @@ from typing import Iterable, List, Sequence, Tuple
 import torch
 
 
+def current_stream() -> int:
+    """The current CUDA stream of the current device, without building a Stream object."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
 def float_outputs(device: torch.device, shapes: Sequence[Tuple[int, ...]],
                   zero: Iterable[int] = ()) -> List[torch.Tensor]:
     """Float32 tensors of ``shapes`` sharing one allocation; those whose index is in ``zero`` are

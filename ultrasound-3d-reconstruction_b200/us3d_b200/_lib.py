@@ -108,6 +108,23 @@ _SIGNATURES = {
          c_void_p, c_float, c_float, c_float, c_float, c_void_p, c_size_t, c_void_p, c_void_p, c_void_p, c_void_p,
          c_void_p],
     ),
+    "us3d_ug_backward_ex": (
+        c_int32,
+        [c_void_p, c_void_p, c_int32, c_int64, c_int64, c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_void_p,
+         c_void_p, c_float, c_float, c_float, c_float, c_void_p, c_size_t, c_void_p, c_void_p, c_void_p, c_void_p,
+         c_void_p],
+    ),
+    "us3d_ug_bin_forward": (
+        c_int32,
+        [c_void_p, c_size_t, c_void_p, c_int32, c_int64, c_int64, c_int64, c_void_p, c_void_p, c_void_p,
+         c_void_p, c_float, c_float, c_int32, c_int64, c_void_p, c_int32, c_float, c_float, c_void_p, c_void_p,
+         c_void_p, c_void_p, POINTER(c_int64), POINTER(c_int64), POINTER(c_int32), c_void_p],
+    ),
+    "us3d_ug_frame_table": (
+        c_int32,
+        [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_float, c_float, c_float, c_int32, c_int32,
+         c_void_p],
+    ),
     "us3d_ug_set_launch_config": (c_int32, [c_int32, c_int32]),
     "us3d_ug_get_launch_config": (c_int32, [POINTER(c_int32), POINTER(c_int32)]),
     "us3d_ug_set_backward_variant": (c_int32, [c_int32]),
@@ -160,6 +177,12 @@ _SIGNATURES = {
          c_void_p, c_int32, c_int32, c_float, c_float, c_float, c_int32, c_float, c_int32, c_int64, c_void_p,
          c_void_p],
     ),
+    "us3d_gp_forward_checked": (
+        c_int32,
+        [c_void_p, c_size_t, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+         c_void_p, c_int32, c_int32, c_float, c_float, c_float, c_int32, c_float, c_int32, c_int64, c_void_p,
+         POINTER(c_int64), POINTER(c_int32), c_void_p],
+    ),
     "us3d_gp_read_status": (c_int32, [c_void_p, POINTER(c_int64), POINTER(c_int32), c_void_p]),
     "us3d_gp_backward": (
         c_int32,
@@ -177,6 +200,11 @@ _SIGNATURES = {
         c_int32,
         [c_void_p, c_size_t, c_int64, c_int32, c_int32, c_float, c_float, c_void_p, c_void_p, c_void_p, c_void_p,
          c_float, c_int64, c_void_p, c_void_p, c_void_p],
+    ),
+    "us3d_sa_bounded_forward_checked": (
+        c_int32,
+        [c_void_p, c_size_t, c_int64, c_int32, c_int32, c_float, c_float, c_void_p, c_void_p, c_void_p, c_void_p,
+         c_float, c_int64, c_void_p, c_void_p, POINTER(c_int64), POINTER(c_int32), c_void_p],
     ),
     "us3d_sa_read_status": (c_int32, [c_void_p, POINTER(c_int64), POINTER(c_int32), c_void_p]),
     "us3d_sa_bounded_backward": (
@@ -213,6 +241,12 @@ _SIGNATURES = {
         + [c_int32, c_int32, c_float, c_float, c_float, c_float, c_float, c_float, c_int32, c_float, c_int64,
            c_void_p, c_void_p],
     ),
+    "us3d_ugr_forward_checked": (
+        c_int32,
+        [c_void_p, c_size_t, c_int64] + [c_void_p] * 13
+        + [c_int32, c_int32, c_float, c_float, c_float, c_float, c_float, c_float, c_int32, c_float, c_int64,
+           c_void_p, POINTER(c_int64), POINTER(c_int32), c_void_p],
+    ),
     "us3d_ugr_read_status": (c_int32, [c_void_p, POINTER(c_int64), POINTER(c_int32), c_void_p]),
     "us3d_ugr_backward": (
         c_int32,
@@ -229,6 +263,11 @@ _SIGNATURES = {
         c_int32,
         [c_void_p, c_size_t, c_int64, c_int32, c_int32, c_void_p, c_int32, c_int32] + [c_void_p] * 5
         + [c_float] + [c_void_p] * 5 + [c_int32, c_int64, c_void_p, c_void_p, c_void_p, c_void_p],
+    ),
+    "us3d_gs_forward_checked": (
+        c_int32,
+        [c_void_p, c_size_t, c_int64, c_int32, c_int32, c_void_p, c_int32, c_int32] + [c_void_p] * 5
+        + [c_float] + [c_void_p] * 5 + [c_int32, c_int64, c_void_p, c_void_p, c_void_p, POINTER(c_int64), POINTER(c_int32), c_void_p],
     ),
     "us3d_gs_read_status": (c_int32, [c_void_p, POINTER(c_int64), POINTER(c_int32), c_void_p]),
     "us3d_gs_backward": (
@@ -290,4 +329,4 @@ def check(status: int, what: str) -> None:
 
 
 def call(name: str, *args) -> int:
-    return getattr(load(), name)(*args)
+    return getattr(_lib or load(), name)(*args)

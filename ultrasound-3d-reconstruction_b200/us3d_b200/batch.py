@@ -21,11 +21,17 @@ class _BatchFunction(torch.autograd.Function):
     def forward(ctx, frames: UG.FrameTable, params: dict, means, tril, opac, inten, pixels, holder):
         want_counts = params.get("want_counts", False)
         cull = params.get("slice_cull", True) and not want_counts
-        b = UG.bin_gaussians(means, tril, opac, inten, frames, params["chi2"], params["beta"], params["sort_by_depth"],
-                             capacity=params.get("capacity"), sync_check=params.get("sync_check", True),
-                             slice_cull_pixels=pixels if cull else None)
-        image, alpha, depth, counts = UG.forward(b, pixels, params["bg_alpha"], params["bg_intensity"],
-                                                 want_counts=params.get("want_counts", False))
+        if params.get("sync_check", True):
+            b, image, alpha, depth, counts = UG.bin_forward(
+                means, tril, opac, inten, frames, params["chi2"], params["beta"], params["sort_by_depth"], pixels,
+                params["bg_alpha"], params["bg_intensity"], cull, want_counts, capacity=params.get("capacity"))
+        else:
+            b = UG.bin_gaussians(means, tril, opac, inten, frames, params["chi2"], params["beta"],
+                                 params["sort_by_depth"], capacity=params.get("capacity"), sync_check=False,
+                                 slice_cull_pixels=pixels if cull else None)
+            image, alpha, depth, counts = UG.forward(b, pixels, params["bg_alpha"], params["bg_intensity"],
+                                                     want_counts=want_counts)
+        ctx.set_materialize_grads(False)
         ctx.b = b
         ctx.params = params
         ctx.save_for_backward(pixels, alpha)
@@ -38,8 +44,11 @@ class _BatchFunction(torch.autograd.Function):
     def backward(ctx, d_image, d_alpha, d_depth):
         pixels, alpha = ctx.saved_tensors
         p = ctx.params
-        dm, dt, do, di = UG.backward(ctx.b, pixels, d_image.contiguous(), d_alpha.contiguous(), d_depth.contiguous(),
-                                     alpha, p["bg_alpha"], p["bg_intensity"])
+        if d_image is None:
+            d_image = torch.zeros_like(alpha)
+        c = lambda t: None if t is None else t.contiguous()  # noqa: E731
+        dm, dt, do, di = UG.backward(ctx.b, pixels, c(d_image), c(d_alpha), c(d_depth), alpha, p["bg_alpha"],
+                                     p["bg_intensity"], absent_zero=True)
         return None, None, dm, dt, do, di, None, None
 
 

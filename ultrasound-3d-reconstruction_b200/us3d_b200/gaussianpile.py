@@ -9,13 +9,9 @@ from typing import Optional
 import torch
 
 from . import _lib
-from ._alloc import float_outputs
+from ._alloc import current_stream as _stream, float_outputs
 
 _capacity_hint: dict = {}
-
-
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
 
 
 @dataclass
@@ -45,14 +41,12 @@ def forward(means, scales, quats, opac, inten, pose, grid, params, H, W, lateral
     for _ in range(3):
         nbytes = int(_lib.call("us3d_gp_workspace_bytes", G, H, W, tile_size, cap))
         ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
-        st = _lib.call("us3d_gp_forward", ws.data_ptr(), nbytes, G, *(t.data_ptr() for t in args), H, W,
+        total, flags = ctypes.c_int64(0), ctypes.c_int32(0)
+        st = _lib.call("us3d_gp_forward_checked", ws.data_ptr(), nbytes, G, *(t.data_ptr() for t in args), H, W,
                        float(lateral_spacing), float(axial_spacing), float(axial_near), int(tile_size), float(k_sigma),
-                       int(bool(sort_by_v)), cap, image.data_ptr(), _stream())
+                       int(bool(sort_by_v)), cap, image.data_ptr(), ctypes.byref(total),
+                       ctypes.byref(flags), _stream())
         _lib.check(st, "us3d_gp_forward")
-        total = ctypes.c_int64(0)
-        flags = ctypes.c_int32(0)
-        _lib.check(_lib.call("us3d_gp_read_status", ws.data_ptr(), ctypes.byref(total), ctypes.byref(flags),
-                             _stream()), "us3d_gp_read_status")
         if flags.value == 0:
             _capacity_hint[key] = max(4096, int(total.value * 1.25) + 1024)
             return image, GPBinning(ws, cap, int(total.value), G, H, W, int(tile_size), float(k_sigma), args)

@@ -9,12 +9,9 @@ from typing import Optional
 import torch
 
 from . import _lib
+from ._alloc import current_stream as _stream
 
 _capacity_hint: dict = {}
-
-
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
 
 
 @dataclass
@@ -42,14 +39,12 @@ def bounded_forward(H, W, half_width, half_height, means2d, inv2d, weights, colo
     for _ in range(3):
         nbytes = int(_lib.call("us3d_sa_workspace_bytes", N, H, W, cap))
         ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
-        st = _lib.call("us3d_sa_bounded_forward", ws.data_ptr(), nbytes, N, H, W, float(half_width), float(half_height),
+        total, flags = ctypes.c_int64(0), ctypes.c_int32(0)
+        st = _lib.call("us3d_sa_bounded_forward_checked", ws.data_ptr(), nbytes, N, H, W, float(half_width), float(half_height),
                        means2d.data_ptr(), inv2d.data_ptr(), weights.data_ptr(), colors.data_ptr(), float(radius_sigma),
-                       cap, image.data_ptr(), alpha.data_ptr(), _stream())
+                       cap, image.data_ptr(), alpha.data_ptr(), ctypes.byref(total),
+                       ctypes.byref(flags), _stream())
         _lib.check(st, "us3d_sa_bounded_forward")
-        total = ctypes.c_int64(0)
-        flags = ctypes.c_int32(0)
-        _lib.check(_lib.call("us3d_sa_read_status", ws.data_ptr(), ctypes.byref(total), ctypes.byref(flags),
-                             _stream()), "us3d_sa_read_status")
         if flags.value == 0:
             _capacity_hint[key] = max(4096, int(total.value * 1.25) + 1024)
             return image, alpha, SABinning(ws, cap, int(total.value), N, H, W)

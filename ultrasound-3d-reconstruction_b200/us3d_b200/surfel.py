@@ -14,13 +14,9 @@ from typing import Optional
 import torch
 
 from . import _lib
-from ._alloc import float_outputs
+from ._alloc import current_stream as _stream, float_outputs
 
 _capacity_hint: dict = {}
-
-
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -65,16 +61,14 @@ def forward(background, means3D, colors, opacity, scales, rotations, scale_modif
     for _ in range(3):
         nbytes = int(_lib.call("us3d_gs_workspace_bytes", P, W, H, cap))
         ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
-        st = _lib.call("us3d_gs_forward", ws.data_ptr(), nbytes, P, int(degree), M, background.data_ptr(), W, H,
+        total, flags = ctypes.c_int64(0), ctypes.c_int32(0)
+        st = _lib.call("us3d_gs_forward_checked", ws.data_ptr(), nbytes, P, int(degree), M, background.data_ptr(), W, H,
                        means3D.data_ptr(), _ptr(sh), _ptr(colors), opacity.data_ptr(), _ptr(scales),
                        float(scale_modifier), _ptr(rotations), _ptr(transmat_precomp), viewmatrix.data_ptr(),
                        projmatrix.data_ptr(), _ptr(campos), 1 if prefiltered else 0, cap, color.data_ptr(),
-                       others.data_ptr(), radii.data_ptr(), _stream())
+                       others.data_ptr(), radii.data_ptr(), ctypes.byref(total),
+                       ctypes.byref(flags), _stream())
         _lib.check(st, "us3d_gs_forward")
-        total = ctypes.c_int64(0)
-        flags = ctypes.c_int32(0)
-        _lib.check(_lib.call("us3d_gs_read_status", ws.data_ptr(), ctypes.byref(total), ctypes.byref(flags),
-                             _stream()), "us3d_gs_read_status")
         if flags.value & 4:
             raise RuntimeError("Point is filtered although prefiltered is set. This shouldn't happen!")
         if flags.value & 2:

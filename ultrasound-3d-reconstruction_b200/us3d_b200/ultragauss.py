@@ -15,16 +15,13 @@ from typing import List, Optional, Sequence, Tuple
 import torch
 
 from . import _lib
+from ._alloc import current_stream as _stream
 
 TILE = 16
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
-
-
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
 
 
 def _set_device(dev: torch.device) -> None:
@@ -65,8 +62,30 @@ class FrameTable:
     gaussian_sets: bool = False
 
 
+def _on_device(s: SliceSpec, device: torch.device) -> bool:
+    """Whether a frame over all Gaussians can be written by one kernel: its geometry is on the device."""
+    return s.gaussian_set is None and all(
+        type(t) is torch.Tensor and t.is_cuda and t.device == device and t.dtype == torch.float32 and t.numel() == 3
+        and t.is_contiguous() for t in (s.origin, s.axis_lat, s.axis_ax, s.axis_ele))
+
+
+def _one_frame_table(s: SliceSpec) -> FrameTable:
+    """The table of one frame, without its geometry passing through the host (a renderer called with
+    one frame per step builds a table per call: about 100 us of tensor operations otherwise)."""
+    H, W = int(s.height), int(s.width)
+    n_tiles = ((W + TILE - 1) // TILE) * ((H + TILE - 1) // TILE)
+    _set_device(s.origin.device)
+    table = torch.empty((1, 24), dtype=torch.float32, device=s.origin.device)
+    _lib.check(_lib.call("us3d_ug_frame_table", _ptr(table), _ptr(s.origin), _ptr(s.axis_lat), _ptr(s.axis_ax),
+                         _ptr(s.axis_ele), float(s.lateral_spacing), float(s.axial_spacing), float(s.axial_near),
+                         float(s.lateral_col_offset), H, W, _stream()), "us3d_ug_frame_table")
+    return FrameTable(table, 1, n_tiles, H * W, [0], [n_tiles], [0], [(H, W)], False)
+
+
 def build_frame_table(specs: Sequence[SliceSpec], device: torch.device) -> FrameTable:
     """Packs slice geometry into the device array of ``us3d_slice_frame``."""
+    if len(specs) == 1 and _on_device(specs[0], device):
+        return _one_frame_table(specs[0])
     F = len(specs)
     ints = torch.zeros((F, 8), dtype=torch.int32)
     scal = torch.zeros((F, 4), dtype=torch.float32)
@@ -164,8 +183,7 @@ def bin_gaussians(means: torch.Tensor, tril: torch.Tensor, opac: torch.Tensor, i
             "us3d_ug_bin_ex", _ptr(ws), int(nbytes), _ptr(frames.table), frames.n_frames, frames.n_tiles,
             frames.n_pixels, G, _ptr(means), _ptr(tril), _ptr(opac), _ptr(inten), float(chi2), float(beta),
             int(bool(sort_by_depth)), cap, _ptr(slice_cull_pixels) if cull else None,
-            (_lib.UG_BIN_SLICE_CULL if cull else 0) | (_lib.UG_BIN_LOGIT_ATTRIBUTES if logit_attributes else 0)
-            | (_lib.UG_BIN_GAUSSIAN_SETS if frames.gaussian_sets else 0), _stream(),
+            _bin_flags(cull, logit_attributes, frames), _stream(),
         )
         _lib.check(st, "us3d_ug_bin_ex")
         b = UGBinning(ws, cap, -1, frames, G, float(chi2), float(beta), bool(sort_by_depth), cull)
@@ -176,8 +194,54 @@ def bin_gaussians(means: torch.Tensor, tril: torch.Tensor, opac: torch.Tensor, i
             raise RuntimeError("us3d_ug_bin: inconsistent frame table")
         b.total = total
         if not flags:
-            _capacity_hint[key] = max(4096, int(total * 1.25) + 1024)
+            # a retry may have been for the (Gaussian, frame) pairs, which the total does not tell
+            _capacity_hint[key] = max(4096, int(total * 1.25) + 1024, cap if _attempt else 0)
             return b
+        if total > 0x7FFFFFFF:
+            raise RuntimeError(f"us3d_ug_bin: {total} instances exceed the int32 index range")
+        cap = int(total * 1.25) + 1024
+    raise RuntimeError("us3d_ug_bin: capacity retry failed")
+
+
+def _bin_flags(cull: bool, logit_attributes: bool, frames: FrameTable) -> int:
+    return ((_lib.UG_BIN_SLICE_CULL if cull else 0) | (_lib.UG_BIN_LOGIT_ATTRIBUTES if logit_attributes else 0)
+            | (_lib.UG_BIN_GAUSSIAN_SETS if frames.gaussian_sets else 0))
+
+
+def bin_forward(means: torch.Tensor, tril: torch.Tensor, opac: torch.Tensor, inten: torch.Tensor, frames: FrameTable,
+                chi2: float, beta: float, sort_by_depth: bool, pixels: torch.Tensor, bg_alpha: float,
+                bg_intensity: float, slice_cull: bool, want_counts: bool, capacity: Optional[int] = None):
+    """``bin_gaussians`` and ``forward`` in one call that checks the binning while the shading runs;
+    returns (binning, image, alpha, depth, counts)."""
+    G = _check_params(means, tril, opac, inten)
+    dev, P = pixels.device, frames.n_pixels
+    _set_device(means.device)
+    key = (G, frames.n_tiles, slice_cull)
+    cap = int(capacity if capacity is not None else _capacity_hint.get(key, max(4096, 4 * G)))
+    image = torch.empty(P, dtype=torch.float32, device=dev)
+    alpha = torch.empty(P, dtype=torch.float32, device=dev)
+    depth = torch.empty(P, dtype=torch.float32, device=dev)
+    counts = torch.empty(P, dtype=torch.int32, device=dev) if (want_counts and not slice_cull) else None
+    c_total, c_tasks, c_flags = ctypes.c_int64(0), ctypes.c_int64(0), ctypes.c_int32(0)
+    for _attempt in range(3):
+        nbytes = int(_lib.call("us3d_ug_workspace_bytes", G, frames.n_frames, frames.n_tiles, P, cap))
+        ws = torch.empty(nbytes, dtype=torch.uint8, device=means.device)
+        st = _lib.call(
+            "us3d_ug_bin_forward", _ptr(ws), nbytes, _ptr(frames.table), frames.n_frames, frames.n_tiles, P, G,
+            _ptr(means), _ptr(tril), _ptr(opac), _ptr(inten), float(chi2), float(beta), int(bool(sort_by_depth)), cap,
+            _ptr(pixels), _bin_flags(slice_cull, False, frames), float(bg_alpha), float(bg_intensity), _ptr(image),
+            _ptr(alpha), _ptr(depth), _ptr(counts), ctypes.byref(c_total), ctypes.byref(c_tasks),
+            ctypes.byref(c_flags), _stream(),
+        )
+        _lib.check(st, "us3d_ug_bin_forward")
+        total, flags = int(c_total.value), int(c_flags.value)
+        if flags & 2:
+            raise RuntimeError("us3d_ug_bin: inconsistent frame table")
+        if not flags:
+            # the capacity also bounds the (Gaussian, frame) pairs: a quarter of it and 4096
+            _capacity_hint[key] = max(4096, int(max(total, 4 * (int(c_tasks.value) - 4096)) * 1.25) + 1024)
+            return (UGBinning(ws, cap, total, frames, G, float(chi2), float(beta), bool(sort_by_depth), slice_cull,
+                              pixels, counts), image, alpha, depth, counts)
         if total > 0x7FFFFFFF:
             raise RuntimeError(f"us3d_ug_bin: {total} instances exceed the int32 index range")
         cap = int(total * 1.25) + 1024
@@ -226,8 +290,8 @@ def _backward_scratch(dev: torch.device, nbytes: int) -> torch.Tensor:
     if torch.cuda.is_current_stream_capturing():
         # a graph keeps its own (private pool) buffer: the cached one may be freed later
         return torch.empty(max(nbytes, 16), dtype=torch.uint8, device=dev)
-    key = (dev.index if dev.index is not None else torch.cuda.current_device(),
-           torch.cuda.current_stream(dev).cuda_stream)
+    index = dev.index if dev.index is not None else torch.cuda.current_device()
+    key = (index, torch._C._cuda_getCurrentRawStream(index))
     buf = _SCRATCH.get(key)
     if buf is None or buf.numel() < nbytes:
         _SCRATCH.pop(key, None)
@@ -241,10 +305,11 @@ def release_scratch() -> None:
     _SCRATCH.clear()
 
 
-def backward(b: UGBinning, pixels: torch.Tensor, d_image: torch.Tensor, d_alpha: torch.Tensor,
-             d_depth: torch.Tensor, saved_alpha: torch.Tensor, bg_alpha: float, bg_intensity: float,
-             scratch: Optional[torch.Tensor] = None, out=None):
-    """Gradients w.r.t. means (G,3), precision_tril (G,6), opacities (G,), intensities (G,)."""
+def backward(b: UGBinning, pixels: torch.Tensor, d_image: torch.Tensor, d_alpha: Optional[torch.Tensor],
+             d_depth: Optional[torch.Tensor], saved_alpha: torch.Tensor, bg_alpha: float, bg_intensity: float,
+             scratch: Optional[torch.Tensor] = None, out=None, absent_zero: bool = False):
+    """Gradients w.r.t. means (G,3), precision_tril (G,6), opacities (G,), intensities (G,). With
+    ``absent_zero``, ``d_alpha`` and ``d_depth`` may be None: zeros."""
     G = b.n_gauss
     dev = pixels.device
     sbytes = int(_lib.call("us3d_ug_backward_scratch_bytes", b.capacity))
@@ -259,7 +324,7 @@ def backward(b: UGBinning, pixels: torch.Tensor, d_image: torch.Tensor, d_alpha:
         )
     dm, dt, do, di = out
     st = _lib.call(
-        "us3d_ug_backward", _ptr(b.workspace), _ptr(b.frames.table), b.frames.n_frames, b.frames.n_tiles,
+        "us3d_ug_backward_ex" if absent_zero else "us3d_ug_backward", _ptr(b.workspace), _ptr(b.frames.table), b.frames.n_frames, b.frames.n_tiles,
         b.frames.n_pixels, G, b.capacity, _ptr(pixels), _ptr(d_image), _ptr(d_alpha), _ptr(d_depth),
         _ptr(saved_alpha), b.chi2, b.beta, float(bg_alpha), float(bg_intensity), _ptr(scratch), int(scratch.numel()),
         _ptr(dm), _ptr(dt), _ptr(do), _ptr(di), _stream(),

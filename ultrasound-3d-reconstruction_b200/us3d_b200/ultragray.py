@@ -16,12 +16,9 @@ from typing import Optional
 import torch
 
 from . import _lib
+from ._alloc import current_stream as _stream
 
 _capacity_hint: dict = {}
-
-
-def _stream() -> int:
-    return torch.cuda.current_stream().cuda_stream
 
 
 def _f32(t: torch.Tensor, dev) -> torch.Tensor:
@@ -65,19 +62,17 @@ def forward(means, scales, quats, attenuations, sh_coeffs, pixel_positions, ray_
     for _ in range(3):
         nbytes = int(_lib.call("us3d_ugr_workspace_bytes", G, W, H, cap))
         ws = torch.empty(nbytes, dtype=torch.uint8, device=dev)
-        st = _lib.call("us3d_ugr_forward", ws.data_ptr(), nbytes, G, means.data_ptr(), scales.data_ptr(),
+        total, flags = ctypes.c_int64(0), ctypes.c_int32(0)
+        st = _lib.call("us3d_ugr_forward_checked", ws.data_ptr(), nbytes, G, means.data_ptr(), scales.data_ptr(),
                        quats.data_ptr(), attenuations.data_ptr(), sh_coeffs.data_ptr(), pixel_positions.data_ptr(),
                        ray_origins.data_ptr(), ray_dirs.data_ptr(), origin.data_ptr(), axis_lateral.data_ptr(),
                        axis_elevational.data_ptr(), axis_axial.data_ptr(), ray_perturbations.data_ptr(), W, H,
                        float(p.width_mm), float(p.near_mm), float(p.lateral_col_offset), float(p.elev_cutoff_mm),
                        float(p.k_sigma), float(p.quadrature_window_radius_mm),
                        1 if p.local_transmission_window_only else 0, float(p.local_transmission_max_window_mm), cap,
-                       image.data_ptr(), _stream())
+                       image.data_ptr(), ctypes.byref(total),
+                       ctypes.byref(flags), _stream())
         _lib.check(st, "us3d_ugr_forward")
-        total = ctypes.c_int64(0)
-        flags = ctypes.c_int32(0)
-        _lib.check(_lib.call("us3d_ugr_read_status", ws.data_ptr(), ctypes.byref(total), ctypes.byref(flags),
-                             _stream()), "us3d_ugr_read_status")
         if flags.value == 0:
             _capacity_hint[key] = max(4096, int(total.value * 1.25) + 1024)
             return image, UGRBinning(ws, cap, int(total.value), G, W, H)
