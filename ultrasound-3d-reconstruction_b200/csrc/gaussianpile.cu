@@ -24,6 +24,10 @@
 // are bit-exact and images match to rounding of the summation.
 #include <algorithm>
 
+#include <float.h>
+#include <type_traits>
+
+#include "f32x2.cuh"
 #include "us3d_common.cuh"
 #include "scan.cuh"
 #include "binning.cuh"
@@ -366,122 +370,179 @@ preprocess_kernel(int64_t G, int H, int W, int tile, int tiles_x, int tiles_y, f
 // Forward
 // ------------------------------------------------------------------------------------
 
-// One block per tile, or per 1/SPLIT of a tile, with PARTS threads per pixel (the block's
-// pixels rounded up to whole warps, times PARTS); candidates of the tile list are staged in
-// shared memory. The sum over a pixel's candidates is split by Gaussian index into four classes
-// (g mod 4), each summed in list order, and the class sums are added as ((c0 + c1) + c2) + c3;
-// thread part p of a pixel owns the classes congruent to p mod PARTS. The grouping depends on
-// neither PARTS, SPLIT nor the tile size, so the image does not either (the reference sums the
-// whole list in order, src/shader/forward.cu:88-210: the results agree up to rounding). SPLIT
-// > 1 serves small frames: a 256x256 slice has 256 tiles, under two 1024-thread blocks per SM,
-// while quarter tiles give 1024 blocks of 256 threads that the SMs can balance.
-template <int PARTS, int SPLIT>
-__global__ void forward_kernel(int H, int W, int tile, int tiles_x, const float* __restrict__ grid,
-                               const float* __restrict__ params, const int* __restrict__ tile_start,
-                               const int* __restrict__ sorted_gid, const long long* __restrict__ header,
-                               const float4* __restrict__ cand, float* __restrict__ image) {
-    constexpr int PER = 4 / PARTS;  // classes per thread
-    __shared__ float4 sc0[FWD_BATCH], sc1[FWD_BATCH];
-    __shared__ float2 sc2[FWD_BATCH];
+// One block of four warps per 8x4 block of a tile's pixels. The sum over a pixel's candidates is split by
+// Gaussian index into 16 classes (g mod 16), each summed in list order, and the class sums are added
+// in class order. The grouping does not depend on the tile size, so the image does not either (the
+// reference sums the whole list in order, src/shader/forward.cu:88-210: the results agree up to rounding).
+//
+// Every batch of candidates is tested once (its box against the pixel block's extent, with a margin for the
+// rounding of the per-pixel test) and queued by class, in list order. A quarter-warp then walks its
+// class's queue, lane l holding the four pixels of column l in packed FP32 pairs: four candidates are
+// visited by one instruction, and the lateral part of the test and of the quadratic form is formed once
+// for four pixels. With one candidate and one pixel per lane the kernel executed 226M warp instructions for
+// a 256x256 slice of 200k Gaussians, in 711 us; 117M and 268 us so, bound by issue and, at the end, by the
+// blocks with the longest lists (1.5 times the mean). 768x768, 200k: 2.10 -> 0.91 ms. Two, four and eight
+// pixel blocks sharing the staged candidates took 315, 394 and 535 us (more warps wait for each
+// batch); 8 classes 336 us, 32 classes 314 us; batches of 128 / 512 337 / 328 us; unrolled 1 / 2 / 4 times
+// 331 / 305 / 272 us; compiled for 10 / 12 blocks per SM 319 / 341 us.
+constexpr int CLASSES = 16, GROUP_WARPS = CLASSES / 4, GROUP = GROUP_WARPS * 32;
+constexpr int FWD_CTAS = 8;
+constexpr int BLK_W = 8, BLK_H = 4;
+constexpr int FWD_ROUNDS = FWD_BATCH / 32;  // warp-wide tests of a batch
+static_assert(FWD_BATCH <= 256 && FWD_ROUNDS % 4 == 0 && FWD_ROUNDS % GROUP_WARPS == 0, "queue entries and counts are bytes");
+
+__global__ void __launch_bounds__(GROUP, FWD_CTAS)
+forward_kernel(int H, int W, int tile, int tiles_x, const float* __restrict__ grid, const float* __restrict__ params,
+               const int* __restrict__ tile_start, const int* __restrict__ sorted_gid,
+               const long long* __restrict__ header, const float4* __restrict__ cand, float* __restrict__ image) {
+    __shared__ float4 sc0[FWD_BATCH + 1], sc1[FWD_BATCH + 1];  // the last candidate reaches no pixel
+    __shared__ float2 sc2[FWD_BATCH + 1];
     __shared__ unsigned char s_cls[FWD_BATCH];
-    __shared__ float s_class_sum[4 * 1024 / PARTS];
+    __shared__ unsigned s_cnt[CLASSES][FWD_ROUNDS / 4];  // per class: a byte per warp-wide test, its candidates
+    __shared__ __align__(16) unsigned char s_queue[CLASSES][FWD_BATCH];
+    static_assert(sizeof(s_queue) >= sizeof(float) * CLASSES * BLK_W * BLK_H, "the class sums reuse the queues");
     if (header[H_FLAGS] != 0) return;
-    const int t = blockIdx.x / SPLIT, sub = blockIdx.x % SPLIT;
+    const int bx = (tile + BLK_W - 1) / BLK_W, by = (tile + BLK_H - 1) / BLK_H;
+    const int t = blockIdx.x / (bx * by), kb = blockIdx.x % (bx * by);  // tile and its pixel block
     const int tx = t % tiles_x, ty = t / tiles_x;
-    // pixel slots per part (whole warps); with SPLIT > 1 the host guarantees tile^2 / SPLIT is
-    // a multiple of 32, so the sub-blocks partition the tile
-    const int npix = SPLIT == 1 ? (tile * tile + 31) / 32 * 32 : tile * tile / SPLIT;
-    const int slot = threadIdx.x % npix + sub * npix, part = threadIdx.x / npix;
-    const int lx = slot % tile, ly = slot / tile;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, col = lane & (BLK_W - 1);
+    const int cls = warp * 4 + (lane >> 3);
+    const int lx = (kb % bx) * BLK_W + col, ly = (kb / bx) * BLK_H;
     const int x = tx * tile + lx, y = ty * tile + ly;
-    // the extra slots of the last warp own no pixel
-    const bool valid = slot < tile * tile && (x < W) && (y < H);
+    const bool col_ok = lx < tile && x < W;
     const float weight_min = params[UF_WEIGHT_MIN];
-    float xi_lat = 0.f, xi_ax = 0.f;
-    if (valid) {
-        xi_lat = (static_cast<float>(x) - grid[SG_LAT_COL_OFFSET]) * grid[SG_DELTA_LAT_MM];
-        xi_ax = static_cast<float>(y) * grid[SG_DELTA_AX_MM] + grid[SG_NEAR_MM];
+    const float xi_lat = (static_cast<float>(x) - grid[SG_LAT_COL_OFFSET]) * grid[SG_DELTA_LAT_MM];
+    float xi_ax[BLK_H];
+    // the block's extent in mm
+    float lat_lo = 3.0e38f, lat_hi = -3.0e38f, ax_lo = 3.0e38f, ax_hi = -3.0e38f;
+#pragma unroll
+    for (int r = 0; r < BLK_H; ++r) {
+        xi_ax[r] = static_cast<float>(y + r) * grid[SG_DELTA_AX_MM] + grid[SG_NEAR_MM];
+        if (col_ok && ly + r < tile && y + r < H) {
+            lat_lo = lat_hi = xi_lat;
+            ax_lo = fminf(ax_lo, xi_ax[r]);
+            ax_hi = fmaxf(ax_hi, xi_ax[r]);
+        }
     }
-    const int s0 = tile_start[t], n = tile_start[t + 1] - s0;
-    float acc[PER];
 #pragma unroll
-    for (int c = 0; c < PER; ++c) acc[c] = 0.f;
-    const int nthreads = blockDim.x;
-    // The warp's pixel extent in mm: a candidate whose box misses it (with a margin for the
-    // rounding of the per-pixel test) is skipped by the whole warp.
-    const int lane = threadIdx.x & 31;
-    float lat_lo = valid ? xi_lat : 3.0e38f, lat_hi = valid ? xi_lat : -3.0e38f;
-    float ax_lo = valid ? xi_ax : 3.0e38f, ax_hi = valid ? xi_ax : -3.0e38f;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
+    for (int o = 1; o < BLK_W; o <<= 1) {
         lat_lo = fminf(lat_lo, __shfl_xor_sync(0xffffffffu, lat_lo, o));
         lat_hi = fmaxf(lat_hi, __shfl_xor_sync(0xffffffffu, lat_hi, o));
         ax_lo = fminf(ax_lo, __shfl_xor_sync(0xffffffffu, ax_lo, o));
         ax_hi = fmaxf(ax_hi, __shfl_xor_sync(0xffffffffu, ax_hi, o));
     }
+    const f32x2 AX0 = pk2(xi_ax[0], xi_ax[1]), AX1 = pk2(xi_ax[2], xi_ax[3]);
+    const f32x2 CE = dup2(-0.72134752044448170f);  // -log2(e) / 2
+    const int s0 = tile_start[t], n = tile_start[t + 1] - s0;
+    f32x2 acc0 = dup2(0.f), acc1 = acc0;
+    if (threadIdx.x == 0) {
+        sc0[FWD_BATCH] = make_float4(0.f, 0.f, 0.f, 0.f);
+        sc1[FWD_BATCH] = make_float4(0.f, 0.f, 0.f, -1.f);
+        sc2[FWD_BATCH] = make_float2(-1.f, 0.f);
+    }
+    const unsigned char* queue = s_queue[cls];
     for (int b0 = 0; b0 < n; b0 += FWD_BATCH) {
         const int nb = min(FWD_BATCH, n - b0);
         __syncthreads();
-        for (int j = threadIdx.x; j < nb; j += nthreads) {
+        for (int j = threadIdx.x; j < nb; j += GROUP) {
             const int g = sorted_gid[s0 + b0 + j];
             sc0[j] = cand[3 * g];
             sc1[j] = cand[3 * g + 1];
             const float4 c2 = cand[3 * g + 2];
             sc2[j] = make_float2(c2.x, c2.y);
-            s_cls[j] = (unsigned char)(g & 3);
+            s_cls[j] = (unsigned char)(g % CLASSES);
         }
+        if (threadIdx.x < CLASSES * (FWD_ROUNDS / 4)) (&s_cnt[0][0])[threadIdx.x] = 0u;
         __syncthreads();
-        for (int jc = 0; jc < nb; jc += 32) {
+        // the candidates that reach this pixel block, queued by class in list order
+        int place[FWD_ROUNDS / GROUP_WARPS], of[FWD_ROUNDS / GROUP_WARPS];
+#pragma unroll
+        for (int i = 0; i < FWD_ROUNDS / GROUP_WARPS; ++i) {
+            const int round = i * GROUP_WARPS + warp, j = round * 32 + lane;
             bool near = false;
-            const int jl = jc + lane;
-            if (jl < nb && (PARTS == 1 || (int)(s_cls[jl] % PARTS) == part)) {
-                const float2 c2 = sc2[jl];
-                const float4 c0 = sc0[jl];
-                const float rl = sc1[jl].w;
+            if (j < nb) {
+                const float4 c0 = sc0[j];
+                const float2 c2 = sc2[j];
+                const float rl = sc1[j].w;
                 const float ml = 1e-5f * (fabsf(c0.z) + rl + fabsf(lat_lo) + fabsf(lat_hi)) + 1e-30f;
                 const float ma = 1e-5f * (fabsf(c0.w) + c2.x + fabsf(ax_lo) + fabsf(ax_hi)) + 1e-30f;
                 near = c2.y != 0.f && lat_hi >= c0.z - rl - ml && lat_lo <= c0.z + rl + ml &&
                        ax_hi >= c0.w - c2.x - ma && ax_lo <= c0.w + c2.x + ma;
             }
-            unsigned bits = __ballot_sync(0xffffffffu, near);
-            if (!valid) continue;
-            while (bits != 0u) {
-                const int j = jc + __ffs(bits) - 1;
-                bits &= bits - 1u;
-                const float2 c2 = sc2[j];
-                const float4 c0 = sc0[j];
-                const float4 c1 = sc1[j];
-                if (fabsf(xi_lat - c0.z) > c1.w || fabsf(xi_ax - c0.w) > c2.x) continue;
-                const float dlat = xi_lat - c0.z;
-                const float dax = xi_ax - c0.w;
-                const float qlat = c1.x * dlat + c1.y * dax;
-                const float qax = c1.y * dlat + c1.z * dax;
-                const float quad = dlat * qlat + dax * qax;
-                if (!(quad >= 0.f) || !isfinite(quad)) continue;
-                const float weight = c0.x * expf(-0.5f * quad);
-                if (!isfinite(weight) || weight < weight_min) continue;
-                const float v = c0.y * weight;
-                if (PER == 1) {
-                    acc[0] += v;
-                } else {
-                    const int k = s_cls[j] / PARTS;  // this thread's class index
-#pragma unroll
-                    for (int c = 0; c < PER; ++c)
-                        if (c == k) acc[c] += v;
-                }
-            }
+            of[i] = near ? s_cls[j] : CLASSES;
+            const unsigned same = __match_any_sync(0xffffffffu, of[i]);
+            place[i] = __popc(same & ((1u << lane) - 1u));
+            if (near && place[i] == 0)
+                reinterpret_cast<unsigned char*>(s_cnt[of[i]])[round] = (unsigned char)__popc(same);
         }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < FWD_ROUNDS / GROUP_WARPS; ++i) {
+            if (of[i] == CLASSES) continue;
+            const int round = i * GROUP_WARPS + warp;
+            int pos = place[i];
+#pragma unroll
+            for (int w = 0; w < FWD_ROUNDS / 4; ++w) {
+                const int in = min(max(round - 4 * w, 0), 4);  // rounds of this word that come before
+                pos = __dp4a(s_cnt[of[i]][w], (unsigned)(0x01010101ull & ((1ull << (8 * in)) - 1ull)), (unsigned)pos);
+            }
+            s_queue[of[i]][pos] = (unsigned char)(round * 32 + lane);
+        }
+        int n_mine = 0;
+#pragma unroll
+        for (int w = 0; w < FWD_ROUNDS / 4; ++w) n_mine = __dp4a(s_cnt[cls][w], 0x01010101u, (unsigned)n_mine);
+        int n_max = max(n_mine, __shfl_xor_sync(0xffffffffu, n_mine, 8));
+        n_max = max(n_max, __shfl_xor_sync(0xffffffffu, n_max, 16));
+        __syncthreads();
+        // With a positive weight_min an infinite quad fails the weight test by itself.
+        auto run = [&](auto positive_t) {
+            constexpr bool POSITIVE = decltype(positive_t)::value;
+#pragma unroll 8
+            for (int k = 0; k < n_max; ++k) {
+                const int j = k < n_mine ? queue[k] : FWD_BATCH;
+                const float4 c0 = sc0[j], c1 = sc1[j];
+                const float r_ax = sc2[j].x;
+                const float dlat = xi_lat - c0.z;
+                const float lim = fabsf(dlat) <= c1.w ? r_ax : -1.f;
+                const f32x2 L = dup2(dlat), QL0 = dup2(c1.x * dlat), QA0 = dup2(c1.y * dlat);
+                auto rows = [&](f32x2 AX, f32x2& acc) {
+                    const f32x2 D = sub2(AX, dup2(c0.w));
+                    const f32x2 QL = fma2(dup2(c1.y), D, QL0), QA = fma2(dup2(c1.z), D, QA0);
+                    const f32x2 Q = fma2(D, QA, mul2(L, QL));
+                    const f32x2 Wt = mul2(dup2(c0.x), ex2_2(mul2(Q, CE)));
+                    float d0, d1, q0, q1, w0, w1, v0, v1;
+                    up2(D, d0, d1);
+                    up2(Q, q0, q1);
+                    up2(Wt, w0, w1);
+                    up2(mul2(dup2(c0.y), Wt), v0, v1);
+                    const bool k0 = fabsf(d0) <= lim && q0 >= 0.f && (POSITIVE || q0 <= FLT_MAX) && w0 >= weight_min;
+                    const bool k1 = fabsf(d1) <= lim && q1 >= 0.f && (POSITIVE || q1 <= FLT_MAX) && w1 >= weight_min;
+                    acc = add2(acc, pk2(k0 ? v0 : 0.f, k1 ? v1 : 0.f));
+                };
+                rows(AX0, acc0);
+                rows(AX1, acc1);
+            }
+        };
+        if (weight_min > 0.f)
+            run(std::true_type{});
+        else
+            run(std::false_type{});
     }
-    // class c's sum sits in part c % PARTS, slot c / PARTS of its accumulators
-    const int ls = slot - sub * npix;  // the slot within this block
-#pragma unroll
-    for (int c = 0; c < PER; ++c) s_class_sum[(c * PARTS + part) * npix + ls] = acc[c];
     __syncthreads();
-    if (part != 0 || !valid) return;
-    float total = s_class_sum[ls];
+    float(*s_sum)[BLK_W * BLK_H] = reinterpret_cast<float(*)[BLK_W * BLK_H]>(&s_queue[0][0]);
+    float v[BLK_H];
+    up2(acc0, v[0], v[1]);
+    up2(acc1, v[2], v[3]);
 #pragma unroll
-    for (int c = 1; c < 4; ++c) total += s_class_sum[c * npix + ls];
-    image[y * W + x] = total;
+    for (int r = 0; r < BLK_H; ++r) s_sum[cls][r * BLK_W + col] = v[r];
+    __syncthreads();
+    if (warp != 0 || !col_ok) return;
+    const int r = lane >> 3;  // warp 0: lane (row, column)
+    if (ly + r >= tile || y + r >= H) return;
+    float total = s_sum[0][lane];
+#pragma unroll
+    for (int c = 1; c < CLASSES; ++c) total += s_sum[c][lane];
+    image[(y + r) * W + x] = total;
 }
 
 // ------------------------------------------------------------------------------------
@@ -1123,21 +1184,9 @@ static int gp_forward_impl(void* workspace, size_t workspace_bytes, int64_t n_ga
         const int rc = status->record(w.header, stream);
         if (rc != US3D_OK) return rc;
     }
-    // up to four threads per pixel (a whole-warp pixel block of at most 1024 threads); frames
-    // with fewer than four tiles per SM split each tile over four blocks when it divides into
-    // whole warps
-    const int npix = (tile_size * tile_size + 31) / 32 * 32;
-    auto launch = [&](auto kernel, int parts, int split) {
-        kernel<<<(unsigned)(T * split), npix / split * parts, 0, stream>>>(
-            H, W, tile_size, tx, grid_pack, focus_params, w.tile_start, w.sorted_gid, w.header, w.cand, out_image);
-    };
-    const bool split4 = T < 4 * 148 && (tile_size * tile_size) % 128 == 0;
-    if (npix <= 256)
-        split4 ? launch(forward_kernel<4, 4>, 4, 4) : launch(forward_kernel<4, 1>, 4, 1);
-    else if (npix <= 512)
-        split4 ? launch(forward_kernel<2, 4>, 2, 4) : launch(forward_kernel<2, 1>, 2, 1);
-    else
-        split4 ? launch(forward_kernel<1, 4>, 1, 4) : launch(forward_kernel<1, 1>, 1, 1);
+    const int blocks = ((tile_size + BLK_W - 1) / BLK_W) * ((tile_size + BLK_H - 1) / BLK_H);  // pixel blocks per tile
+    forward_kernel<<<(unsigned)(T * blocks), GROUP, 0, stream>>>(H, W, tile_size, tx, grid_pack, focus_params,
+                                                                 w.tile_start, w.sorted_gid, w.header, w.cand, out_image);
     US3D_CHECK_LAUNCH("gp forward");
     prof_end(prof, stream);
     count_launches(1 + (n_gauss > 0) + bins_launches(n_gauss, T, w.keys == nullptr, sort_by_v != 0) + 1);
