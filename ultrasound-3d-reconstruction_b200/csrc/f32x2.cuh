@@ -35,6 +35,7 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
     asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
     return r;
 }
+__device__ __forceinline__ f32x2 neg2(f32x2 v) { return v ^ 0x8000000080000000ull; }
 __device__ __forceinline__ f32x2 dup2(float v) { return pk2(v, v); }
 __device__ __forceinline__ f32x2 lo2(const float4& v) { return pk2(v.x, v.y); }
 __device__ __forceinline__ f32x2 hi2(const float4& v) { return pk2(v.z, v.w); }

@@ -45,7 +45,7 @@ enum { UF_SIGMA_ELE_0 = 0, UF_SIGMA_ELE_1 = 1, UF_SIGMA_ELE_MIN = 2, UF_SIGMA_EL
        UF_WEIGHT_MIN = 10, UF_USE_LATERAL_FOCUS = 11, UF_INFLATE_LAT_MM = 12, UF_INFLATE_AX_MM = 13 };
 
 constexpr int FWD_BATCH = 256;
-constexpr int PARTIAL_F4 = 5;  // per-instance partial record: 20 floats
+constexpr int PARTIAL_F4 = 3;  // per-instance partial record: nine moments in 12 floats
 constexpr float GRAD_CLAMP = 1e3f;
 
 struct Workspace {
@@ -515,8 +515,8 @@ forward_kernel(int H, int W, int tile, int tiles_x, const float* __restrict__ gr
                     up2(Q, q0, q1);
                     up2(Wt, w0, w1);
                     up2(mul2(dup2(c0.y), Wt), v0, v1);
-                    const bool k0 = fabsf(d0) <= lim && q0 >= 0.f && (POSITIVE || q0 <= FLT_MAX) && w0 >= weight_min;
-                    const bool k1 = fabsf(d1) <= lim && q1 >= 0.f && (POSITIVE || q1 <= FLT_MAX) && w1 >= weight_min;
+                    const bool k0 = fabsf(d0) <= lim && q0 >= 0.f && (POSITIVE || q0 <= FLT_MAX) && !(w0 < weight_min);
+                    const bool k1 = fabsf(d1) <= lim && q1 >= 0.f && (POSITIVE || q1 <= FLT_MAX) && !(w1 < weight_min);
                     acc = add2(acc, pk2(k0 ? v0 : 0.f, k1 ? v1 : 0.f));
                 };
                 rows(AX0, acc0);
@@ -549,41 +549,47 @@ forward_kernel(int H, int W, int tile, int tiles_x, const float* __restrict__ gr
 // Backward
 // ------------------------------------------------------------------------------------
 
-// Per-instance partial record (20 floats); only the sufficient statistics that can be
-// non-zero for the additive us_focus footprint are kept (the reference's 35-float
-// workspace carries structurally zero entries).
-enum { P_MU_PROBE1 = 0, P_MU_PROBE2, P_SC22, P_MU_E0, P_MU_E1, P_SE00, P_SE01, P_SE11, P_OPACITY, P_INTENSITY,
-       P_FP_MU2_LAT, P_FP_MU2_AX, P_FP_INV00, P_FP_INV01, P_FP_INV11, P_FP_DET2, P_FP_MU_ELE, P_FP_SC22,
-       P_FP_SIGMA_ELE, P_COUNT };
+// Every term of a Gaussian's adjoint is a fixed combination of nine sums over its contributing pixels, which an
+// instance's record holds: ub = up * bno (bno = the weight without the opacity) times q_lat, q_ax,
+// q_lat^2, q_lat q_ax, q_ax^2 (q = inv2 d), dlat^2, dlat dax, dax^2 and 1. The finalize
+// forms the terms (the reference keeps 35 of them per instance).
+// The q-weighted sums are taken per pixel, not expanded from moments of d: for an elongated
+// footprint q nearly cancels along the long axis, and the expansion inv00^2 S(dlat^2) + 2 inv00 inv01
+// S(dlat dax) + ... loses in fp32 the digits that the chain through Se and Lc (with entries in
+// the hundreds for such footprints) then amplifies.
+enum { M_QL = 0, M_QA, M_QLL, M_QLA, M_QAA, M_XX, M_XY, M_YY, M_ONE, M_COUNT };
 
-// One warp per instance of the sorted instance list (tile by tile): the lanes share the
-// pixels of the footprint's bounding box within the instance's tile and accumulate the
-// per-pixel adjoint of the footprint (reference src/shader/us_focus.cu:398-477, 805-966); the
-// 19 sums are then reduced over the warp in a fixed order. The footprints are the forward's
-// (cached per Gaussian by the preprocess).
+// One half-warp per instance of the sorted instance list (tile by tile): its lanes share the pixels of the
+// footprint's bounding box within the instance's tile, lane l the pixels l and l + 16 of every 32 in a packed
+// FP32 pair, and accumulate the per-pixel adjoint of the footprint (reference src/shader/us_focus.cu:398-477,
+// 805-966); the sums are then reduced over the half-warp in a fixed order. The footprints are the
+// forward's (cached per Gaussian by the preprocess). A whole warp per instance, one pixel per lane and
+// 19 terms written per instance executed 369M warp instructions for a 256x256 slice of 200k Gaussians, at
+// 74 % of the issue rate, a good part of them for the reduction and the terms: 453 us, and 16 us to sum the
+// records. With half-warps, the box walked in floats and nine moments per instance 282 us, bound by
+// issue (72 %); the finalize, which now forms the terms, 44 -> 61 us.
 constexpr int BWD_WARPS = 8;  // warps per CTA
 
 __global__ void __launch_bounds__(BWD_WARPS * 32, 4)
 backward_inst_kernel(int T, int W, int tile, int tiles_x, const float* __restrict__ opac,
-                     const float* __restrict__ inten, const float4* __restrict__ bfp,
+                     const float4* __restrict__ bfp,
                      const float* __restrict__ grid, const float* __restrict__ params,
                      const int* __restrict__ tile_start, const int* __restrict__ sorted_gid,
                      const int* __restrict__ sorted_inst, const long long* __restrict__ header,
                      const float* __restrict__ grad_image, float* __restrict__ partial, int H) {
     if (header[H_FLAGS] != 0) return;
-    const int lane = threadIdx.x & 31;
-    const int64_t total = tile_start[T];
-    const float det_gamma = params[UF_DET_GAMMA];
+    const int lane = threadIdx.x & 31, l = lane & 15, half = lane >> 4;
+    const int total = tile_start[T];
     const float weight_min = params[UF_WEIGHT_MIN];
     const float lat_delta = grid[SG_DELTA_LAT_MM], ax_delta = grid[SG_DELTA_AX_MM];
     const float col_off = grid[SG_LAT_COL_OFFSET], near_mm = grid[SG_NEAR_MM];
     // Each warp owns a contiguous run of instances, so the instance's tile (the last t with
     // tile_start[t] <= k; empty tiles share a start) is found by one binary search per warp and
     // then followed forward as k advances.
-    const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t chunk = (total + n_warps - 1) / n_warps;
-    const int64_t k_begin = wid * chunk, k_end = min(total, k_begin + chunk);
+    const int n_warps = (int)(gridDim.x * blockDim.x) >> 5;
+    const int wid = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int chunk = (int)(((int64_t)total + n_warps - 1) / n_warps);
+    const int k_begin = (int)min((int64_t)total, (int64_t)wid * chunk), k_end = min(total - k_begin, chunk) + k_begin;
     int t = 0;
     if (k_begin < k_end) {
         int lo = 0, hi = T;
@@ -593,140 +599,132 @@ backward_inst_kernel(int T, int W, int tile, int tiles_x, const float* __restric
         }
         t = lo;
     }
-    for (int64_t k = k_begin; k < k_end; ++k) {
-        while (t + 1 < T && tile_start[t + 1] <= k) ++t;
-        const int tx = t % tiles_x, ty = t / tiles_x;
-        const int x0 = tx * tile, y0 = ty * tile;
-        const int x1 = min(W, (tx + 1) * tile), y1 = min(H, (ty + 1) * tile);
+    const f32x2 CE = dup2(-0.72134752044448170f);  // -log2(e) / 2
+    int x0 = 0, y0 = 0, x1 = 0, y1 = 0, t_end = k_begin < k_end ? k_begin : 0;
+    for (int k0 = k_begin; k0 < k_end; k0 += 2) {
+        const bool live = half < k_end - k0;
+        const int k = live ? k0 + half : k0;
+        if (k >= t_end) {  // another tile (the first one included)
+            while (t + 1 < T && (t_end = tile_start[t + 1]) <= k) ++t;
+            t_end = tile_start[t + 1];
+            const int tx = t % tiles_x, ty = t / tiles_x;
+            x0 = tx * tile;
+            y0 = ty * tile;
+            x1 = min(W, x0 + tile);
+            y1 = min(H, y0 + tile);
+        }
         const int g = sorted_gid[k];
         const float4 f0 = bfp[4 * (int64_t)g], f1 = bfp[4 * (int64_t)g + 1];
-        const float4 f2 = bfp[4 * (int64_t)g + 2], f3 = bfp[4 * (int64_t)g + 3];
         const float mu2_lat = f0.x, mu2_ax = f0.y, r_lat = f0.z, r_ax = f0.w;
         const float inv00 = f1.x, inv01 = f1.y, inv11 = f1.z, bno_const = f1.w;
-        const float s2_00 = f2.x, s2_01 = f2.y, s2_11 = f2.z, inv_det_norm = f2.w;
-        const float mu_ele = f3.x, inv_de = f3.y, dse_dax = f3.z, sigma_ele = f3.w;
-        // Every term of the per-instance partial is a fixed combination of nine sums over the
-        // contributing pixels of ub = up * bno (bno = the weight without the opacity) times 1,
-        // q_lat, q_ax, q_lat^2, q_lat q_ax, q_ax^2 (q = inv2 d) and dlat^2, dlat dax, dax^2: the
-        // lanes accumulate those and the terms are formed once. The q-weighted sums are taken
-        // per pixel, not expanded from moments of d: for an elongated footprint q nearly
-        // cancels along the long axis, and the expansion inv00^2 S(dlat^2) + 2 inv00 inv01
-        // S(dlat dax) + ... loses in fp32 the digits that the chain through Se and Lc (with
-        // entries in the hundreds for such footprints) then amplifies.
-        float m0 = 0.f, sl = 0.f, sa = 0.f, sll = 0.f, sla = 0.f, saa = 0.f, mxx = 0.f, mxy = 0.f, myy = 0.f;
-        float o = 0.f, c = 0.f;
+        f32x2 M0 = dup2(0.f), SL = M0, SA = M0, SLL = M0, SLA = M0, SAA = M0, MXX = M0, MXY = M0, MYY = M0;
         if (r_lat >= 0.f) {
             const int cx0 = max(x0, (int)ceilf((mu2_lat - r_lat) / lat_delta + col_off));
             const int cx1 = min(x1, (int)floorf((mu2_lat + r_lat) / lat_delta + col_off) + 1);
             const int cy0 = max(y0, (int)ceilf((mu2_ax - r_ax - near_mm) / ax_delta));
             const int cy1 = min(y1, (int)floorf((mu2_ax + r_ax - near_mm) / ax_delta) + 1);
             const int bw = cx1 - cx0, npx = bw > 0 && cy1 > cy0 ? bw * (cy1 - cy0) : 0;
-            o = opac[g];
-            c = inten[g];
-            // pixel pi = lane + 32 i of the box, row-major: (row, column) stepped without divisions
-            int ry = bw > 0 ? lane / bw : 0, rx = lane - ry * bw;
-            const int step_y = bw > 0 ? 32 / bw : 0, step_x = 32 - step_y * bw;
-            for (int pi = lane; pi < npx; pi += 32) {
-                const int x = cx0 + rx, y = cy0 + ry;
-                rx += step_x;
-                ry += step_y;
-                if (rx >= bw) {
-                    rx -= bw;
-                    ++ry;
+            const float o = opac[g];
+            // Pixels l + 32 i and l + 16 + 32 i of the box, row-major: (row, column) of each stepped without
+            // divisions, in whole floats. The quotients of at most 32.5 by at most 32 are 1/64
+            // away from a whole number or more.
+            const float rbw = bw > 0 ? (float)bw : 1.f;
+            const int ra = (int)__fdividef((float)l + 0.5f, rbw), rb = (int)__fdividef((float)l + 16.5f, rbw);
+            const int step_y = (int)__fdividef(32.5f, rbw), step_x = 32 - step_y * bw;
+            float xa = (float)(cx0 + l - ra * bw), xb = (float)(cx0 + l + 16 - rb * bw);
+            float ya = (float)(cy0 + ra), yb = (float)(cy0 + rb);
+            const float fx = (float)step_x, fy = (float)step_y, x_end = (float)cx1;
+            int at_a = (cy0 + ra) * W + cx0 + l - ra * bw, at_b = (cy0 + rb) * W + cx0 + l + 16 - rb * bw;
+            const int step = step_y * W + step_x, wrap = W - bw;
+            const f32x2 ML = dup2(mu2_lat), MA = dup2(mu2_ax), I00 = dup2(inv00), I01 = dup2(inv01), I11 = dup2(inv11);
+            const f32x2 CO = dup2(col_off), LD = dup2(lat_delta), AD = dup2(ax_delta), NR = dup2(near_mm);
+            // Ordinary: a pixel that does not contribute adds exact zeros, and an infinite quad or weight
+            // fails the weight test, without tests of their own.
+            const bool ordinary = weight_min > 0.f && fabsf(o * bno_const) <= FLT_MAX && fabsf(bno_const) <= FLT_MAX &&
+                                  (fabsf(inv00) + fabsf(inv01) + fabsf(inv11)) * (r_lat + r_ax) <= 1e30f;
+            auto sweep = [&](auto ordinary_t) {
+                constexpr bool ORD = decltype(ordinary_t)::value;
+                for (int pi = l; pi < npx; pi += 32) {
+                    const bool second = pi + 16 < npx;
+                    const f32x2 GI = pk2(grad_image[at_a], second ? grad_image[at_b] : 0.f);
+                    const f32x2 XC = sub2(pk2(xa, xb), CO), YF = pk2(ya, yb);
+                    const f32x2 DL = fma2(XC, LD, neg2(ML)), D = sub2(fma2(YF, AD, NR), MA);
+                    xa += fx;
+                    ya += fy;
+                    at_a += step;
+                    if (xa >= x_end) {
+                        xa -= rbw;
+                        ya += 1.f;
+                        at_a += wrap;
+                    }
+                    xb += fx;
+                    yb += fy;
+                    at_b += step;
+                    if (xb >= x_end) {
+                        xb -= rbw;
+                        yb += 1.f;
+                        at_b += wrap;
+                    }
+                    // the contractions of the compiled scalar expressions: every sum is the one a whole warp with
+                    // one pixel per lane forms (the finite differences of the finalize magnify rounding)
+                    f32x2 QL = fma2(I01, D, mul2(I00, DL)), QA = fma2(I11, D, mul2(I01, DL));
+                    const f32x2 Q = fma2(DL, QL, mul2(D, QA));
+                    const f32x2 BNO = mul2(dup2(bno_const), ex2_2(mul2(Q, CE)));
+                    float e0, e1, d0, d1, q0, q1, w0, w1, u0, u1;
+                    up2(DL, e0, e1);
+                    up2(D, d0, d1);
+                    up2(Q, q0, q1);
+                    up2(mul2(dup2(o), BNO), w0, w1);
+                    up2(mul2(GI, BNO), u0, u1);
+                    bool in0 = fabsf(e0) <= r_lat && fabsf(d0) <= r_ax && q0 >= 0.f && !(w0 < weight_min);
+                    bool in1 = second && fabsf(e1) <= r_lat && fabsf(d1) <= r_ax && q1 >= 0.f && !(w1 < weight_min);
+                    if (!ORD) {
+                        in0 = in0 && q0 <= FLT_MAX && fabsf(w0) <= FLT_MAX;
+                        in1 = in1 && q1 <= FLT_MAX && fabsf(w1) <= FLT_MAX;
+                        float a0, a1, b0, b1;
+                        up2(QL, a0, a1);
+                        up2(QA, b0, b1);
+                        QL = pk2(in0 ? a0 : 0.f, in1 ? a1 : 0.f);
+                        QA = pk2(in0 ? b0 : 0.f, in1 ? b1 : 0.f);
+                    }
+                    const f32x2 UB = pk2(in0 ? u0 : 0.f, in1 ? u1 : 0.f);
+                    const f32x2 UL = mul2(UB, QL), UA = mul2(UB, QA), UX = mul2(UB, DL), UY = mul2(UB, D);
+                    M0 = add2(M0, UB);
+                    SL = add2(SL, UL);
+                    SA = add2(SA, UA);
+                    SLL = fma2(UL, QL, SLL);
+                    SLA = fma2(UL, QA, SLA);
+                    SAA = fma2(UA, QA, SAA);
+                    MXX = fma2(UX, DL, MXX);
+                    MXY = fma2(UX, D, MXY);
+                    MYY = fma2(UY, D, MYY);
                 }
-                const float xi_ax = static_cast<float>(y) * ax_delta + near_mm;
-                const float xi_lat = (static_cast<float>(x) - col_off) * lat_delta;
-                if (fabsf(xi_lat - mu2_lat) > r_lat || fabsf(xi_ax - mu2_ax) > r_ax) continue;
-                const float dlat = xi_lat - mu2_lat;
-                const float dax = xi_ax - mu2_ax;
-                const float qlat = inv00 * dlat + inv01 * dax;
-                const float qax = inv01 * dlat + inv11 * dax;
-                const float quad = dlat * qlat + dax * qax;
-                if (!(quad >= 0.f) || !isfinite(quad)) continue;
-                const float phi = expf(-0.5f * quad);
-                const float bno = bno_const * phi;
-                const float weight = o * bno;
-                if (!isfinite(weight) || weight < weight_min) continue;
-                const float ub = grad_image[y * W + x] * bno;
-                const float ul = ub * qlat, ua = ub * qax;
-                const float ux = ub * dlat, uy = ub * dax;
-                m0 += ub;
-                sl += ul;
-                sa += ua;
-                sll += ul * qlat;
-                sla += ul * qax;
-                saa += ua * qax;
-                mxx += ux * dlat;
-                mxy += ux * dax;
-                myy += uy * dax;
-            }
+            };
+            if (ordinary)
+                sweep(std::true_type{});
+            else
+                sweep(std::false_type{});
         }
-        // Transposed warp reduction of the nine sums (padded to 16): each exchange halves the
-        // values a lane carries, so after four exchanges lanes 2j and 2j + 1 hold partial sums
-        // of value j over 16 lanes, the fifth completes them, and every lane then reads the
-        // nine totals from lanes 0, 2, ..., 16 (25 shuffles instead of 45; fixed order).
-        {
-            const unsigned FULL = 0xffffffffu;
-            const float v[16] = {m0, sl, sa, sll, sla, saa, mxx, mxy, myy, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            float a8[8], b4[4], c2[2];
-            const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4, h2 = lane & 2;
+        __syncwarp();
+        // Reduction of the nine sums over the half-warp: eight of them transposed (each exchange halves
+        // the values a lane carries, so lanes 2j and 2j + 1 end with sum j), the ninth plainly.
+        const unsigned FULL = 0xffffffffu;
+        const float v[8] = {sum2(SL), sum2(SA), sum2(SLL), sum2(SLA), sum2(SAA), sum2(MXX), sum2(MXY), sum2(MYY)};
+        float m0 = sum2(M0), b4[4], c2[2];
+        const bool h8 = lane & 8, h4 = lane & 4, h2 = lane & 2;
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-                a8[i] = (h16 ? v[8 + i] : v[i]) + __shfl_xor_sync(FULL, h16 ? v[i] : v[8 + i], 16);
+        for (int i = 0; i < 4; ++i)
+            b4[i] = (h8 ? v[4 + i] : v[i]) + __shfl_xor_sync(FULL, h8 ? v[i] : v[4 + i], 8);
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
-                b4[i] = (h8 ? a8[4 + i] : a8[i]) + __shfl_xor_sync(FULL, h8 ? a8[i] : a8[4 + i], 8);
+        for (int i = 0; i < 2; ++i)
+            c2[i] = (h4 ? b4[2 + i] : b4[i]) + __shfl_xor_sync(FULL, h4 ? b4[i] : b4[2 + i], 4);
+        float d = (h2 ? c2[1] : c2[0]) + __shfl_xor_sync(FULL, h2 ? c2[0] : c2[1], 2);
+        d += __shfl_xor_sync(FULL, d, 1);
 #pragma unroll
-            for (int i = 0; i < 2; ++i)
-                c2[i] = (h4 ? b4[2 + i] : b4[i]) + __shfl_xor_sync(FULL, h4 ? b4[i] : b4[2 + i], 4);
-            float d = (h2 ? c2[1] : c2[0]) + __shfl_xor_sync(FULL, h2 ? c2[0] : c2[1], 2);
-            d += __shfl_xor_sync(FULL, d, 1);
-            // value j = bits 4..1 of the lane (bit 4 selected the upper eight, bit 3 the upper four, ...)
-            m0 = __shfl_sync(FULL, d, 0);
-            sl = __shfl_sync(FULL, d, 2);
-            sa = __shfl_sync(FULL, d, 4);
-            sll = __shfl_sync(FULL, d, 6);
-            sla = __shfl_sync(FULL, d, 8);
-            saa = __shfl_sync(FULL, d, 10);
-            mxx = __shfl_sync(FULL, d, 12);
-            mxy = __shfl_sync(FULL, d, 14);
-            myy = __shfl_sync(FULL, d, 16);
-        }
-        // The terms of reference us_focus.cu:398-477 (per pixel: up * weight, up c bno and
-        // cm = up c weight times the footprint derivatives) from the six moments.
-        float acc[P_COUNT];
-        {
-            const float co = c * o;  // cm = co * up * bno
-            const float ql = sl, qa = sa, qll = sll, qla = sla, qaa = saa;
-            const float ele2 = mu_ele * mu_ele * inv_de * inv_de;
-            acc[P_INTENSITY] = o * m0;
-            acc[P_OPACITY] = c * m0;
-            acc[P_MU_E0] = co * ql;
-            acc[P_MU_E1] = co * qa;
-            acc[P_FP_MU2_LAT] = co * ql;
-            acc[P_FP_MU2_AX] = co * qa;
-            acc[P_FP_INV00] = co * (-0.5f * mxx);
-            acc[P_FP_INV01] = co * (-mxy);
-            acc[P_FP_INV11] = co * (-0.5f * myy);
-            acc[P_FP_DET2] = co * m0 * (-det_gamma * inv_det_norm);
-            acc[P_SE00] = co * (0.5f * qll - det_gamma * s2_11 * inv_det_norm * m0);
-            acc[P_SE01] = 0.5f * co * (qla + 2.f * det_gamma * s2_01 * inv_det_norm * m0);
-            acc[P_SE11] = co * (0.5f * qaa - det_gamma * s2_00 * inv_det_norm * m0);
-            acc[P_MU_PROBE2] = co * m0 * (-mu_ele * inv_de);
-            acc[P_SC22] = co * m0 * (0.5f * ele2);
-            acc[P_MU_PROBE1] = co * m0 * (ele2 * dse_dax);
-            acc[P_FP_MU_ELE] = co * m0 * (-mu_ele * inv_de);
-            acc[P_FP_SC22] = co * m0 * (0.5f * ele2);
-            acc[P_FP_SIGMA_ELE] = co * m0 * (ele2 * sigma_ele);
-        }
-        float4* out = reinterpret_cast<float4*>(partial) + (int64_t)PARTIAL_F4 * sorted_inst[k];
-        if (lane == 0) {
-            out[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
-            out[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
-            out[2] = make_float4(acc[8], acc[9], acc[10], acc[11]);
-            out[3] = make_float4(acc[12], acc[13], acc[14], acc[15]);
-            out[4] = make_float4(acc[16], acc[17], acc[18], 0.f);
-        }
+        for (int x = 8; x >= 1; x >>= 1) m0 += __shfl_xor_sync(FULL, m0, x);
+        // value j = bits 3..1 of the lane within its half (bit 3 selected the upper four, bit 2 the upper two)
+        if (live && ((l & 1) == 0 || l == 1))
+            partial[(int64_t)(4 * PARTIAL_F4) * sorted_inst[k] + (l == 1 ? (int)M_ONE : l >> 1)] = l == 1 ? m0 : d;
     }
 }
 
@@ -864,52 +862,50 @@ __device__ __forceinline__ float3 normalize3_bwd(const float3 raw, const float3 
     return make_float3((g.x - n.x * dn) * il, (g.y - n.y * dn) * il, (g.z - n.z * dn) * il);
 }
 
-// Per-Gaussian sums of its instances' partial records, in instance order, written over its first
-// instance's record: PARTIAL_F4 threads per Gaussian, thread f summing float4 column f, so that
-// the threads of a Gaussian read each 80-byte record together and many Gaussians' loads are in
-// flight (the sums are the ones a thread summing all columns would form).
-constexpr int REDUCE_THREADS = 32 * PARTIAL_F4;  // 32 Gaussians per block
-__global__ void __launch_bounds__(REDUCE_THREADS)
-reduce_partials_kernel(int64_t G, const int* __restrict__ inst_offset, const long long* __restrict__ header,
-                       float4* __restrict__ partial) {
-    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t g = t / PARTIAL_F4;
-    const int f = (int)(t % PARTIAL_F4);
-    if (g >= G || header[H_FLAGS] != 0) return;
-    const int i0 = inst_offset[g], i1 = inst_offset[g + 1];
-    if (i1 <= i0) return;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    int i = i0;
-    for (; i + 4 <= i1; i += 4) {  // four instances' loads in flight
-        float4 v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) v[u] = partial[(int64_t)PARTIAL_F4 * (i + u) + f];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            acc.x += v[u].x;
-            acc.y += v[u].y;
-            acc.z += v[u].z;
-            acc.w += v[u].w;
-        }
-    }
-    for (; i < i1; ++i) {
-        const float4 v = partial[(int64_t)PARTIAL_F4 * i + f];
-        acc.x += v.x;
-        acc.y += v.y;
-        acc.z += v.z;
-        acc.w += v.w;
-    }
-    partial[(int64_t)PARTIAL_F4 * i0 + f] = acc;
+// The terms of one instance (reference us_focus.cu:398-477: per pixel up * weight, up c bno and cm = up c weight
+// times the footprint derivatives) from its moments; cm = co * up * bno.
+enum { P_MU_PROBE1 = 0, P_MU_PROBE2, P_SC22, P_MU_E0, P_MU_E1, P_SE00, P_SE01, P_SE11, P_OPACITY, P_INTENSITY,
+       P_FP_MU2_LAT, P_FP_MU2_AX, P_FP_INV00, P_FP_INV01, P_FP_INV11, P_FP_DET2, P_FP_MU_ELE, P_FP_SC22,
+       P_FP_SIGMA_ELE, P_COUNT };
+
+__device__ __forceinline__ void instance_terms(const float4 a, const float4 b, const float m0, const float4 f2,
+                                               const float4 f3, const float o, const float c, const float det_gamma,
+                                               float acc[P_COUNT]) {
+    const float s2_00 = f2.x, s2_01 = f2.y, s2_11 = f2.z, inv_det_norm = f2.w;
+    const float mu_ele = f3.x, inv_de = f3.y, dse_dax = f3.z, sigma_ele = f3.w;
+    const float ql = a.x, qa = a.y, qll = a.z, qla = a.w, qaa = b.x, mxx = b.y, mxy = b.z, myy = b.w;
+    const float co = c * o;  // cm = co * up * bno
+    const float ele2 = mu_ele * mu_ele * inv_de * inv_de;
+    acc[P_INTENSITY] = o * m0;
+    acc[P_OPACITY] = c * m0;
+    acc[P_MU_E0] = co * ql;
+    acc[P_MU_E1] = co * qa;
+    acc[P_FP_MU2_LAT] = co * ql;
+    acc[P_FP_MU2_AX] = co * qa;
+    acc[P_FP_INV00] = co * (-0.5f * mxx);
+    acc[P_FP_INV01] = co * (-mxy);
+    acc[P_FP_INV11] = co * (-0.5f * myy);
+    acc[P_FP_DET2] = co * m0 * (-det_gamma * inv_det_norm);
+    acc[P_SE00] = co * (0.5f * qll - det_gamma * s2_11 * inv_det_norm * m0);
+    acc[P_SE01] = 0.5f * co * (qla + 2.f * det_gamma * s2_01 * inv_det_norm * m0);
+    acc[P_SE11] = co * (0.5f * qaa - det_gamma * s2_00 * inv_det_norm * m0);
+    acc[P_MU_PROBE2] = co * m0 * (-mu_ele * inv_de);
+    acc[P_SC22] = co * m0 * (0.5f * ele2);
+    acc[P_MU_PROBE1] = co * m0 * (ele2 * dse_dax);
+    acc[P_FP_MU_ELE] = co * m0 * (-mu_ele * inv_de);
+    acc[P_FP_SC22] = co * m0 * (0.5f * ele2);
+    acc[P_FP_SIGMA_ELE] = co * m0 * (ele2 * sigma_ele);
 }
 
-// Per Gaussian: its instance partials summed by reduce_partials_kernel, then the chain rule
+// Per Gaussian: the terms of its instances summed in instance order, then the chain rule
 // through Se and Lc, finite-difference shape gradients, sanitising, and the pose contribution
 // (reference us_focus.cu:479-803).
 __global__ void __launch_bounds__(128)
 finalize_kernel(int64_t G, float k_sigma, const int* __restrict__ inst_offset, const int4* __restrict__ rects,
                 const float* __restrict__ means, const float* __restrict__ scales, const float* __restrict__ quats,
+                const float* __restrict__ opac, const float* __restrict__ inten, const float4* __restrict__ bfp,
                 const float* __restrict__ pose, const float* __restrict__ grid, const float* __restrict__ params,
-                const long long* __restrict__ header, const float* __restrict__ partial, int pose_grad,
+                const long long* __restrict__ header, const float4* __restrict__ partial, int pose_grad,
                 int shape_analytic_mode, float* __restrict__ d_means, float* __restrict__ d_scales, float* __restrict__ d_quats,
                 float* __restrict__ d_opac, float* __restrict__ d_inten, float* __restrict__ pose_partial) {
     const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -943,14 +939,17 @@ finalize_kernel(int64_t G, float k_sigma, const int* __restrict__ inst_offset, c
     float acc[P_COUNT];
 #pragma unroll
     for (int i = 0; i < P_COUNT; ++i) acc[i] = 0.f;
-    if (inst_offset[g + 1] > inst_offset[g]) {  // the sums reduce_partials_kernel left in the first record
-        const float4* r = reinterpret_cast<const float4*>(partial) + (int64_t)PARTIAL_F4 * inst_offset[g];
-        const float4 a = r[0], b = r[1], c = r[2], d = r[3], e = r[4];
-        acc[0] = a.x; acc[1] = a.y; acc[2] = a.z; acc[3] = a.w;
-        acc[4] = b.x; acc[5] = b.y; acc[6] = b.z; acc[7] = b.w;
-        acc[8] = c.x; acc[9] = c.y; acc[10] = c.z; acc[11] = c.w;
-        acc[12] = d.x; acc[13] = d.y; acc[14] = d.z; acc[15] = d.w;
-        acc[16] = e.x; acc[17] = e.y; acc[18] = e.z;
+    {
+        const float4 f2 = bfp[4 * g + 2], f3 = bfp[4 * g + 3];
+        const float det_gamma = params[UF_DET_GAMMA], c_opac = opac[g], c_inten = inten[g];
+        const int i1 = inst_offset[g + 1];
+        for (int i = inst_offset[g]; i < i1; ++i) {
+            const float4* r = partial + (int64_t)PARTIAL_F4 * i;
+            float v[P_COUNT];
+            instance_terms(r[0], r[1], reinterpret_cast<const float*>(r)[M_ONE], f2, f3, c_opac, c_inten, det_gamma, v);
+#pragma unroll
+            for (int k = 0; k < P_COUNT; ++k) acc[k] = __fadd_rn(acc[k], v[k]);
+        }
     }
 
     const float depth = fmaxf(F.mu_ax - near_mm, 0.f);
@@ -1260,19 +1259,15 @@ extern "C" int us3d_gp_backward(void* workspace, int64_t n_gauss, const float* m
     int launches = 0;
     if (T > 0) {
         backward_inst_kernel<<<148 * 8, BWD_WARPS * 32, 0, stream>>>(
-            (int)T, W, tile_size, tx, opacities, intensities, w.bfp, grid_pack, focus_params, w.tile_start,
+            (int)T, W, tile_size, tx, opacities, w.bfp, grid_pack, focus_params, w.tile_start,
             w.sorted_gid, w.sorted_inst, w.header, grad_image, partial, H);
         US3D_CHECK_LAUNCH("gp backward instances");
         launches = 1;
     }
     if (n_gauss > 0) {
-        reduce_partials_kernel<<<(unsigned)((n_gauss * PARTIAL_F4 + REDUCE_THREADS - 1) / REDUCE_THREADS),
-                                 REDUCE_THREADS, 0, stream>>>(n_gauss, w.inst_offset, w.header,
-                                                              reinterpret_cast<float4*>(partial));
-        ++launches;
         finalize_kernel<<<(unsigned)((n_gauss + 127) / 128), 128, 0, stream>>>(
-            n_gauss, k_sigma, w.inst_offset, w.rects, means, scales, quats, pose, grid_pack, focus_params, w.header,
-            partial, pose_grad, shape_analytic_mode, d_means, d_scales, d_quats, d_opacities, d_intensities,
+            n_gauss, k_sigma, w.inst_offset, w.rects, means, scales, quats, opacities, intensities, w.bfp, pose, grid_pack,
+            focus_params, w.header, reinterpret_cast<const float4*>(partial), pose_grad, shape_analytic_mode, d_means, d_scales, d_quats, d_opacities, d_intensities,
             pose_partial);
         US3D_CHECK_LAUNCH("gp finalize");
         ++launches;
