@@ -495,11 +495,25 @@ US3D_API int us3d_sa_bounded_forward_checked(void* workspace, size_t workspace_b
                                              float radius_sigma, int64_t instance_capacity, float* out_image,
                                              float* out_alpha, int64_t* total_instances, int32_t* flags,
                                              void* stream);
+/* The grey image (n_pixels) of a rendered image (n_pixels x 3): bg_color added, clamped to [0, 1] if `clamp`,
+ * 0.299 r + 0.587 g + 0.114 b (the output step of baselines/slice_adapted_3dgs/render.py:60-129), and its
+ * gradient d_image (n_pixels x 3). */
+US3D_API int us3d_sa_finish(int64_t n_pixels, const float* image, float bg_color, int32_t clamp, float* out_gray,
+                            void* stream);
+US3D_API int us3d_sa_finish_backward(int64_t n_pixels, const float* image, float bg_color, int32_t clamp,
+                                     const float* d_gray, float* d_image, void* stream);
 US3D_API int us3d_sa_read_status(const void* workspace, int64_t* total_instances, int32_t* overflow,
                                  void* stream);
 /* Replaces bounded_backward (render.cu:923-1013): gradients w.r.t. means2d (N,2),
  * inv2d (N,2,2), weights (N) and colors (N,3). Deterministic. */
 US3D_API int us3d_sa_bounded_backward(void* workspace, int64_t n, int32_t height, int32_t width, float half_width,
+                                      float half_height, const float* means2d, const float* inv2d,
+                                      const float* weights, const float* colors, const float* grad_image,
+                                      const float* grad_alpha, float radius_sigma, int64_t instance_capacity,
+                                      void* scratch, size_t scratch_bytes, float* d_means2d, float* d_inv2d,
+                                      float* d_weights, float* d_colors, void* stream);
+/* us3d_sa_bounded_backward with grad_alpha optional: NULL stands for zeros. */
+US3D_API int us3d_sa_bounded_backward_ex(void* workspace, int64_t n, int32_t height, int32_t width, float half_width,
                                       float half_height, const float* means2d, const float* inv2d,
                                       const float* weights, const float* colors, const float* grad_image,
                                       const float* grad_alpha, float radius_sigma, int64_t instance_capacity,

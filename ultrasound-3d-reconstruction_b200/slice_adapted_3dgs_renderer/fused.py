@@ -16,7 +16,7 @@ import torch
 
 from us3d_b200 import slice_adapted as _sa
 
-from .api import additive_splat_bounded
+from .api import _check_bounded_inputs
 
 
 @dataclass
@@ -57,26 +57,35 @@ class RenderOutput:
     extras: Dict[str, torch.Tensor] = field(default_factory=dict)
 
 
-class _SliceProject(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, means, scales, quats, opacities, colors, view, settings):
-        c = lambda t: t.detach().to(dtype=torch.float32).contiguous()  # noqa: E731
-        m, s, q, o, col, v = c(means), c(scales), c(quats), c(opacities).reshape(-1), c(colors), c(view)
-        m2, inv, w, colk, idx, mask = _sa.project(m, s, q, o, col, v, settings)
-        ctx.settings = settings
-        ctx.opacity_shape = opacities.shape
-        ctx.save_for_backward(m, s, q, o, v, idx)
-        ctx.mark_non_differentiable(mask)
-        return m2, inv, w, colk, mask
+class _SliceRender(torch.autograd.Function):
+    """Image and alpha image (H*W, 1) of the Gaussians whose projection ``projected`` holds, as one node: the bounded
+    splat with the background added (H*W, 3), or the grey image (H*W,) with the clamp applied."""
 
     @staticmethod
-    def backward(ctx, d_m2, d_inv, d_w, d_col, _d_mask):
-        m, s, q, o, v, idx = ctx.saved_tensors
-        n = idx.shape[0]
-        z = lambda g, *sh: torch.zeros(sh, device=m.device) if g is None else g  # noqa: E731
-        dm, ds, dq, dop, dc = _sa.project_backward(idx, m, s, q, o, v, ctx.settings, z(d_m2, n, 2), z(d_inv, n, 2, 2),
-                                                   z(d_w, n, 1), z(d_col, n, 3))
-        return dm, ds, dq, dop.reshape(ctx.opacity_shape), dc, None, None
+    def forward(ctx, means, scales, quats, opacities, colors, inputs, projected, settings, frame):
+        H, W, half_w, half_h, sigma, bg, gray, clamp = frame
+        m2, inv, w, colk, idx = projected
+        _check_bounded_inputs(H, W, half_w, half_h, m2, inv, w, colk, sigma)
+        image, alpha, b = _sa.bounded_forward(H, W, half_w, half_h, m2, inv, w, colk, sigma)
+        ctx.set_materialize_grads(False)
+        ctx.b, ctx.settings, ctx.frame, ctx.opacity_shape = b, settings, frame, opacities.shape
+        if gray:
+            ctx.save_for_backward(*inputs, idx, m2, inv, w, colk, image)
+            return _sa.finish(image, bg, clamp), alpha
+        ctx.save_for_backward(*inputs, idx, m2, inv, w, colk)
+        return image.add_(bg), alpha
+
+    @staticmethod
+    def backward(ctx, d_out, d_alpha):
+        m, s, q, o, v, idx, m2, inv, w, colk, *image = ctx.saved_tensors
+        H, W, half_w, half_h, sigma, bg, gray, clamp = ctx.frame
+        if d_out is None:
+            d_out = torch.zeros((H * W, 3), device=m.device)
+        elif gray:
+            d_out = _sa.finish_backward(image[0], bg, clamp, d_out.contiguous())
+        g = _sa.bounded_backward(ctx.b, half_w, half_h, m2, inv, w, colk, d_out, d_alpha, sigma, absent_zero=True)
+        dm, ds, dq, dop, dc = _sa.project_backward(idx, m, s, q, o, v, ctx.settings, *g)
+        return dm, ds, dq, dop.reshape(ctx.opacity_shape), dc, None, None, None, None
 
 
 def _finalize(image, alpha, keep, settings):
@@ -95,17 +104,24 @@ def render_slice_adapted_3dgs(gaussians, camera, settings) -> RenderOutput:
                                 thickness_scale=float(settings.thickness_scale),
                                 min_covariance=float(settings.min_covariance),
                                 normalize_by_footprint=bool(settings.normalize_by_footprint))
-    means2d, inv, weights, colors, keep = _SliceProject.apply(gaussians.means, gaussians.scales_3d, gaussians.quats,
-                                                              gaussians.opacities, gaussians.colors, view, ps)
+    c = lambda t: t.detach().to(dtype=torch.float32).contiguous()  # noqa: E731
+    inputs = (c(gaussians.means), c(gaussians.scales_3d), c(gaussians.quats), c(gaussians.opacities).reshape(-1),
+              c(view))
+    *projected, keep = _sa.project(*inputs[:4], c(gaussians.colors), inputs[4], ps)
     H, W = int(camera.image_height), int(camera.image_width)
-    if means2d.shape[0] == 0:
+    if projected[0].shape[0] == 0:
         image = torch.full((3, H, W), float(settings.bg_color), device=device, dtype=gaussians.means.dtype)
         return _finalize(image, None, keep, settings)
-    image_flat, alpha_flat = additive_splat_bounded(H, W, float(camera.half_width_mm), float(camera.half_height_mm),
-                                                    means2d, inv, weights, colors, float(settings.cull_std))
-    image_flat = image_flat + float(settings.bg_color)
-    if settings.clamp_output:
-        image_flat = image_flat.clamp(0.0, 1.0)
-    image = image_flat.transpose(0, 1).reshape(3, H, W)
-    alpha = alpha_flat.transpose(0, 1).reshape(1, H, W)
-    return _finalize(image, alpha, keep, settings)
+    gray, clamp = bool(settings.output_grayscale), bool(settings.clamp_output)
+    frame = (H, W, float(camera.half_width_mm), float(camera.half_height_mm), float(settings.cull_std),
+             float(settings.bg_color), gray, clamp)
+    image, alpha = _SliceRender.apply(gaussians.means, gaussians.scales_3d, gaussians.quats, gaussians.opacities,
+                                      gaussians.colors, inputs, projected, ps, frame)
+    if gray:
+        image = image.view(1, H, W)
+    else:
+        if clamp:
+            image = image.clamp(0.0, 1.0)
+        image = image.transpose(0, 1).reshape(3, H, W)
+    return RenderOutput(image=image, depth=None,
+                        extras={"visibility_filter": keep, "alpha_image": alpha.view(1, H, W)})

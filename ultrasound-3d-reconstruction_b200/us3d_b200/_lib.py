@@ -206,8 +206,17 @@ _SIGNATURES = {
         [c_void_p, c_size_t, c_int64, c_int32, c_int32, c_float, c_float, c_void_p, c_void_p, c_void_p, c_void_p,
          c_float, c_int64, c_void_p, c_void_p, POINTER(c_int64), POINTER(c_int32), c_void_p],
     ),
+    "us3d_sa_finish": (c_int32, [c_int64, c_void_p, c_float, c_int32, c_void_p, c_void_p]),
+    "us3d_sa_finish_backward": (
+        c_int32, [c_int64, c_void_p, c_float, c_int32, c_void_p, c_void_p, c_void_p]
+    ),
     "us3d_sa_read_status": (c_int32, [c_void_p, POINTER(c_int64), POINTER(c_int32), c_void_p]),
     "us3d_sa_bounded_backward": (
+        c_int32,
+        [c_void_p, c_int64, c_int32, c_int32, c_float, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+         c_void_p, c_float, c_int64, c_void_p, c_size_t, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],
+    ),
+    "us3d_sa_bounded_backward_ex": (
         c_int32,
         [c_void_p, c_int64, c_int32, c_int32, c_float, c_float, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
          c_void_p, c_float, c_int64, c_void_p, c_size_t, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p],

@@ -9,7 +9,7 @@ from typing import Optional
 import torch
 
 from . import _lib
-from ._alloc import current_stream as _stream
+from ._alloc import current_stream as _stream, float_outputs
 
 _capacity_hint: dict = {}
 
@@ -53,23 +53,38 @@ def bounded_forward(H, W, half_width, half_height, means2d, inv2d, weights, colo
 
 
 def bounded_backward(b: SABinning, half_width, half_height, means2d, inv2d, weights, colors, grad_image, grad_alpha,
-                     radius_sigma=3.0):
+                     radius_sigma=3.0, absent_zero: bool = False):
+    """With ``absent_zero``, ``grad_alpha`` may be None: zeros."""
     dev = means2d.device
     N = b.n
     scratch = torch.empty(max(int(_lib.call("us3d_sa_backward_scratch_bytes", b.capacity)), 16), dtype=torch.uint8,
                           device=dev)
-    dm = torch.empty((N, 2), dtype=torch.float32, device=dev)
-    di = torch.empty((N, 2, 2), dtype=torch.float32, device=dev)
-    dw = torch.empty((N, 1), dtype=torch.float32, device=dev)
-    dc = torch.empty((N, 3), dtype=torch.float32, device=dev)
+    dm, di, dw, dc = float_outputs(dev, [(N, 2), (N, 2, 2), (N, 1), (N, 3)])
     gi = grad_image.contiguous().float()
-    ga = grad_alpha.contiguous().float()
-    st = _lib.call("us3d_sa_bounded_backward", b.workspace.data_ptr(), N, b.H, b.W, float(half_width),
+    ga = None if absent_zero and grad_alpha is None else grad_alpha.contiguous().float()
+    st = _lib.call("us3d_sa_bounded_backward_ex" if ga is None else "us3d_sa_bounded_backward", b.workspace.data_ptr(), N, b.H, b.W, float(half_width),
                    float(half_height), means2d.data_ptr(), inv2d.data_ptr(), weights.data_ptr(), colors.data_ptr(),
-                   gi.data_ptr(), ga.data_ptr(), float(radius_sigma), b.capacity, scratch.data_ptr(), scratch.numel(),
+                   gi.data_ptr(), None if ga is None else ga.data_ptr(), float(radius_sigma), b.capacity, scratch.data_ptr(), scratch.numel(),
                    dm.data_ptr(), di.data_ptr(), dw.data_ptr(), dc.data_ptr(), _stream())
     _lib.check(st, "us3d_sa_bounded_backward")
     return dm, di, dw, dc
+
+
+def finish(image, bg_color, clamp):
+    """The grey image (P,) of a rendered image (P,3): background, clamp, 0.299 r + 0.587 g + 0.114 b."""
+    out = torch.empty(image.shape[0], dtype=torch.float32, device=image.device)
+    _lib.check(_lib.call("us3d_sa_finish", image.shape[0], image.data_ptr(), float(bg_color), 1 if clamp else 0,
+                         out.data_ptr(), _stream()), "us3d_sa_finish")
+    return out
+
+
+def finish_backward(image, bg_color, clamp, d_gray):
+    """d_image (P,3) for the gradient d_gray (P,) of ``finish``."""
+    d_image = torch.empty_like(image)
+    _lib.check(_lib.call("us3d_sa_finish_backward", image.shape[0], image.data_ptr(), float(bg_color),
+                         1 if clamp else 0, d_gray.data_ptr(), d_image.data_ptr(), _stream()),
+               "us3d_sa_finish_backward")
+    return d_image
 
 
 def export_bins(b: SABinning):
@@ -132,7 +147,7 @@ def project(means, scales, quats, opacities, colors, viewmatrix, s: ProjectionSe
     w = torch.empty((G, 1), dtype=torch.float32, device=dev)
     col = torch.empty((G, 3), dtype=torch.float32, device=dev)
     idx = torch.empty((G,), dtype=torch.int32, device=dev)
-    mask = torch.zeros((G,), dtype=torch.uint8, device=dev)
+    mask = torch.empty((G,), dtype=torch.uint8, device=dev)  # written in full
     kept = ctypes.c_int64(0)
     _lib.check(_lib.call("us3d_sa_project", ws.data_ptr(), ws.numel(), G, means.data_ptr(), scales.data_ptr(),
                          quats.data_ptr(), opacities.data_ptr(), colors.data_ptr(), viewmatrix.data_ptr(),
@@ -141,15 +156,14 @@ def project(means, scales, quats, opacities, colors, viewmatrix, s: ProjectionSe
                          w.data_ptr(), col.data_ptr(), idx.data_ptr(), mask.data_ptr(), ctypes.byref(kept),
                          _stream()), "us3d_sa_project")
     n = int(kept.value)
-    return m2[:n], inv[:n], w[:n], col[:n], idx[:n], mask.bool()
+    return m2[:n], inv[:n], w[:n], col[:n], idx[:n], mask.view(torch.bool)  # zeros and ones
 
 
 def project_backward(keep_idx, means, scales, quats, opacities, viewmatrix, s: ProjectionSettings, d_means2d,
                      d_inv2d, d_weights, d_colors_kept):
     G, N = int(means.shape[0]), int(keep_idx.shape[0])
     dev = means.device
-    z = lambda *sh: torch.empty(sh, dtype=torch.float32, device=dev)  # noqa: E731
-    dm, ds, dq, dop, dc = z(G, 3), z(G, 3), z(G, 4), z(G), z(G, 3)
+    dm, ds, dq, dop, dc = float_outputs(dev, [(G, 3), (G, 3), (G, 4), (G,), (G, 3)])
     c = lambda t: t.to(dtype=torch.float32).contiguous()  # noqa: E731
     g = [c(d_means2d), c(d_inv2d), c(d_weights), c(d_colors_kept)]
     _lib.check(_lib.call("us3d_sa_project_backward", G, N, keep_idx.data_ptr(), means.data_ptr(), scales.data_ptr(),
