@@ -77,3 +77,27 @@ def test_more_frames_than_a_mask_word(n_frames, cuda_device):
                 assert torch.equal(a[off:off + m], b)
             off += m
         assert all(torch.isfinite(g).all() for g in grads)
+
+
+@pytest.mark.parametrize("use", [12, 20, 27])
+def test_gradients_do_not_depend_on_the_blocks_per_tile(use, cuda_device):
+    """Forty frames (2,560 tiles, one block each in the backward) with an adjoint on one of them against that
+    frame alone (64 tiles, four blocks each): the same bits."""
+    from us3d_b200 import ultragauss as UG
+
+    params = _scene(cuda_device, 6000, 13)
+    frames = _frames(40, 128, 128, 0.5, 13)
+    grads = []
+    for sel in (frames, frames[use:use + 1]):
+        pix = torch.cat([p for _, p in sel]).to(cuda_device)
+        b = UG.bin_gaussians(*params, UG.build_frame_table([s for s, _ in sel], cuda_device), 7.815, 1e-4, True,
+                             slice_cull_pixels=pix)
+        assert (b.frames.n_tiles < 4 * 4 * 148) == (len(sel) == 1)
+        alpha = UG.forward(b, pix, 1e-6, 0.0, want_counts=False)[1]
+        g = torch.zeros((2, pix.shape[0]), device=cuda_device)
+        at = use * 128 * 128 if len(sel) > 1 else 0
+        g[:, at:at + 128 * 128] = torch.linspace(-1.0, 1.0, 2 * 128 * 128, device=cuda_device).reshape(2, -1)
+        zero = torch.zeros_like(g[0])
+        grads.append(UG.backward(b, pix, g[0].contiguous(), g[1].contiguous(), zero, alpha, 1e-6, 0.0))
+    for a, b in zip(*grads):
+        assert torch.count_nonzero(b) > 0 and torch.equal(a, b)

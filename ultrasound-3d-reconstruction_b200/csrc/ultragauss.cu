@@ -1276,7 +1276,7 @@ backward_packed_kernel(int64_t T, int64_t P, const us3d_slice_frame* __restrict_
                        const float* __restrict__ d_depth, const float* __restrict__ saved_alpha,
                        const float2* __restrict__ pixel_aux, float chi2, float beta, float bg_alpha,
                        float bg_intensity, const float* __restrict__ loss_image, const float* __restrict__ loss_target,
-                       const float4* __restrict__ loss_coef, float4* __restrict__ partial) {
+                       const float4* __restrict__ loss_coef, float4* __restrict__ partial, int parts) {
     constexpr int PAIRS = TILE_PIX / 2;       // 128 pixel pairs per tile
     constexpr int SUB_PAIRS = SUB_PIX / 2;    // 8 per sub-block
     // Per sub-block c, entries [16 c, 16 c + 16) hold its 8 pairs twice, so that the sweep
@@ -1286,11 +1286,16 @@ backward_packed_kernel(int64_t T, int64_t P, const us3d_slice_frame* __restrict_
     __shared__ float4 s_c[2 * PAIRS];  // (dtot0, dtot1, ddw0, ddw1)
     __shared__ short s_perm[BWD_CHUNK];
     __shared__ int s_class[NSUB + 1];
-    const int64_t t = blockIdx.x;
+    const int64_t t = blockIdx.x / (unsigned)parts;
     if (t >= T || header[H_FLAGS] != 0) return;
     const int s0 = tile_start[t];
     const int n = tile_start[t + 1] - s0;
     if (n <= 0 || tile_frame[t] < 0) return;
+    // this block's part of the list: whole rounds of the block
+    const int part = blockIdx.x % (unsigned)parts, rounds = (n + THREADS - 1) / THREADS;
+    const int p0 = (int)((int64_t)rounds * part / parts) * THREADS;
+    const int p1 = min(n, (int)((int64_t)rounds * (part + 1) / parts) * THREADS);
+    if (p0 >= p1) return;
     const Geo geo = load_geo(frames + tile_frame[t]);
     int tx, ty;
     find_tile_coords(geo, t, tx, ty);
@@ -1344,8 +1349,8 @@ backward_packed_kernel(int64_t T, int64_t P, const us3d_slice_frame* __restrict_
     // 33 a pair, and are left out
     const bool depth = !LOSS && __syncthreads_or(any_depth) != 0;
 
-    for (int c0 = 0; c0 < n; c0 += BWD_CHUNK) {
-        const int nc = min(BWD_CHUNK, n - c0);
+    for (int c0 = p0; c0 < p1; c0 += BWD_CHUNK) {
+        const int nc = min(BWD_CHUNK, p1 - c0);
         if (threadIdx.x <= NSUB) s_class[threadIdx.x] = 0;
         __syncthreads();
         if (culled) {
@@ -1906,6 +1911,14 @@ extern "C" int us3d_ug_frame_table(us3d_slice_frame* frame, const float* origin,
     return US3D_OK;
 }
 
+// Blocks that share a tile's list in the packed backward, whole rounds of 256 instances each (an instance's sums
+// are one thread's, so results do not depend on it). With few tiles the longest list is the kernel's time: one
+// clustered 256x256 frame (255 tiles, up to 1,272 instances) 50 -> 27 us with four blocks, a training
+// batch (1,152 tiles, up to 2,857) 122 -> 75 us; two blocks take 30 and 88 us, eight 29 and 79 us. Four
+// waves of tiles balance themselves, and the blocks without a part then only cost: 5,546 tiles
+// 174 us with one, 182 with two, 205 with four; 16,384 tiles 2.47, 2.57 and 2.90 ms.
+static int backward_parts(int64_t n_tiles) { return n_tiles < 4 * 4 * 148 ? 4 : 1; }
+
 static int ug_backward_impl(void* workspace, const us3d_slice_frame* frames, int32_t n_frames, int64_t n_tiles,
                             int64_t n_pixels, int64_t n_gauss, int64_t cap, const float* pixels,
                             const float* d_image, const float* d_alpha, const float* d_depth,
@@ -1939,14 +1952,21 @@ static int ug_backward_impl(void* workspace, const us3d_slice_frame* frames, int
                 bg_intensity, loss_image, loss_target, loss_coef, partial);
         };
         const bool packed = g_bwd_variant.load() == 1;
+        auto launch_packed = [&](auto kernel, int nthreads) {
+            const int parts = backward_parts(n_tiles);
+            kernel<<<(unsigned)(n_tiles * parts), nthreads, 0, stream>>>(
+                n_tiles, n_pixels, frames, w.tile_frame, w.tile_start, w.sorted_gid, w.sorted_inst, w.sorted_mask,
+                w.header, w.pack, pixels, d_image, d_alpha, d_depth, saved_alpha, w.pixel_aux, chi2, beta, bg_alpha,
+                bg_intensity, loss_image, loss_target, loss_coef, partial, parts);
+        };
         if (!window_implied(beta))
             fused ? launch(backward_kernel<true, 256, true>, 256) : launch(backward_kernel<false, 256, true>, 256);
         else if (packed && fused)
-            threads == 128 ? launch(backward_packed_kernel<true, 128>, 128)
-                           : launch(backward_packed_kernel<true, 256>, 256);
+            threads == 128 ? launch_packed(backward_packed_kernel<true, 128>, 128)
+                           : launch_packed(backward_packed_kernel<true, 256>, 256);
         else if (packed)
-            threads == 128 ? launch(backward_packed_kernel<false, 128>, 128)
-                           : launch(backward_packed_kernel<false, 256>, 256);
+            threads == 128 ? launch_packed(backward_packed_kernel<false, 128>, 128)
+                           : launch_packed(backward_packed_kernel<false, 256>, 256);
         else if (fused)
             threads == 128 ? launch(backward_kernel<true, 128, false>, 128)
                            : launch(backward_kernel<true, 256, false>, 256);
