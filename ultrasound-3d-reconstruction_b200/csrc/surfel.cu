@@ -467,20 +467,22 @@ constexpr int BLK_W = 8, BLK_H = 4;
 __device__ __forceinline__ int block_x(int t) { return ((t >> 5) & 1) * BLK_W + (t & (BLK_W - 1)); }
 __device__ __forceinline__ int block_y(int t) { return (t >> 6) * BLK_H + ((t & 31) >> 3); }
 
-// One CTA per tile, one pixel per thread. Per staged batch every warp lists, by ballot and in order, the
-// surfels whose reach box meets its 8x4 pixels and composites only those: the others fail the alpha
-// test on all of them (decisions and sums are those of the whole list, and a contributor's number is
-// its place in the tile's list). The intersections of two listed surfels are evaluated together,
-// since what bounds the kernel is the dependent chain of the tile with the longest list (a clustered
-// scene of 200k surfels at 256x256: SMs 690k cycles busy on average, 2.07M at most). That
-// scene: 1.053 -> 0.452 ms.
+// One CTA per tile, one pixel per thread, the warps independent of one another: of every 32 surfels of the tile's
+// list a warp keeps, by ballot and in order, those whose reach box meets its 8x4 pixels, copies their
+// records into its own staging buffer while it composites the ones before, and stops when its pixels are
+// done. The others fail the alpha test on all its pixels (decisions and sums are those of the whole list, and
+// a contributor's number is its place in the tile's list). The intersections of two kept surfels are
+// evaluated together. What bounds the kernel is the dependent chain of the longest list (a
+// clustered scene of 200k surfels at 256x256: 1.053 ms with one list for the tile, 0.452 ms with lists per
+// warp of batches staged by the whole CTA, whose warps then spent half their stall cycles waiting
+// for one another at its barriers (SMs 345k cycles busy on average, 895k at most); 0.294 ms so).
 __global__ void __launch_bounds__(BLOCK)
 forward_kernel(int W, int H, int gx, const int* __restrict__ tile_start, const int* __restrict__ sorted_gid,
                const long long* __restrict__ header, const float4* __restrict__ rec, const float* __restrict__ bg,
                float* __restrict__ out_color, float* __restrict__ out_others, float* __restrict__ accum,
                uint32_t* __restrict__ n_contrib) {
-    __shared__ float4 s_rec[2][REC_F4][BLOCK];  // double-buffered staging
-    __shared__ unsigned char s_list[BLOCK / 32][BLOCK];
+    __shared__ float4 s_rec[BLOCK / 32][2][REC_F4][32];  // per warp: double-buffered staging
+    __shared__ unsigned char s_list[BLOCK / 32][2][32];  // their places among the 32
     if (header[H_FLAGS] != 0) return;
     const int tile = blockIdx.x;
     const int tx = tile % gx, ty = tile / gx;
@@ -491,44 +493,50 @@ forward_kernel(int W, int H, int gx, const int* __restrict__ tile_start, const i
     const float pxf = (float)pxi, pyf = (float)pyi;
     bool done = !inside;
     const int s0 = tile_start[tile], n = tile_start[tile + 1] - s0;
-    const int rounds = (n + BLOCK - 1) / BLOCK;
-    int todo = n;
     float T = 1.0f;
     uint32_t last_contributor = 0;
     float C[3] = {0.f, 0.f, 0.f};
     float N[3] = {0.f, 0.f, 0.f};
     float D = 0.f, M1 = 0.f, M2 = 0.f, distortion = 0.f, median_depth = 0.f, median_contributor = -1.f;
     const float mscale = FAR_N / (FAR_N - NEAR_N);
-    // round i's records go to buffer i & 1; the copies of round i + 1 are issued once every
-    // thread has passed round i's barrier (so nobody still reads that buffer from round i - 1)
-    // and run while round i is shaded
-    auto stage = [&](int i) {
-        const int prog = i * BLOCK + threadIdx.x;
-        if (prog < n) {
-            const float4* r = rec + (int64_t)REC_F4 * sorted_gid[s0 + prog];
+    const unsigned FULL = 0xffffffffu;
+    auto load_gid = [&](int c) {
+        const int k = 32 * c + lane;
+        return k < n ? sorted_gid[s0 + k] : -1;
+    };
+    auto load_box = [&](int gid) {
+        return gid >= 0 ? reinterpret_cast<const uint2*>(rec + (int64_t)REC_F4 * gid + 4)[1] : make_uint2(0u, 0u);
+    };
+    // the kept ones of 32 surfels into buffer b; returns their number
+    auto stage = [&](int gid, uint2 box, int b) {
+        const bool mine = gid >= 0 && reaches(box.x, box.y, bx, by, BLK_W, BLK_H);
+        const unsigned bits = __ballot_sync(FULL, mine);
+        if (mine) {
+            const int at = __popc(bits & ((1u << lane) - 1u));
+            const float4* r = rec + (int64_t)REC_F4 * gid;
 #pragma unroll
-            for (int f = 0; f < REC_F4; ++f) cp_async16(&s_rec[i & 1][f][threadIdx.x], r + f);
+            for (int f = 0; f < REC_F4; ++f) cp_async16(&s_rec[warp][b][f][at], r + f);
+            s_list[warp][b][at] = (unsigned char)lane;
         }
         cp_async_commit();
+        return __popc(bits);
     };
-    if (rounds > 0) stage(0);
-    for (int i = 0; i < rounds; ++i, todo -= BLOCK) {
-        cp_async_wait_all();  // this thread's copies of round i have landed
-        if (__syncthreads_count(done) == BLOCK) break;  // ... and everyone's; no copy is in flight
-        if (i + 1 < rounds) stage(i + 1);
-        if (__all_sync(0xffffffffu, done)) continue;
-        const float4(*sr)[BLOCK] = s_rec[i & 1];
-        const int nb = min(BLOCK, todo);
-        int nl = 0;
-        for (int jc = 0; jc < nb; jc += 32) {
-            const int jl = jc + lane;
-            const bool mine = jl < nb && reaches(__float_as_uint(sr[4][jl].z), __float_as_uint(sr[4][jl].w), bx, by,
-                                                 BLK_W, BLK_H);
-            const unsigned bits = __ballot_sync(0xffffffffu, mine);
-            if (mine) s_list[warp][nl + __popc(bits & ((1u << lane) - 1u))] = (unsigned char)jl;
-            nl += __popc(bits);
-        }
-        __syncwarp();
+    // chunk c is composited while the records of chunk c + 1 are copied, the boxes of chunk c + 2 and the
+    // indices of chunk c + 3 are read
+    const int chunks = __all_sync(FULL, done) ? 0 : (n + 31) / 32;
+    int g1 = load_gid(0), g2 = load_gid(1), g3 = load_gid(2);
+    uint2 b1 = load_box(g1), b2 = load_box(g2);
+    int nl_next = stage(g1, b1, 0);
+    for (int c = 0; c < chunks; ++c) {
+        const int nl = nl_next;
+        nl_next = stage(g2, b2, (c + 1) & 1);
+        g2 = g3;
+        b2 = load_box(g3);
+        g3 = load_gid(c + 3);
+        asm volatile("cp.async.wait_group 1;\n" ::: "memory");  // this lane's copies of chunk c have landed
+        __syncwarp();                                           // ... and every lane's
+        const float4(*sr)[32] = s_rec[warp][c & 1];
+        const unsigned char* list = s_list[warp][c & 1];
         // alpha of surfel j at this pixel, 0 when the pair is skipped
         auto alpha_of = [&](int j, float& depth) {
             const float4 r2 = sr[2][j];
@@ -553,7 +561,7 @@ forward_kernel(int W, int H, int gx, const int* __restrict__ tile_start, const i
             D += depth * w;
             M1 += m * w;
             M2 += m * m * w;
-            last_contributor = (uint32_t)(i * BLOCK + j + 1);
+            last_contributor = (uint32_t)(32 * c + list[j] + 1);
             if (T > 0.5) {
                 median_depth = depth;
                 median_contributor = (float)last_contributor;
@@ -570,19 +578,19 @@ forward_kernel(int W, int H, int gx, const int* __restrict__ tile_start, const i
         };
         int e = 0;
         for (; e + 2 <= nl; e += 2) {
-            const int ja = s_list[warp][e], jb = s_list[warp][e + 1];
             float da, db;
-            const float aa = alpha_of(ja, da), ab = alpha_of(jb, db);
-            composite(ja, aa, da);
-            composite(jb, ab, db);
+            const float aa = alpha_of(e, da), ab = alpha_of(e + 1, db);
+            composite(e, aa, da);
+            composite(e + 1, ab, db);
         }
         if (e < nl) {
-            const int ja = s_list[warp][e];
             float da;
-            const float aa = alpha_of(ja, da);
-            composite(ja, aa, da);
+            const float aa = alpha_of(e, da);
+            composite(e, aa, da);
         }
+        if (__all_sync(FULL, done)) break;  // (also: every lane has left buffer c & 1)
     }
+    cp_async_wait_all();
     if (inside) {
         const int64_t HW = (int64_t)H * W;
         const int64_t pix = (int64_t)W * pyi + pxi;
