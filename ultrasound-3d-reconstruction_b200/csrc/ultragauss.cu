@@ -1130,8 +1130,8 @@ __device__ __forceinline__ f32x2 tri2(f32x2 a, f32x2 b, f32x2 c, f32x2 d, f32x2 
 // clustered Gaussians 57 -> 45 us. Unrolled 1 / 2 / 8 times 2.03 / 1.90 / 1.87 ms; compiled for 3 / 5 CTAs per
 // SM 1.91 / 1.95 ms.
 constexpr int FWD_CTAS = 4, FWD_UNROLL = 4;
-template <int BATCH>
-__global__ void __launch_bounds__(TILE_PIX, FWD_CTAS)
+template <int BATCH, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, FWD_CTAS * (TILE_PIX / 32) / WARPS)
 forward_pair_kernel(int64_t T, int64_t P, const us3d_slice_frame* __restrict__ frames,
                     const int* __restrict__ tile_frame, const int* __restrict__ tile_start,
                     const int* __restrict__ sorted_gid, const blockmask_t* __restrict__ sorted_mask,
@@ -1142,15 +1142,17 @@ forward_pair_kernel(int64_t T, int64_t P, const us3d_slice_frame* __restrict__ f
     constexpr int REC = 48;  // bytes of a staged Gaussian: mean + opacity, Lambda, intensity + depth term
     __shared__ float4 s_st[3 * (BATCH + 1)];  // the last record adds nothing
     __shared__ unsigned s_blocks[BATCH];      // sub-block mask, bit 16: odd index
-    __shared__ unsigned short s_list[TILE_PIX / 32][2][BATCH];  // per half-warp: byte offsets of its Gaussians
-    __shared__ float4 s_tiny[TILE_PIX];  // per thread: the pairs the image leaves out (forward_kernel's kc, kd), rare
+    __shared__ unsigned short s_list[WARPS][2][BATCH];  // per half-warp: byte offsets of its Gaussians
+    __shared__ float4 s_tiny[32 * WARPS];  // per thread: the pairs the image leaves out (forward_kernel's kc, kd), rare
     static_assert(BATCH * REC <= 0xffff, "staged offsets must fit 16 bits");
-    const int64_t t = blockIdx.x;
+    constexpr int PARTS = TILE_PIX / 32 / WARPS;  // blocks per tile
+    const int64_t t = blockIdx.x / PARTS;
     if (t >= T || header[H_FLAGS] != 0 || tile_frame[t] < 0) return;
     const Geo geo = load_geo(frames + tile_frame[t]);
     int tx, ty;
     find_tile_coords(geo, t, tx, ty);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, half = lane >> 4;
+    const int own = threadIdx.x >> 5, warp = own + WARPS * (blockIdx.x % PARTS);
+    const int lane = threadIdx.x & 31, half = lane >> 4;
     const int px = tx * TILE + (warp & 1) * BLK_W + (lane & 7);
     const int py0 = ty * TILE + (warp >> 1) * BLK_H + ((lane >> 3) & 1), py1 = py0 + 2;
     auto pixel = [&](int py) {  // index of the block's pixel (px, py), -1 outside the frame
@@ -1201,7 +1203,7 @@ forward_pair_kernel(int64_t T, int64_t P, const us3d_slice_frame* __restrict__ f
     };
     if (threadIdx.x < 3) s_st[3 * BATCH + threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
     const float ah_floor = exp2f(chi2 * kNegHalfLog2e) * 0.99999f;  // as in forward_kernel
-    unsigned short* list = s_list[warp][half];
+    unsigned short* list = s_list[own][half];
     for (int b0 = 0; b0 < n; b0 += BATCH) {
         const int nb = min(BATCH, n - b0);
         __syncthreads();
@@ -1227,7 +1229,7 @@ forward_pair_kernel(int64_t T, int64_t P, const us3d_slice_frame* __restrict__ f
             const bool mine = (m >> (2 * warp)) & 3u, odd = m >> 16;
             const unsigned be = __ballot_sync(0xffffffffu, mine && !odd), bo = __ballot_sync(0xffffffffu, mine && odd);
             const unsigned lt = (1u << lane) - 1u;
-            if (mine) s_list[warp][odd][odd ? n_odd + __popc(bo & lt) : n_even + __popc(be & lt)] = (unsigned short)(jl * REC);
+            if (mine) s_list[own][odd][odd ? n_odd + __popc(bo & lt) : n_even + __popc(be & lt)] = (unsigned short)(jl * REC);
             n_even += __popc(be);
             n_odd += __popc(bo);
         }
@@ -1815,6 +1817,16 @@ extern "C" int us3d_ug_read_status(const void* workspace, int64_t* total, int32_
     return US3D_OK;
 }
 
+// With few tiles the longest list, on one SM, is the time of the shading kernels, and a tile is shared by several
+// blocks: in the forward each takes half of the tile's warps, in the packed backward a quarter of its list
+// in whole rounds of 256 instances. Neither changes a bit (a warp's pixels, an instance's sums are its own).
+//   one clustered 256x256 frame (255 tiles, up to 1,272 instances): forward 45 -> 36 us (42 with a quarter of
+//   the warps, 53 with one warp each), backward 50 -> 27 us (30 with two blocks, 29 with eight);
+//   a training batch (1,152 tiles, up to 2,857): forward 116 -> 99 us, backward 122 -> 75 us (88, 79).
+// Four waves of tiles balance themselves, and sharing then only costs: 5,546 tiles forward 86 / 87 us, backward
+// 174 / 205 us; 16,384 tiles 1.87 / 1.93 and 2.47 / 2.90 ms.
+static bool few_tiles(int64_t n_tiles) { return n_tiles < 4 * 4 * 148; }
+
 extern "C" int us3d_ug_forward(void* workspace, const us3d_slice_frame* frames, int32_t n_frames, int64_t n_tiles,
                                int64_t n_pixels, int64_t n_gauss, int64_t cap, const float* pixels, float chi2,
                                float beta, float bg_alpha, float bg_intensity, float* out_image, float* out_alpha,
@@ -1828,19 +1840,22 @@ extern "C" int us3d_ug_forward(void* workspace, const us3d_slice_frame* frames, 
     if (n_tiles == 0) return US3D_OK;
     cudaStream_t stream = (cudaStream_t)stream_;
     const int prof = prof_begin("ug_forward", stream);
-    auto launch = [&](auto kernel) {
-        kernel<<<(unsigned)n_tiles, TILE_PIX, 0, stream>>>(
+    auto launch = [&](auto kernel, int warps) {
+        kernel<<<(unsigned)(n_tiles * (TILE_PIX / 32 / warps)), 32 * warps, 0, stream>>>(
             n_tiles, n_pixels, frames, w.tile_frame, w.tile_start, w.sorted_gid, w.sorted_mask, w.header, w.pack,
             pixels, chi2, beta, bg_alpha, bg_intensity, out_image, out_alpha, out_depth, w.pixel_aux);
     };
     if (!window_implied(beta)) {
-        launch(forward_kernel<256>);
+        launch(forward_kernel<256>, 8);
     } else {
-        switch (g_fwd_batch.load()) {
-            case 128: launch(forward_pair_kernel<128>); break;
-            case 256: launch(forward_pair_kernel<256>); break;
-            default: launch(forward_pair_kernel<512>); break;
-        }
+        if (few_tiles(n_tiles))
+            launch(forward_pair_kernel<256, 4>, 4);
+        else
+            switch (g_fwd_batch.load()) {
+                case 128: launch(forward_pair_kernel<128, 8>, 8); break;
+                case 256: launch(forward_pair_kernel<256, 8>, 8); break;
+                default: launch(forward_pair_kernel<512, 8>, 8); break;
+            }
     }
     US3D_CHECK_LAUNCH("ug forward");
     if (out_counts) {  // the reference's per-pixel candidate counts (full binning only)
@@ -1911,14 +1926,6 @@ extern "C" int us3d_ug_frame_table(us3d_slice_frame* frame, const float* origin,
     return US3D_OK;
 }
 
-// Blocks that share a tile's list in the packed backward, whole rounds of 256 instances each (an instance's sums
-// are one thread's, so results do not depend on it). With few tiles the longest list is the kernel's time: one
-// clustered 256x256 frame (255 tiles, up to 1,272 instances) 50 -> 27 us with four blocks, a training
-// batch (1,152 tiles, up to 2,857) 122 -> 75 us; two blocks take 30 and 88 us, eight 29 and 79 us. Four
-// waves of tiles balance themselves, and the blocks without a part then only cost: 5,546 tiles
-// 174 us with one, 182 with two, 205 with four; 16,384 tiles 2.47, 2.57 and 2.90 ms.
-static int backward_parts(int64_t n_tiles) { return n_tiles < 4 * 4 * 148 ? 4 : 1; }
-
 static int ug_backward_impl(void* workspace, const us3d_slice_frame* frames, int32_t n_frames, int64_t n_tiles,
                             int64_t n_pixels, int64_t n_gauss, int64_t cap, const float* pixels,
                             const float* d_image, const float* d_alpha, const float* d_depth,
@@ -1953,7 +1960,7 @@ static int ug_backward_impl(void* workspace, const us3d_slice_frame* frames, int
         };
         const bool packed = g_bwd_variant.load() == 1;
         auto launch_packed = [&](auto kernel, int nthreads) {
-            const int parts = backward_parts(n_tiles);
+            const int parts = few_tiles(n_tiles) ? 4 : 1;
             kernel<<<(unsigned)(n_tiles * parts), nthreads, 0, stream>>>(
                 n_tiles, n_pixels, frames, w.tile_frame, w.tile_start, w.sorted_gid, w.sorted_inst, w.sorted_mask,
                 w.header, w.pack, pixels, d_image, d_alpha, d_depth, saved_alpha, w.pixel_aux, chi2, beta, bg_alpha,
