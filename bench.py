@@ -37,23 +37,22 @@ UNIT = "frames/s"
 BP, BG, BO, BD = 44, 44, 12, 12  # algorithmic bytes per Gaussian / pixel (params, grads, outputs, upstream)
 
 # Per-frame ncu figures of each stage's kernels, from one capture of a 4-frame launch of the
-# same scene (ncu --set full; profiles/ultragauss_*_4frames.md), keyed by stage and by that
-# stage's kernel variant (0 one pixel per FP32 instruction, 1 packed FP32x2 pairs):
+# same scene (profiles/current_kernels.md), keyed by stage and by that stage's kernel variant
+# (0 one pixel per FP32 instruction, 1 packed FP32x2 pairs; the forward has the packed kernel only):
 #   traffic: dram__bytes_read.sum + dram__bytes_write.sum per frame (the backward stage is the
 #            shading adjoint + the per-Gaussian reduce_kernel), scaled to the launch's frames;
 #   inst:    (smsp__inst_executed.sum per frame, per launch) -- the reduction runs once per launch;
 #   fma:     sm__pipe_fma_cycles_active share of the shading kernel.
 # A variant without a capture has no entry and reports no issue figure.
 NCU_STAGE = {
-    "ug_forward": {
-        0: dict(traffic=(52.290304e6 + 4.972288e6) / 4, inst=(466223281 / 4, 0.0), fma=0.5092),
-        1: dict(traffic=(52.252416e6 + 4.260352e6) / 4, inst=(487111780 / 4, 0.0), fma=0.5661),
+    "ug_forward": {  # one kernel, whatever the variant
+        v: dict(traffic=(52.272128e6 + 3.503872e6) / 4, inst=(304468887 / 4, 0.0), fma=0.6566) for v in (0, 1)
     },
     "ug_backward": {
-        0: dict(traffic=(100.252416e6 + 114.988544e6 + 156.020480e6 + 28.401920e6) / 4,
-                inst=(594881545 / 4, 21e6), fma=0.6857),
-        1: dict(traffic=(99.148032e6 + 114.697984e6 + 156.020480e6 + 28.401920e6) / 4,
-                inst=(377437123 / 4, 21e6), fma=0.7181),
+        0: dict(traffic=(100.244480e6 + 112.822016e6 + 156.032768e6 + 27.768320e6) / 4,
+                inst=(595110921 / 4, 21e6), fma=0.6863),
+        1: dict(traffic=(98.460416e6 + 114.056192e6 + 156.032768e6 + 27.768320e6) / 4,
+                inst=(363441209 / 4, 21e6), fma=0.7284),
     },
 }
 SM_COUNT, SCHEDULERS_PER_SM = 148, 4
@@ -358,7 +357,7 @@ def run_b200(a):
         "batched_form": "CUDA-graph replay of bin + forward + L1 gradient + backward per 16-frame batch",
         "launch_config": {"forward_batch": launch_shape[0], "backward_threads": launch_shape[1],
                           "backward_variant": ["scalar fp32", "packed fp32x2"][launch_shape[2]],
-                          "forward_variant": ["scalar fp32", "packed fp32x2"][launch_shape[3]],
+                          "forward_variant": "packed fp32x2",
                           "autotune_ms_per_step": {"/".join(map(str, k)): round(v, 3) for k, v in tuned.items()}},
         "uncaptured": {"value": round(uncaptured_value, 3), "unit": UNIT,
                        "note": "same step launched from Python with one instance-total readback; "

@@ -235,8 +235,9 @@ US3D_API int us3d_ug_frame_table(us3d_slice_frame* frame_dev, const float* origi
 
 /*
  * Launch shapes of the UltraGauss shading kernels, process-wide (read at every launch; set
- * them before capturing a CUDA graph): Gaussians staged per forward batch (128, 256 or 512)
- * and threads per backward CTA (128 or 256). Results do not depend on them. The defaults
+ * them before capturing a CUDA graph): Gaussians staged per forward batch (128, 256 or 512; calls of
+ * fewer than 2,368 tiles share a tile between blocks and stage 256) and threads per backward CTA (128 or
+ * 256). Results do not depend on them. The defaults
  * (512, 256) are the fastest measured on the headline scene; us3d_b200.batch.autotune_launch
  * times every pair on a caller's workload and keeps the fastest. No counterpart in the
  * reference (its kernels have fixed launch shapes).
@@ -248,17 +249,13 @@ US3D_API int us3d_ug_get_launch_config(int32_t* forward_batch, int32_t* backward
  * launch): 0 = one pixel per FP32 instruction, 1 = two pixels per packed FP32 instruction
  * (sm_100 f32x2; same pair selection, each lane rounding as the scalar instruction, sums
  * of even and odd pixels kept apart and added once per instance). Both are deterministic;
- * they differ in summation order only. Default 0. No counterpart in the reference. */
+ * they differ in summation order only. Default 1. No counterpart in the reference. */
 US3D_API int us3d_ug_set_backward_variant(int32_t variant);
 US3D_API int us3d_ug_get_backward_variant(int32_t* variant);
 
-/* Forward kernel variant of the UltraGauss shading (process-wide, read at every launch): 0 =
- * one pixel per thread and FP32 instruction, 1 = two pixels per thread and packed FP32
- * instruction (sm_100 f32x2; 128-thread blocks whose warps own 8x8 quadrants, at most 256
- * staged Gaussians per batch (a forward batch of 512 runs as 256); each lane
- * rounds as the scalar kernel, so images, alpha, depth and the saved sums are bit-identical).
- * The windowed case (diag_beta < 1e-10) always uses variant 0. Default 0. No counterpart in
- * the reference. */
+/* Forward kernel variant of the UltraGauss shading (process-wide): 0 and 1 are accepted and kept, and
+ * both run the one kernel there is (two pixels per thread in packed FP32; one pixel per thread in the
+ * windowed case, diag_beta < 1e-10). Default 0. No counterpart in the reference. */
 US3D_API int us3d_ug_set_forward_variant(int32_t variant);
 US3D_API int us3d_ug_get_forward_variant(int32_t* variant);
 

@@ -781,7 +781,7 @@ static inline cudaError_t launch_tile_sort(int64_t T, int64_t n_elems, const int
         tile_sort_kernel<false><<<(unsigned)T, SORT_THREADS, 0, stream>>>(
             T, tile_start, header, count, cursor, keys, slot_inst, sorted_gid, sorted_inst, slot_mask, sorted_mask);
     cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess || n_elems <= SORT_SMEM_CAP) return e;  // a bucket holds an element once
+    if (e != cudaSuccess) return e;
     int dev = 0;
     e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -797,6 +797,7 @@ static inline cudaError_t launch_tile_sort(int64_t T, int64_t n_elems, const int
         if (e != cudaSuccess) return e;
         if (dev >= 0 && dev < 128) attr_done[dev] = true;
     }
+    if (n_elems <= SORT_SMEM_CAP) return cudaSuccess;  // a bucket holds an element once
     const bool mid = tile_sort_mid(n_elems);
     if (mid) {
         const unsigned mgrid = (unsigned)(T < SORT_MID_GRID ? T : SORT_MID_GRID);

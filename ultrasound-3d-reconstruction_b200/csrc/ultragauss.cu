@@ -11,9 +11,9 @@
 // B200 design (not the reference's): one launch sequence bins any number of frames at
 // once; instances are bucketed straight into their tile (atomic cursor) and each tile's
 // bucket is put into the reference's (depth key, Gaussian index) order by an in-shared-
-// memory bitonic sort, so no global 64-bit radix sort and no host synchronisation is
-// needed. The forward stages each tile's Gaussians in shared memory (one pixel per
-// thread, reference summation order); the backward gives each thread one (tile, Gaussian)
+// memory sort, so no global 64-bit radix sort and no host synchronisation is
+// needed. The forward stages each tile's Gaussians in shared memory (two pixels per
+// thread, Gaussians of even and odd index summed apart); the backward gives each thread one (tile, Gaussian)
 // instance, walks the tile's pixels from shared memory and accumulates that instance's
 // gradient in registers, so there are no float atomics and no warp reductions. Partials
 // are reduced per Gaussian in a fixed order (deterministic gradients).
