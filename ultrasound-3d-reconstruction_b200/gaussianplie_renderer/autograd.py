@@ -45,7 +45,7 @@ def _us_focus_params_vector(config: GaussianPlieRenderConfig, device: torch.devi
     vals[10] = max(float(config.opacity_cull_threshold), 1.0e-12)
     if device.type == "cuda" and not torch.cuda.is_current_stream_capturing():
         # from pinned memory: a copy from pageable memory waits for everything queued on the stream
-        return torch.tensor(vals, dtype=torch.float32, pin_memory=True).to(device, non_blocking=True)
+        return torch.tensor(vals, dtype=torch.float32, device="cpu", pin_memory=True).to(device, non_blocking=True)
     return torch.tensor(vals, dtype=torch.float32, device=device)
 
 
