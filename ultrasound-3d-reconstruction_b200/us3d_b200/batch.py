@@ -186,11 +186,11 @@ def set_launch_config(forward_batch: int, backward_threads: int) -> None:
 def autotune_launch(frames: UG.FrameTable, params, pixels: torch.Tensor, reps: int = 3,
                     chi2_threshold: float = 7.815, diag_beta: float = 1e-4, bg_alpha: float = 1e-6):
     """Times the batched step (slice-culled bin, forward, backward with a seeded upstream
-    gradient) on the caller's frames for every launch shape the library is built for and every
-    forward and backward variant, keeps the fastest (set_launch_config, set_backward_variant,
+    gradient) on the caller's frames for every launch shape the library is built for and both
+    backward variants, keeps the fastest (set_launch_config, set_backward_variant,
     set_forward_variant) and returns {(forward_batch, backward_threads, backward_variant,
-    forward_variant): ms per step}. Neither the shapes nor the forward variants change any
-    result; the backward variants differ in summation order only. Synchronises; run it before
+    forward_variant): ms per step} (the forward has one kernel: variant 0). The shapes change
+    no result; the backward variants differ in summation order only. Synchronises; run it before
     capturing graphs."""
     means, tril, opac, inten = params[0], params[1].contiguous(), params[2].reshape(-1), params[3].reshape(-1)
     g = torch.Generator(device=pixels.device)
