@@ -648,7 +648,10 @@ tile_sort_kernel(int64_t T, const int* __restrict__ tile_start, long long* heade
     __shared__ __align__(16) int s_idx[PACKED ? 4 : SORT_SMEM_CAP];
     __shared__ BinSortShared s_bins;
     const int64_t t = blockIdx.x;
-    if (t >= T || header[H_FLAGS] != 0) return;
+    if (t >= T) return;
+    // Another block may be raising the flag below: one thread reads the word and the block stays or leaves as a
+    // whole (a block that lost some of its threads would sort with bins that nobody cleared).
+    if (__syncthreads_or(threadIdx.x == 0 && header[H_FLAGS] != 0)) return;
     const int s0 = tile_start[t];
     const int n = tile_start[t + 1] - s0;
     if (count != nullptr && cursor[t] != count[t]) {
