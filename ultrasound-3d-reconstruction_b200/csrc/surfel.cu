@@ -310,7 +310,8 @@ __global__ void init_kernel(int64_t T, int* __restrict__ tile_count, int* __rest
 // with the cutoff c = 2 ln(255 opacity) in the place of 9) together with the filter's disc
 // {rho2d <= c}, in double precision and half a pixel wider than that, which covers the float
 // rounding of the per-pixel test (about 1e-3 pixel). Everything when the box is unbounded (the
-// splat's plane passes the camera) or not finite; nothing when the opacity is below 1/255.
+// splat's plane passes the camera) or not finite; nothing when the opacity is below 1/255. An end that
+// does not fit 16 bits stands for all pixels beyond (see reaches).
 __device__ __forceinline__ uint2 reach_box(const V3 T0, const V3 T1, const V3 T2, float px, float py, float opacity) {
     const uint2 all = make_uint2(0x7fff8000u, 0x7fff8000u);  // low half: first, high half: last
     if (opacity * 255.0f < 0.999f) return make_uint2(0x80007fffu, 0x80007fffu);
@@ -330,10 +331,11 @@ __device__ __forceinline__ uint2 reach_box(const V3 T0, const V3 T1, const V3 T2
     return make_uint2(half(a) | (half(b) << 16), half(e) | (half(f) << 16));
 }
 
-// Whether a reach box meets columns [bx, bx + w) and rows [by, by + h).
+// Whether a reach box meets columns [bx, bx + w) and rows [by, by + h). A last column or row of 32,767 is not
+// an end: frames may be wider, and such a box goes on.
 __device__ __forceinline__ bool reaches(unsigned xr, unsigned yr, int bx, int by, int w, int h) {
-    return (int)(short)(xr & 0xffffu) < bx + w && (int)(short)(xr >> 16) >= bx &&
-           (int)(short)(yr & 0xffffu) < by + h && (int)(short)(yr >> 16) >= by;
+    return (int)(short)(xr & 0xffffu) < bx + w && (int)(short)(xr >> 16) >= min(bx, 0x7fff) &&
+           (int)(short)(yr & 0xffffu) < by + h && (int)(short)(yr >> 16) >= min(by, 0x7fff);
 }
 
 // Per Gaussian: near cull, homography, dual-visible normal, AABB radius, tile rectangle,
