@@ -1,0 +1,84 @@
+"""A Gaussian with an infinite or NaN amplitude shows only where it reaches: everything else keeps every bit."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+ODD = [float("inf"), float("-inf"), float("nan")]
+
+
+def _bits(a, b):
+    return np.testing.assert_array_equal(a.cpu().numpy().view(np.int32), b.cpu().numpy().view(np.int32))
+
+
+def _slice_case(dev, centre, t, opacity):
+    """A 32x32 frame (1 mm pixels) of 300 Gaussians and one more, of precision t^4 at `centre`, in the middle of the
+    list."""
+    from us3d_b200 import ultragauss as UG
+
+    rng = np.random.default_rng(11)
+    n, k = 301, 150
+    means = np.stack([rng.uniform(-16, 16, n), rng.uniform(0, 32, n), rng.uniform(-0.5, 0.5, n)], 1)
+    tril = np.tile([0.9, 0.1, -0.1, 1.0, 0.05, 1.1], (n, 1))
+    opac, inten = rng.uniform(0.05, 0.9, n), rng.uniform(0.1, 1.0, n)
+    means[k], tril[k], opac[k] = [*centre, 0.0], [t, 0, 0, t, 0, t], opacity
+    f = lambda a: torch.as_tensor(np.ascontiguousarray(a, np.float32)).to(dev)  # noqa: E731
+    eye = torch.eye(3)
+    spec = UG.SliceSpec(32, 32, 1.0, 1.0, 0.0, 15.5, torch.zeros(3), eye[0], eye[1], eye[2])
+    y, x = torch.meshgrid(torch.arange(32.0), torch.arange(32.0), indexing="ij")
+    pix = torch.stack([x - 15.5, y, torch.zeros(32, 32)], -1).reshape(-1, 3).to(dev)
+    return [f(means), f(tril), f(opac), f(inten)], k, spec, pix
+
+
+def _slice_render(params, spec, pix, cull, dev):
+    from us3d_b200 import ultragauss as UG
+
+    b = UG.bin_gaussians(*params, UG.build_frame_table([spec], dev), 7.815, 1e-4, True,
+                         slice_cull_pixels=pix if cull else None)
+    img, alp, dep, _ = UG.forward(b, pix, 1e-6, 0.1, want_counts=False)
+    return b, img, alp, dep
+
+
+@pytest.mark.parametrize("value", ODD)
+@pytest.mark.parametrize("cull", [False, True])
+@pytest.mark.parametrize("opacity", [0.7, 3e-8])  # 3e-8: some of its pairs are left out of the image
+def test_slice_intensity_stays_where_it_reaches(value, cull, opacity, cuda_device):
+    dev = cuda_device
+    params, k, spec, pix = _slice_case(dev, (3.2, 14.3), 0.9, opacity)
+    want = _slice_render(params, spec, pix, cull, dev)[1:]
+    odd = [p.clone() for p in params]
+    odd[3][k] = value
+    got = _slice_render(odd, spec, pix, cull, dev)[1:]
+    # precision (t^2 + beta)^2 = 0.656: it reaches 3.451 mm
+    d = (pix - params[0][k]).double().norm(dim=1)
+    out = d > 3.46
+    assert 20 < int((~out).sum()) < 60
+    for a, b in zip(got, want):
+        _bits(a[out], b[out])
+    for a, b in zip(got[1:], want[1:]):  # alpha and depth don't depend on it anywhere
+        _bits(a, b)
+
+
+@pytest.mark.parametrize("value", ODD)
+@pytest.mark.parametrize("cull", [False, True])
+def test_slice_intensity_between_the_pixels(value, cull, cuda_device):
+    """It is in the lists (a rectangle is a pixel wide at least) and reaches no pixel centre."""
+    from us3d_b200 import ultragauss as UG
+
+    dev = cuda_device
+    params, k, spec, pix = _slice_case(dev, (3.0, 14.5), 4.0, 0.7)
+    odd = [p.clone() for p in params]
+    odd[3][k] = value
+    others = torch.arange(params[0].shape[0], device=dev) != k
+    up = torch.linspace(-1, 1, pix.shape[0], device=dev)
+    res = []
+    for p in (params, odd):
+        b, img, alp, dep = _slice_render(p, spec, pix, cull, dev)
+        grads = UG.backward(b, pix, up, up.flip(0), up, alp, 1e-6, 0.1)
+        res.append([img, alp, dep] + [g[others] for g in grads])
+    for a, b in zip(*res):
+        assert torch.isfinite(a).all()
+        _bits(b, a)

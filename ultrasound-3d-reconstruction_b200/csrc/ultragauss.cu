@@ -24,6 +24,8 @@
 // counts agree bit for bit.
 #include <algorithm>
 
+#include <float.h>
+
 #include <atomic>
 #include <type_traits>
 
@@ -1169,8 +1171,10 @@ forward_pair_kernel(int64_t T, int64_t P, const us3d_slice_frame* __restrict__ f
     const int n = tile_start[t + 1] - s0;
 
     f32x2 sa = dup2(0.f), sc = sa, sd = sa;
-    auto shade = [&](int off, auto tiny) {  // off: byte offset of the staged Gaussian in s_st
-        constexpr bool TINY = decltype(tiny)::value;
+    // EXACT: for a batch with a Gaussian whose alpha-hat can fall to 1e-8 inside the chi-square region, as in
+    // forward_kernel, or whose intensity or depth term is infinite or NaN
+    auto shade = [&](int off, auto exact) {  // off: byte offset of the staged Gaussian in s_st
+        constexpr bool EXACT = decltype(exact)::value;
         const float4* f = reinterpret_cast<const float4*>(reinterpret_cast<const char*>(s_st) + off);
         const float4 f0 = f[0], f1 = f[1], f2 = f[2];
         const f32x2 dx = sub2(PX, dup2(f0.x)), dy = sub2(PY, dup2(f0.y)), dz = sub2(PZ, dup2(f0.z));
@@ -1185,19 +1189,24 @@ forward_pair_kernel(int64_t T, int64_t P, const us3d_slice_frame* __restrict__ f
         float ah0, ah1;
         up2(mul2(dup2(f0.w), ex2_2(mul2(q, CE))), ah0, ah1);  // o * exp(-q/2)
         const bool pass0 = q0 <= chi2, pass1 = q1 <= chi2;
-        const bool keep0 = pass0 && (!TINY || ah0 > 1e-8f), keep1 = pass1 && (!TINY || ah1 > 1e-8f);
+        const bool keep0 = pass0 && (!EXACT || ah0 > 1e-8f), keep1 = pass1 && (!EXACT || ah1 > 1e-8f);
         const f32x2 ak = pk2(keep0 ? ah0 : 0.f, keep1 ? ah1 : 0.f);
-        const f32x2 C = dup2(f2.z), D = dup2(f2.w);
         sa = add2(sa, ak);
+        // 0 times a finite value adds nothing; in a batch with others the value is left out too
+        const f32x2 C = EXACT ? pk2(keep0 ? f2.z : 0.f, keep1 ? f2.z : 0.f) : dup2(f2.z);
+        const f32x2 D = EXACT ? pk2(keep0 ? f2.w : 0.f, keep1 ? f2.w : 0.f) : dup2(f2.w);
         sc = fma2(ak, C, sc);
         sd = fma2(ak, D, sd);
-        if (TINY && (pass0 != keep0 || pass1 != keep1)) {  // the reference's alpha-hat <= 1e-8 pairs (rare)
-            const float a0 = pass0 && !keep0 ? ah0 : 0.f, a1 = pass1 && !keep1 ? ah1 : 0.f;
+        if (EXACT && (pass0 != keep0 || pass1 != keep1)) {  // the reference's alpha-hat <= 1e-8 pairs (rare)
             float4 k = s_tiny[threadIdx.x];
-            k.x = fmaf(a0, f2.z, k.x);
-            k.y = fmaf(a1, f2.z, k.y);
-            k.z = fmaf(a0, f2.w, k.z);
-            k.w = fmaf(a1, f2.w, k.w);
+            if (pass0 && !keep0) {
+                k.x = fmaf(ah0, f2.z, k.x);
+                k.z = fmaf(ah0, f2.w, k.z);
+            }
+            if (pass1 && !keep1) {
+                k.y = fmaf(ah1, f2.z, k.y);
+                k.w = fmaf(ah1, f2.w, k.w);
+            }
             s_tiny[threadIdx.x] = k;
         }
     };
@@ -1207,12 +1216,12 @@ forward_pair_kernel(int64_t T, int64_t P, const us3d_slice_frame* __restrict__ f
     for (int b0 = 0; b0 < n; b0 += BATCH) {
         const int nb = min(BATCH, n - b0);
         __syncthreads();
-        int tiny = 0;
+        int odd = 0;
         for (int j = threadIdx.x; j < nb; j += blockDim.x) {
             const int g = sorted_gid[s0 + b0 + j];
             const float4 a = pack[3 * g], b = pack[3 * g + 1], c = pack[3 * g + 2];
-            tiny |= !(a.w * ah_floor > 1e-8f);
             const float dterm = f3_dot(f3_sub(make_float3(a.x, a.y, a.z), geo.o), geo.ele);
+            odd |= !(a.w * ah_floor > 1e-8f) || !(fabsf(c.z) <= FLT_MAX) || !(fabsf(dterm) <= FLT_MAX);
             float4 q1;
             float s12, s22;
             precision_from_raw(b.x, b.y, b.z, b.w, c.x, c.y, beta, q1, s12, s22);
@@ -1221,7 +1230,7 @@ forward_pair_kernel(int64_t T, int64_t P, const us3d_slice_frame* __restrict__ f
             s_st[3 * j + 2] = make_float4(s12, s22, c.z, dterm);
             s_blocks[j] = (unsigned)sorted_mask[s0 + b0 + j] | ((unsigned)(g & 1) << 16);
         }
-        const bool any_tiny = __syncthreads_or(tiny) != 0;
+        const bool any_odd = __syncthreads_or(odd) != 0;
         int n_even = 0, n_odd = 0;
         for (int jc = 0; jc < nb; jc += 32) {
             const int jl = jc + lane;
@@ -1237,11 +1246,11 @@ forward_pair_kernel(int64_t T, int64_t P, const us3d_slice_frame* __restrict__ f
         const int n_max = max(n_even, n_odd);
         for (int k = (half ? n_odd : n_even) + (lane & 15); k < n_max; k += 16) list[k] = (unsigned short)(BATCH * REC);
         __syncwarp();
-        auto run = [&](auto tiny_t) {
+        auto run = [&](auto exact_t) {
 #pragma unroll FWD_UNROLL
-            for (int k = 0; k < n_max; ++k) shade(list[k], tiny_t);
+            for (int k = 0; k < n_max; ++k) shade(list[k], exact_t);
         };
-        if (any_tiny)
+        if (any_odd)
             run(std::true_type{});
         else
             run(std::false_type{});
