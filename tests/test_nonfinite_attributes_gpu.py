@@ -82,3 +82,34 @@ def test_slice_intensity_between_the_pixels(value, cull, cuda_device):
     for a, b in zip(*res):
         assert torch.isfinite(a).all()
         _bits(b, a)
+
+
+def _scanline_case(G, W, H, seed):
+    from ugr_helpers import make_scene
+
+    return make_scene(G, W, H, seed, scale_range=(0.3, 0.6), width_mm=4.0)
+
+
+def _depths(scene):
+    """Depth of every Gaussian along the (parallel) scanlines, its echo radius, and the samples' depths."""
+    t = (scene["means"].astype(np.float64) - scene["origin"]) @ scene["ax"].astype(np.float64)
+    z = (scene["pixels"][0].astype(np.float64) - scene["ray_o"][0]) @ scene["ray_d"][0].astype(np.float64)
+    return t, scene["scales"].max(1).astype(np.float64) * scene["k_sigma"], z
+
+
+@pytest.mark.parametrize("value", ODD)
+@pytest.mark.parametrize("G,W,H", [(40, 3, 64), (41, 1, 97), (400, 2, 300)])
+def test_scanline_amplitude_stays_where_it_echoes(value, G, W, H, cuda_device):
+    from ugr_helpers import run_b200_ugr
+
+    scene = _scanline_case(G, W, H, 5 + G)
+    t, radius, z = _depths(scene)
+    k = int(np.argmin(np.abs(t - z[H // 2])))
+    want = run_b200_ugr(scene, cuda_device, backward=False)
+    scene["sh"][k, 0] = value
+    got = run_b200_ugr(scene, cuda_device, backward=False)
+    out = np.abs(z - t[k]) > radius[k] + 1e-3
+    assert want["counts"].min() > 10 and 0 < out.sum() < H
+    np.testing.assert_array_equal(got["image"].reshape(H, W)[out].view(np.int32),
+                                  want["image"].reshape(H, W)[out].view(np.int32))
+    assert not np.array_equal(got["image"], want["image"])

@@ -24,6 +24,9 @@
 // instance's gradient in registers, including dL/dR and dL/dSigma^-1, which are mapped to
 // quaternion and scale gradients once per instance; partials are reduced per Gaussian in a
 // fixed order (the reference issues 16 float atomics per pair).
+#include <float.h>
+#include <type_traits>
+
 #include "us3d_common.cuh"
 #include "scan.cuh"
 #include "binning.cuh"
@@ -762,7 +765,9 @@ forward_ckpt_kernel(int W, int H, const int* __restrict__ ray_start, const int* 
                 d[12] = __int_as_float(sp.x);
                 d[14] = __int_as_float(sp.y - sp.x);
             }
+            float amp = 0.f;
             if (echo) {
+                amp = r.sh.x + r.sh.y * rg.d.x + r.sh.z * rg.d.y + r.sh.w * rg.d.z;
                 float* d = echo_f + (eo >> 1) * 24 + (eo & 1);
                 d[0] = r.mu.x;
                 d[2] = r.mu.y;
@@ -773,14 +778,14 @@ forward_ckpt_kernel(int W, int H, const int* __restrict__ ray_start, const int* 
                 d[12] = kNegHalfLog2e * r.P[4];
                 d[14] = 2.0f * kNegHalfLog2e * r.P[5];
                 d[16] = kNegHalfLog2e * r.P[8];
-                d[18] = r.sh.x + r.sh.y * rg.d.x + r.sh.z * rg.d.y + r.sh.w * rg.d.z;
+                d[18] = amp;
                 d[20] = __int_as_float(sp.z);
                 d[22] = __int_as_float(sp.w - sp.z);
             }
             // an odd list's last pair: an instance with no samples and finite constants
             if (threadIdx.x < 8 && (nw & 1)) win_f[(nw >> 1) * 16 + 1 + 2 * threadIdx.x] = 0.f;
             if (threadIdx.x < 12 && (ne & 1)) echo_f[(ne >> 1) * 24 + 1 + 2 * threadIdx.x] = 0.f;
-            __syncthreads();
+            const bool odd = __syncthreads_or(!(fabsf(amp) <= FLT_MAX)) != 0;
             for (int e = warp; 2 * e < nw; e += CKPT_WARPS) {
                 const float4 c0v = s_win[e][0], c1v = s_win[e][1], c2v = s_win[e][2], c3v = s_win[e][3];
                 const f32x2 A0 = hi2(c0v), K2 = lo2(c1v), K1 = hi2(c1v), K0 = lo2(c2v), TAU = hi2(c2v);
@@ -799,21 +804,30 @@ forward_ckpt_kernel(int W, int H, const int* __restrict__ ray_start, const int* 
                 const bool in1 = (unsigned)(y - __float_as_int(c3v.y)) < (unsigned)__float_as_int(c3v.w);
                 trans = mul2(trans, pk2(in0 ? a : 1.f, in1 ? b : 1.f));
             }
-            for (int e = warp; 2 * e < ne; e += CKPT_WARPS) {
-                const float4 c0v = s_echo[e][0], c1v = s_echo[e][1], c2v = s_echo[e][2], c3v = s_echo[e][3],
-                             c4v = s_echo[e][4], c5v = s_echo[e][5];
-                const f32x2 DX = sub2(PX, lo2(c0v)), DY = sub2(PY, hi2(c0v)), DZ = sub2(PZ, lo2(c1v));
-                f32x2 Q = mul2(DX, fma2(lo2(c2v), DY, fma2(hi2(c2v), DZ, mul2(hi2(c1v), DX))));
-                Q = fma2(DY, fma2(hi2(c3v), DZ, mul2(lo2(c3v), DY)), Q);
-                Q = fma2(mul2(lo2(c4v), DZ), DZ, Q);
-                float a, b;
-                up2(ex2_2(Q), a, b);
-                const bool in0 = (unsigned)(y - __float_as_int(c5v.x)) < (unsigned)__float_as_int(c5v.z);
-                const bool in1 = (unsigned)(y - __float_as_int(c5v.y)) < (unsigned)__float_as_int(c5v.w);
-                const f32x2 WG = pk2(in0 ? a : 0.f, in1 ? b : 0.f);
-                num = fma2(hi2(c4v), WG, num);
-                den = add2(den, WG);
-            }
+            auto echoes = [&](auto exact_t) {
+                constexpr bool EXACT = decltype(exact_t)::value;
+                for (int e = warp; 2 * e < ne; e += CKPT_WARPS) {
+                    const float4 c0v = s_echo[e][0], c1v = s_echo[e][1], c2v = s_echo[e][2], c3v = s_echo[e][3],
+                                 c4v = s_echo[e][4], c5v = s_echo[e][5];
+                    const f32x2 DX = sub2(PX, lo2(c0v)), DY = sub2(PY, hi2(c0v)), DZ = sub2(PZ, lo2(c1v));
+                    f32x2 Q = mul2(DX, fma2(lo2(c2v), DY, fma2(hi2(c2v), DZ, mul2(hi2(c1v), DX))));
+                    Q = fma2(DY, fma2(hi2(c3v), DZ, mul2(lo2(c3v), DY)), Q);
+                    Q = fma2(mul2(lo2(c4v), DZ), DZ, Q);
+                    float a, b;
+                    up2(ex2_2(Q), a, b);
+                    const bool in0 = (unsigned)(y - __float_as_int(c5v.x)) < (unsigned)__float_as_int(c5v.z);
+                    const bool in1 = (unsigned)(y - __float_as_int(c5v.y)) < (unsigned)__float_as_int(c5v.w);
+                    const f32x2 WG = pk2(in0 ? a : 0.f, in1 ? b : 0.f);
+                    // 0 times a finite amplitude adds nothing; an infinite or NaN one is left out
+                    const f32x2 AMP = EXACT ? pk2(in0 ? c4v.z : 0.f, in1 ? c4v.w : 0.f) : hi2(c4v);
+                    num = fma2(AMP, WG, num);
+                    den = add2(den, WG);
+                }
+            };
+            if (odd)
+                echoes(std::true_type{});
+            else
+                echoes(std::false_type{});
         }
     }
     {
