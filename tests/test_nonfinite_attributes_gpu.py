@@ -1,4 +1,5 @@
-"""A Gaussian with an infinite or NaN amplitude shows only where it reaches: everything else keeps every bit."""
+"""A Gaussian with an infinite or NaN amplitude, or an infinite or NaN upstream gradient at one sample, shows only
+where it reaches: everything else keeps every bit."""
 
 from __future__ import annotations
 
@@ -113,3 +114,30 @@ def test_scanline_amplitude_stays_where_it_echoes(value, G, W, H, cuda_device):
     np.testing.assert_array_equal(got["image"].reshape(H, W)[out].view(np.int32),
                                   want["image"].reshape(H, W)[out].view(np.int32))
     assert not np.array_equal(got["image"], want["image"])
+
+
+@pytest.mark.parametrize("value", ODD)
+@pytest.mark.parametrize("y0", [20, 21])  # either half of a pair of samples
+def test_scanline_gradient_stays_with_its_sample(value, y0, cuda_device):
+    """Gaussians whose echo begins at the sample after the odd one, and all deeper ones, get the gradients that they
+    get when that sample's gradient is zero."""
+    from ugr_helpers import run_b200_ugr
+
+    scene = _scanline_case(300, 2, 120, 9)
+    t, radius, z = _depths(scene)
+    # every other Gaussian from just behind the sample on
+    step = z[1] - z[0]
+    deep = t - radius > z[y0] + 1e-3
+    edge = np.nonzero(deep)[0][:20]
+    shift = z[y0] + np.linspace(0.1, 0.9, edge.size) * step - (t - radius)[edge]
+    scene["means"][edge] += (shift[:, None] * scene["ax"]).astype(np.float32)
+    t, radius, _ = _depths(scene)
+    deep = t - radius > z[y0] + 1e-3
+    assert ((t - radius)[edge] < z[y0] + step).all() and deep[edge].all() and 100 < deep.sum() < 290
+    scene["grad_image"][y0] = 0.0
+    want = run_b200_ugr(scene, cuda_device)
+    scene["grad_image"][y0] = value
+    got = run_b200_ugr(scene, cuda_device)
+    for k in ("d_means", "d_scales", "d_quats", "d_attens", "d_sh"):
+        assert want[k][edge].any()
+        np.testing.assert_array_equal(got[k][deep].view(np.int32), want[k][deep].view(np.int32), err_msg=k)

@@ -73,7 +73,8 @@ struct Workspace {
     float4* b_zn;         // (z0, z1, dL/dnum 0, 1)
     float4* b_tt;         // (t0, t1, dL/dT * T 0, 1)
     float2* b_dw;         // dL/dw 0, 1
-    int* b_end;           // W: samples from here on have zero coefficients (transmittance used up)
+    int* b_end;           // W: samples from here on have zero coefficients (transmittance used up); its
+                          //    complement when a coefficient of the ray is infinite or NaN
     float* b_suffix;      // P: backward: sum over the ray's samples y' >= y of dL/dT * T
     size_t bytes;
 };
@@ -971,6 +972,7 @@ ckpt_coef_kernel(int W, int H, const long long* __restrict__ header, const int* 
     const int lane = threadIdx.x;
     double carry = 0.0;
     int end = 0;
+    bool odd = false;
     const int nchunks = (H + 31) / 32;
     for (int c = nchunks - 1; c >= 0; --c) {  // from the deepest samples up: suffix sums
         const int y = c * 32 + lane;
@@ -1005,6 +1007,7 @@ ckpt_coef_kernel(int W, int H, const long long* __restrict__ header, const int* 
             v = active ? (double)dT * (double)st.x : 0.0;
         }
         if (c_t != 0.f || c_n != 0.f || c_w != 0.f) end = max(end, y + 1);
+        odd |= !(fabsf(c_t) <= FLT_MAX && fabsf(c_n) <= FLT_MAX && fabsf(c_w) <= FLT_MAX);
         if (y < 2 * ((H + 1) / 2)) {  // an odd ray's last pair is completed with zeros
             const int64_t pr = (int64_t)x * ((H + 1) / 2) + (y >> 1);
             const int h = y & 1;
@@ -1030,7 +1033,8 @@ ckpt_coef_kernel(int W, int H, const long long* __restrict__ header, const int* 
         carry = __shfl_sync(0xffffffffu, v, 0);
     }
     end = __reduce_max_sync(0xffffffffu, end);
-    if (lane == 0) b_end[x] = end;
+    odd = __any_sync(0xffffffffu, odd);
+    if (lane == 0) b_end[x] = odd ? ~end : end;
 }
 
 // Sums over samples of one instance's backward. The integral's adjoint is linear in the canonical
@@ -1148,7 +1152,8 @@ backward_ckpt_kernel(int W, int H, const int* __restrict__ ray_start, const int*
     const int s0 = ray_start[x], n = ray_start[x + 1] - s0;
     const RayGeo rg = ray_geo(x, ray_o, ray_d, a_ele, pert);
     const int64_t row = (int64_t)x * ((H + 1) / 2);
-    const int y_end = b_end[x];
+    const bool odd_ray = b_end[x] < 0;
+    const int y_end = odd_ray ? ~b_end[x] : b_end[x];
     for (int k0 = blockIdx.y * CKPT_CHUNK; k0 < n; k0 += gridDim.y * CKPT_CHUNK) {
         const int nc = min(CKPT_CHUNK, n - k0);
         __syncthreads();  // the previous chunk's arrays are read to the end
@@ -1214,7 +1219,12 @@ backward_ckpt_kernel(int W, int H, const int* __restrict__ ray_start, const int*
             const int4 sp = live_span(full, y_end);
             const RayWindow w = ray_window(rg, r.mu, r.s, r.R, wr);
             InstanceSums acc;
-            auto sweep = [&](const float4* xy, const float4* zn, const float4* tt, const float2* dw, int first) {
+            const float amp = r.sh.x + r.sh.y * rg.d.x + r.sh.z * rg.d.y + r.sh.w * rg.d.z;
+            // EXACT: the amplitude or a coefficient of the ray is infinite or NaN, and zero times it not zero: the
+            // half of a pair outside the range and skipped samples are left out
+            auto sweep = [&](auto exact_t, const float4* xy, const float4* zn, const float4* tt, const float2* dw,
+                             int first) {
+                constexpr bool EXACT = decltype(exact_t)::value;
                 {  // window samples: dL/dF = dL/dT T / F of the factor F = tau + (1 - tau) e
                     const f32x2 TC = dup2(w.tc), A0 = dup2(w.a0), NA0 = dup2(-w.a0), K2 = dup2(w.k2), K1 = dup2(w.k1),
                                 K0 = dup2(w.k0), TAU = dup2(r.tau), OMT = dup2(1.0f - r.tau);
@@ -1235,7 +1245,8 @@ backward_ckpt_kernel(int W, int H, const int* __restrict__ ray_start, const int*
                         const f32x2 E = ex2_2(mul2(mul2(HW, NL), fma2(F1, W1, mul2(add2(F0, F2), W0))));
                         up2(fma2(OMT, E, TAU), a, b);
                         const bool in0 = 2 * i >= sp.x && a > 1e-6f, in1 = 2 * i + 1 < sp.y && b > 1e-6f;
-                        const f32x2 DF = mul2(hi2(v), pk2(in0 ? 1.0f / a : 0.f, in1 ? 1.0f / b : 0.f));
+                        const f32x2 CT = EXACT ? pk2(in0 ? v.z : 0.f, in1 ? v.w : 0.f) : hi2(v);
+                        const f32x2 DF = mul2(CT, pk2(in0 ? 1.0f / a : 0.f, in1 ? 1.0f / b : 0.f));
                         const f32x2 DE = mul2(DF, E);
                         ST = fma2(DF, sub2(ONE, E), ST);
                         const f32x2 C = mul2(DE, HW), C0 = mul2(C, W0);
@@ -1255,7 +1266,6 @@ backward_ckpt_kernel(int W, int H, const int* __restrict__ ray_start, const int*
                     const f32x2 P00 = dup2(kNegHalfLog2e * r.P[0]), P01 = dup2(2.0f * kNegHalfLog2e * r.P[1]),
                                 P02 = dup2(2.0f * kNegHalfLog2e * r.P[2]), P11 = dup2(kNegHalfLog2e * r.P[4]),
                                 P12 = dup2(2.0f * kNegHalfLog2e * r.P[5]), P22 = dup2(kNegHalfLog2e * r.P[8]);
-                    const f32x2 AMP = dup2(r.sh.x + r.sh.y * rg.d.x + r.sh.z * rg.d.y + r.sh.w * rg.d.z);
                     f32x2 SA = dup2(0.f), UX = SA, UY = SA, UZ = SA, XX = SA, XY = SA, XZ = SA, YY = SA, YZ = SA, ZZ = SA;
                     for (int i = sp.z >> 1; 2 * i < sp.w; ++i) {
                         const float4 v0 = xy[i - first], v1 = zn[i - first];
@@ -1266,10 +1276,17 @@ backward_ckpt_kernel(int W, int H, const int* __restrict__ ray_start, const int*
                         Q = fma2(mul2(P22, DZ), DZ, Q);
                         float a, b;
                         up2(ex2_2(Q), a, b);
-                        const f32x2 WG = pk2(2 * i >= sp.z ? a : 0.f, 2 * i + 1 < sp.w ? b : 0.f);
-                        const f32x2 DN = hi2(v1);
+                        const bool in0 = 2 * i >= sp.z, in1 = 2 * i + 1 < sp.w;
+                        const f32x2 WG = pk2(in0 ? a : 0.f, in1 ? b : 0.f);
+                        f32x2 DN = hi2(v1), DW = pk2(v2.x, v2.y), AMP = dup2(amp);
+                        if constexpr (EXACT) {
+                            const bool on0 = in0 && (v1.z != 0.f || v2.x != 0.f), on1 = in1 && (v1.w != 0.f || v2.y != 0.f);
+                            DN = pk2(on0 ? v1.z : 0.f, on1 ? v1.w : 0.f);
+                            DW = pk2(on0 ? v2.x : 0.f, on1 ? v2.y : 0.f);
+                            AMP = pk2(on0 ? amp : 0.f, on1 ? amp : 0.f);
+                        }
                         SA = fma2(DN, WG, SA);
-                        const f32x2 V = mul2(fma2(DN, AMP, pk2(v2.x, v2.y)), WG);
+                        const f32x2 V = mul2(fma2(DN, AMP, DW), WG);
                         const f32x2 VX = mul2(V, DX), VY = mul2(V, DY), VZ = mul2(V, DZ);
                         UX = add2(UX, VX);
                         UY = add2(UY, VY);
@@ -1287,10 +1304,12 @@ backward_ckpt_kernel(int W, int H, const int* __restrict__ ray_start, const int*
                     acc.m[3] = sum2(YY); acc.m[4] = sum2(YZ); acc.m[5] = sum2(ZZ);
                 }
             };
-            if (staged)
-                sweep(s_xy, s_zn, s_tt, s_dw, lo);
+            if (odd_ray || !(fabsf(amp) <= FLT_MAX))
+                sweep(std::true_type{}, b_xy + row, b_zn + row, b_tt + row, b_dw + row, 0);
+            else if (staged)
+                sweep(std::false_type{}, s_xy, s_zn, s_tt, s_dw, lo);
             else
-                sweep(b_xy + row, b_zn + row, b_tt + row, b_dw + row, 0);
+                sweep(std::false_type{}, b_xy + row, b_zn + row, b_tt + row, b_dw + row, 0);
             const float far_sum = y_far < H ? b_suffix[(int64_t)x * H + y_far] : 0.0f;
             instance_finish(rg, r, w, wr, far_sum, acc, quats, g, partial + (int64_t)PARTIAL_F4 * sorted_inst[k]);
         }
