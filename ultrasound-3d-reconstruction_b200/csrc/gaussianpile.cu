@@ -64,12 +64,22 @@ struct Workspace {
                         // (mu2_lat, mu2_ax, r_lat (< 0: no footprint), r_ax) (inv00, inv01, inv11, bno_const)
                         // (s2_00, s2_01, s2_11, 1 / det_norm) (mu_ele, 1 / denom_ele, dsigma_ele/dax, sigma_ele)
     StableScratch stable;    // small bucket grids (stable_bins)
-    unsigned long long* keys;  // the other ones: instances before the sort
+    unsigned long long* keys;  // the other ones, and few elements with depth keys: instances before the sort
     int* slot_inst;
     int* sorted_gid;
     int* sorted_inst;
     size_t bytes;
 };
+
+// Whether the buckets are filled in element order (stable_bins.cuh) or sorted one by one. With depth keys the fill
+// needs the radix sort's twelve launches, and a slice's lists are short: the whole forward with the sort /
+// with the fill, us: 64x64 pixels 89 / 122 for 20k Gaussians, 112 / 146 for 45k, 187 / 165 for 70k; 256x256 89 / 129,
+// 119 / 158, 142 / 181 and 198 / 226 for 120k; 512x512 141 / 174, 214 / 242, 276 / 302, 417 / 426; 720x704 206 / 224,
+// 334 / 338, 443 / 456, 715 / 674.
+constexpr int64_t FILL_MIN_KEYED = 65536;
+static inline bool fills(int64_t G, int64_t T, bool keyed) {
+    return stable_bins(G, T, keyed) && (!keyed || G >= FILL_MIN_KEYED);
+}
 
 static Workspace carve(void* base, int64_t G, int64_t T, int64_t cap) {
     Carver c(base);
@@ -86,15 +96,11 @@ static Workspace carve(void* base, int64_t G, int64_t T, int64_t cap) {
     w.bs_t = c.take<long long>((size_t)scan_num_blocks(T) + 1);
     w.cand = c.take<float4>((size_t)G * 3);
     w.bfp = c.take<float4>((size_t)G * 4);
-    if (stable_bins(G, T, false)) {
-        w.stable = stable_carve(c, G, T, true);
-        w.keys = nullptr;
-        w.slot_inst = nullptr;
-    } else {
-        w.stable = {};
-        w.keys = c.take<unsigned long long>((size_t)cap);
-        w.slot_inst = c.take<int>((size_t)cap);
-    }
+    // a workspace serves calls with depth keys (sort_by_v) and without: a small one has both
+    const bool all = fills(G, T, true);
+    w.stable = fills(G, T, false) ? stable_carve(c, G, T, all) : StableScratch{};
+    w.keys = all ? nullptr : c.take<unsigned long long>((size_t)cap);
+    w.slot_inst = all ? nullptr : c.take<int>((size_t)cap);
     w.sorted_gid = c.take<int>((size_t)cap);
     w.sorted_inst = c.take<int>((size_t)cap);
     w.bytes = align_up(c.off, 256);
@@ -1176,9 +1182,10 @@ static int gp_forward_impl(void* workspace, size_t workspace_bytes, int64_t n_ga
                                                   intensities, pose, grid_pack, focus_params, w.rects, w.dkey,
                                                   w.touched, w.tile_count, w.cand, w.bfp);
     US3D_CHECK_LAUNCH("gp preprocess");
-    US3D_CHECK_CUDA(launch_bins(n_gauss, tx, T, RectOf4{w.rects}, sort_by_v ? w.dkey : nullptr, w.touched, w.stable, w.tile_count,
-                                w.tile_start, w.tile_cursor, w.inst_offset, w.bs_g, w.bs_t, w.header, cap, w.keys, w.slot_inst,
-                                w.sorted_gid, w.sorted_inst, g_gp_sort_attr, stream));
+    const bool fill = fills(n_gauss, T, sort_by_v != 0);
+    US3D_CHECK_CUDA(launch_bins(n_gauss, tx, T, RectOf4{w.rects}, sort_by_v ? w.dkey : nullptr, w.touched, w.stable,
+                                w.tile_count, w.tile_start, w.tile_cursor, w.inst_offset, w.bs_g, w.bs_t, w.header, cap,
+                                fill ? nullptr : w.keys, w.slot_inst, w.sorted_gid, w.sorted_inst, g_gp_sort_attr, stream));
     if (status != nullptr) {
         const int rc = status->record(w.header, stream);
         if (rc != US3D_OK) return rc;
@@ -1188,7 +1195,7 @@ static int gp_forward_impl(void* workspace, size_t workspace_bytes, int64_t n_ga
                                                                  w.tile_start, w.sorted_gid, w.header, w.cand, out_image);
     US3D_CHECK_LAUNCH("gp forward");
     prof_end(prof, stream);
-    count_launches(1 + (n_gauss > 0) + bins_launches(n_gauss, T, w.keys == nullptr, sort_by_v != 0) + 1);
+    count_launches(1 + (n_gauss > 0) + bins_launches(n_gauss, T, fill, sort_by_v != 0) + 1);
     return US3D_OK;
 }
 

@@ -375,8 +375,8 @@ struct BinAttr {
 };
 
 // Bucket starts, instance offsets and every bucket's elements and instance ids in (depth key, element)
-// order (dkey NULL: element order): by the stable fill when the workspace has no instance keys (keys NULL,
-// see stable_bins), else by scattering every instance and sorting each bucket. count[] must be zero on entry.
+// order (dkey NULL: element order): by the stable fill when there are no instance keys (keys NULL, the caller's
+// choice by stable_bins), else by scattering every instance and sorting each bucket. count[] must be zero on entry.
 template <class Rect>
 static inline cudaError_t launch_bins(int64_t n, int gx, int64_t n_buckets, Rect rect, const uint32_t* dkey,
                                       const int* touched, const StableScratch& stable, int* count, int* start,
@@ -385,7 +385,7 @@ static inline cudaError_t launch_bins(int64_t n, int gx, int64_t n_buckets, Rect
                                       int* sorted_inst, BinAttr& attr, cudaStream_t stream) {
     cudaError_t e = exclusive_scan(touched, n, inst_offset, bs_g, header + H_SCAN_G, stream);
     if (e != cudaSuccess) return e;
-    const bool fill = keys == nullptr;  // the workspace was carved for the stable fill
+    const bool fill = keys == nullptr;
     const int* order = nullptr;
     if (fill) {
         if (dkey) e = launch_order(n, dkey, stable, &order, stream);
