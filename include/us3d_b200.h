@@ -170,6 +170,11 @@ US3D_API int us3d_ug_bin_ex(void* workspace, size_t workspace_bytes, const us3d_
 US3D_API int us3d_ug_read_status(const void* workspace, int64_t* total_instances, int32_t* overflow,
                         void* stream);
 
+/* us3d_ug_read_status with the number of (Gaussian, frame) pairs that survived the cull, for which a workspace has
+ * room for instance_capacity / 4 + 4096. Any of the outputs may be NULL. */
+US3D_API int us3d_ug_read_status_ex(const void* workspace, int64_t* total_instances, int64_t* total_tasks,
+                                    int32_t* overflow, void* stream);
+
 /*
  * Forward shading: per pixel, the candidates that pass the reference's lateral/axial
  * window test, then q <= chi2, alpha_hat = o*exp(-q/2) (skipped if <= 1e-8);

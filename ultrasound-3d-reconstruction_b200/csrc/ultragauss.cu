@@ -1817,13 +1817,19 @@ extern "C" int us3d_ug_bin(void* workspace, size_t workspace_bytes, const us3d_s
                           inten, chi2, beta, sort_by_depth, cap, nullptr, 0, stream);
 }
 
-extern "C" int us3d_ug_read_status(const void* workspace, int64_t* total, int32_t* overflow, void* stream_) {
+extern "C" int us3d_ug_read_status_ex(const void* workspace, int64_t* total, int64_t* n_tasks, int32_t* overflow,
+                                      void* stream_) {
     long long hdr[H_WORDS];
     int st = read_header(workspace, hdr, (cudaStream_t)stream_);
     if (st != US3D_OK) return st;
     if (total) *total = hdr[H_TOTAL];
+    if (n_tasks) *n_tasks = hdr[H_NTASK];
     if (overflow) *overflow = (int32_t)hdr[H_FLAGS];
     return US3D_OK;
+}
+
+extern "C" int us3d_ug_read_status(const void* workspace, int64_t* total, int32_t* overflow, void* stream_) {
+    return us3d_ug_read_status_ex(workspace, total, nullptr, overflow, stream_);
 }
 
 // With few tiles the longest list, on one SM, is the time of the shading kernels, and a tile is shared by several

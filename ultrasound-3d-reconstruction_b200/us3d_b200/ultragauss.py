@@ -189,18 +189,23 @@ def bin_gaussians(means: torch.Tensor, tril: torch.Tensor, opac: torch.Tensor, i
         b = UGBinning(ws, cap, -1, frames, G, float(chi2), float(beta), bool(sort_by_depth), cull)
         if not sync_check:
             return b
-        total, flags = read_status(b)
+        total, tasks, flags = _read_status(b)
         if flags & 2:
             raise RuntimeError("us3d_ug_bin: inconsistent frame table")
         b.total = total
         if not flags:
-            # a retry may have been for the (Gaussian, frame) pairs, which the total does not tell
-            _capacity_hint[key] = max(4096, int(total * 1.25) + 1024, cap if _attempt else 0)
+            _capacity_hint[key] = _next_capacity(total, tasks)
             return b
         if total > 0x7FFFFFFF:
             raise RuntimeError(f"us3d_ug_bin: {total} instances exceed the int32 index range")
         cap = int(total * 1.25) + 1024
     raise RuntimeError("us3d_ug_bin: capacity retry failed")
+
+
+def _next_capacity(total: int, tasks: int) -> int:
+    """A capacity with room to spare for that many instances and (Gaussian, frame) pairs, for which a workspace has a
+    quarter of its capacity and 4096."""
+    return max(4096, int(max(total, 4 * (tasks - 4096)) * 1.25) + 1024)
 
 
 def _bin_flags(cull: bool, logit_attributes: bool, frames: FrameTable) -> int:
@@ -238,8 +243,7 @@ def bin_forward(means: torch.Tensor, tril: torch.Tensor, opac: torch.Tensor, int
         if flags & 2:
             raise RuntimeError("us3d_ug_bin: inconsistent frame table")
         if not flags:
-            # the capacity also bounds the (Gaussian, frame) pairs: a quarter of it and 4096
-            _capacity_hint[key] = max(4096, int(max(total, 4 * (int(c_tasks.value) - 4096)) * 1.25) + 1024)
+            _capacity_hint[key] = _next_capacity(total, int(c_tasks.value))
             return (UGBinning(ws, cap, total, frames, G, float(chi2), float(beta), bool(sort_by_depth), slice_cull,
                               pixels, counts), image, alpha, depth, counts)
         if total > 0x7FFFFFFF:
@@ -248,12 +252,16 @@ def bin_forward(means: torch.Tensor, tril: torch.Tensor, opac: torch.Tensor, int
     raise RuntimeError("us3d_ug_bin: capacity retry failed")
 
 
+def _read_status(b: UGBinning):
+    total, tasks, flags = ctypes.c_int64(0), ctypes.c_int64(0), ctypes.c_int32(0)
+    _lib.check(_lib.call("us3d_ug_read_status_ex", _ptr(b.workspace), ctypes.byref(total), ctypes.byref(tasks),
+                         ctypes.byref(flags), _stream()), "us3d_ug_read_status")
+    return int(total.value), int(tasks.value), int(flags.value)
+
+
 def read_status(b: UGBinning):
-    total = ctypes.c_int64(0)
-    flags = ctypes.c_int32(0)
-    _lib.check(_lib.call("us3d_ug_read_status", _ptr(b.workspace), ctypes.byref(total), ctypes.byref(flags),
-                         _stream()), "us3d_ug_read_status")
-    return int(total.value), int(flags.value)
+    total, _, flags = _read_status(b)
+    return total, flags
 
 
 def forward(b: UGBinning, pixels: torch.Tensor, bg_alpha: float, bg_intensity: float,
