@@ -503,6 +503,11 @@ __device__ __forceinline__ int first_sample(const float* __restrict__ t, int H, 
 // digits that og + dg t loses when both terms are tens of canonical units.
 constexpr float kNegHalfLog2e = -0.72134752044448170f;  // -log2(e) / 2
 constexpr float kNegLog2e = -1.4426950408889634f;
+// -log2(e) times the quadrature weights 5/9 and 8/9, rounded once: the product of the rounded factors is a unit in
+// the last place off for 5/9, and all transmission factors of a ray then lean the same way. Relative L2
+// error against 64 bits, mean of 32 frames of 3k-200k Gaussians: image 2.92e-6 -> 2.66e-6, gradients 2.93e-6
+// to 3.06e-6 -> 2.68e-6 to 2.82e-6.
+constexpr float kNegLog2eOuter = -0.80149724493831300f, kNegLog2eMiddle = -1.2823955919013008f;
 
 struct RayWindow {
     float3 diff, is, xc, dg;  // ro - mu, 1/s, canonical closest point, canonical direction
@@ -697,7 +702,7 @@ forward_ckpt_kernel(int W, int H, const int* __restrict__ ray_start, const int* 
     const f32x2 PX = dup2(pp[0]), PY = dup2(pp[1]), PZ = dup2(pp[2]);
     const f32x2 T2 = dup2(t_pix[(int64_t)x * H + y]);
     const f32x2 HALF = dup2(0.5f), NODE = dup2(0.7745966692f), NNODE = dup2(-0.7745966692f);
-    const f32x2 W0 = dup2(kNegLog2e * 0.5555555556f), W1 = dup2(kNegLog2e * 0.8888888889f), ONE = dup2(1.0f);
+    const f32x2 W0 = dup2(kNegLog2eOuter), W1 = dup2(kNegLog2eMiddle), ONE = dup2(1.0f);
     f32x2 trans = ONE, num = dup2(0.f), den = dup2(0.f);
     float* win_f = reinterpret_cast<float*>(s_win);
     float* echo_f = reinterpret_cast<float*>(s_echo);
