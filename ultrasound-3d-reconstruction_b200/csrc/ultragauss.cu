@@ -62,7 +62,7 @@ constexpr int BWD_CHUNK = 1024;      // instances regrouped per backward pass
 
 struct Workspace {
     long long* header;
-    float4* pack;            // G x 3 float4: (m.xyz, o) (t0..t3) (t4, t5, c, 0)
+    float4* pack;            // G x 3 float4: (m.xyz, o) (t0..t3) (t4, t5, c, frames it survives in as bits)
     int* gtasks;             // G: frames in which the Gaussian survives the cull (tasks)
     int* task_offset;        // G + 1: exclusive scan of gtasks
     long long* bs_g;         // scan block sums over G
@@ -77,9 +77,9 @@ struct Workspace {
     int* tile_start;         // T + 1
     int* tile_cursor;        // T
     long long* bs_t;         // scan block sums over T
-    int* tile_frame;
-    float* tile_dev;     // per tile: largest distance of a pixel from its frame's grid (slice cull)
-    unsigned* frame_dev; // at a frame's first tile: the largest deviation of its tiles (float bits)         // T
+    int* tile_frame;         // T
+    unsigned* frame_dev;     // T; at a frame's first tile: the largest distance of its pixels from its grid (float
+                             //    bits; slice cull)
     unsigned long long* keys;  // cap: (depth_key << 32) | g, sorted in place per tile
     int* slot_inst;          // cap: instance index of each bucket slot (unsorted)
     int* sorted_gid;         // cap
@@ -112,7 +112,6 @@ static Workspace carve(void* base, int64_t G, int64_t T, int64_t P, int64_t cap,
     w.tile_cursor = c.take<int>((size_t)T);
     w.bs_t = c.take<long long>((size_t)scan_num_blocks(T) + 1);
     w.tile_frame = c.take<int>((size_t)T);
-    w.tile_dev = c.take<float>((size_t)T);
     w.frame_dev = c.take<unsigned>((size_t)T);
     w.keys = c.take<unsigned long long>((size_t)cap);
     w.slot_inst = c.take<int>((size_t)cap);
@@ -281,7 +280,7 @@ __device__ __forceinline__ void precision_from_raw(float t0, float t1, float t2,
 // P(x, y) = o + (x - col_offset) dlat lat + (near + y dax) ax the quadratic is a 2D convex
 // quadratic in pixel coordinates; its minimum over the tile's pixel-centre rectangle is
 // found exactly (in double precision) and compared with chi2 plus a margin that bounds the
-// distance of the real pixels from the grid (`tile_dev`) and the float rounding of the
+// distance of the real pixels from the grid (`frame_dev`) and the float rounding of the
 // per-pixel test. A pixel that passes the chi-square test therefore always finds the
 // Gaussian in its tile list, in the same relative order: images are unchanged and the
 // dropped instances would have contributed nothing. Only the window-test counts (and the
@@ -397,17 +396,13 @@ __device__ __forceinline__ bool ellipse_row_range(const SliceEllipse& E, double 
     return true;
 }
 
-// Largest distance of a tile's pixels from its frame's grid (double precision grid).
+// Largest distance of a frame's pixels from its grid (double precision grid), tile by tile.
 __global__ void __launch_bounds__(TILE_PIX)
 tile_dev_kernel(int64_t T, int64_t P, const us3d_slice_frame* __restrict__ frames, const int* __restrict__ tile_frame,
-                const float* __restrict__ pixels, float* __restrict__ tile_dev, unsigned* __restrict__ frame_dev) {
+                const float* __restrict__ pixels, unsigned* __restrict__ frame_dev) {
     __shared__ unsigned s_max;
     const int64_t t = blockIdx.x;
-    if (t >= T) return;
-    if (tile_frame[t] < 0) {
-        if (threadIdx.x == 0) tile_dev[t] = 0.f;
-        return;
-    }
+    if (t >= T || tile_frame[t] < 0) return;
     const Geo F = load_geo(frames + tile_frame[t]);
     const int lt = (int)(t - F.tile_off);
     const int tx = lt % F.tx, ty = lt / F.tx;
@@ -428,10 +423,7 @@ tile_dev_kernel(int64_t T, int64_t P, const us3d_slice_frame* __restrict__ frame
         atomicMax(&s_max, __float_as_uint(e));
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        tile_dev[t] = __uint_as_float(s_max);
-        atomicMax(frame_dev + F.tile_off, s_max);
-    }
+    if (threadIdx.x == 0) atomicMax(frame_dev + F.tile_off, s_max);
 }
 
 // Binning in three steps that keep every thread busy: (1) per Gaussian, the reference's
@@ -1770,7 +1762,7 @@ int us3d::ug::bin_with_task_capacity(void* workspace, size_t workspace_bytes, co
     US3D_CHECK_LAUNCH("ug setup");
     if (slice_cull && n_tiles > 0)
         tile_dev_kernel<<<(unsigned)n_tiles, TILE_PIX, 0, stream>>>(n_tiles, n_pixels, frames, w.tile_frame, pixels,
-                                                                    w.tile_dev, w.frame_dev);
+                                                                    w.frame_dev);
     const unsigned* tdev = slice_cull ? w.frame_dev : nullptr;
     const int gb = (int)((n_gauss + 255) / 256);
     const unsigned tb = (unsigned)std::min<int64_t>((tc + 127) / 128, 148 * 16);
