@@ -13,10 +13,10 @@
 //
 // B200 design: each Gaussian's footprint is computed once per call and cached (the reference
 // recomputes it in the mapper, once per tile in the forward and again per tile in the
-// backward); instances are bucketed per tile and ordered in shared memory like the UltraGauss
-// path; the backward writes one partial record per (tile, Gaussian) instance and a
-// per-Gaussian pass reduces them in a fixed order (the reference adds ~35 float atomics per
-// instance into a per-Gaussian workspace) before the finalize.
+// backward); tiles are filled in Gaussian order on small grids, else scattered and sorted like the UltraGauss
+// path (see fills); the backward writes one record of nine moments per (tile, Gaussian) instance, from which the
+// per-Gaussian finalize forms the gradient terms in instance order (the reference adds ~35 float
+// atomics per instance into a per-Gaussian workspace).
 //
 // Arithmetic that decides integer outputs or that the forward image depends on (footprint,
 // rectangles, window test, weights) uses the reference's operations in the reference's

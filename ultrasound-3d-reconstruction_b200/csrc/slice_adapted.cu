@@ -8,9 +8,9 @@
 //   :354-515   per-pixel forward over the tile list, per-pair backward
 //
 // B200 design: the reference switches between per-Gaussian atomic scatter (fewer than
-// 16384 Gaussians) and tile binning; here every size is tile-binned through the shared
-// bucket + per-tile sort, the forward stages each tile's Gaussians in shared memory (one
-// pixel per thread, tile-list order = Gaussian order), and the backward gives each thread
+// 16384 Gaussians) and tile binning; here every size is tile-binned (tiles filled in Gaussian order
+// on grids of up to 2,048 tiles, scattered and sorted per tile on larger ones), the forward stages each tile's
+// Gaussians in shared memory (one pixel per thread, tile-list order = Gaussian order), and the backward gives each thread
 // one (tile, Gaussian) instance whose bounding box it sweeps inside the tile, accumulating
 // the ten parameter gradients in registers; per-instance partials are reduced per Gaussian
 // in a fixed order (the reference issues up to 10 float atomics per pair).

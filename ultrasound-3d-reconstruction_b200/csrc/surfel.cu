@@ -12,15 +12,17 @@
 //   cuda_rasterizer/backward.cu:103-404    back-to-front replay and per-pair gradients
 //   cuda_rasterizer/backward.cu:406-602    homography / AABB / rotation / SH gradients
 //
-// B200 design. Binning puts every (tile, Gaussian) instance into its tile's bucket and orders
-// each bucket in shared memory by (depth bits, Gaussian index), the order the reference's
-// stable radix sort produces. The forward stages 256 80-byte records per batch and gives
-// each thread one pixel. The backward keeps the reference's per-pixel back-to-front replay
-// (its recurrences need it) but replaces the per-pair float atomics by a fixed-order
-// reduction: per staged Gaussian, each warp reduces its 32 pixels' 18 gradient terms with a
-// transposed butterfly (27 shuffles), the 8 warp sums are added in warp order into one
-// per-instance partial, and one thread per Gaussian sums its instances in order and runs
-// the preprocess backward in the same kernel. Results are deterministic.
+// B200 design. Binning gives every tile its (tile, Gaussian) instances in (depth bits, Gaussian index) order,
+// the order the reference's stable radix sort produces: on small grids by ordering the Gaussians once
+// and filling the tiles in that order, else by sorting each tile's bucket in shared memory. The
+// forward gives each thread one pixel; every warp keeps, of 32 surfels of the list at a time, those whose
+// exact reach box meets its 8x4 pixels and stages their 80-byte records itself, independently of
+// the other warps. The backward keeps the reference's per-pixel back-to-front replay (its recurrences
+// need it) on the same kind of lists, but replaces the per-pair float atomics by a fixed-order
+// reduction: two surfels at a time, each warp reduces its 32 pixels' 18 gradient terms of both with
+// one transposed butterfly (37 shuffles), the sums of the warps that replayed a surfel are added in
+// warp order into one per-instance partial, and per Gaussian the instances are summed in order and the
+// preprocess backward follows. Results are deterministic.
 //
 // Matrix products are evaluated with the summation order of the GLM operators the
 // reference uses (column-major, k ascending, zero entries included), so that pixel

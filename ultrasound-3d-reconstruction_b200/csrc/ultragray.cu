@@ -14,9 +14,11 @@
 // call sites imply (normalised (w,x,y,z) quaternion, row-major R with the Gaussian's axes
 // as columns).
 //
-// B200 design: rays are binned like tiles (bucket per ray + in-shared-memory ordering by
-// (depth key, Gaussian)); every Gaussian's rotation, precision and sigmoid attenuation are
-// computed once per call into a 112-byte record; the forward stages a ray's records in
+// B200 design: rays are binned like tiles (a list per ray in (depth key, Gaussian) order); every
+// Gaussian's rotation, precision and sigmoid attenuation are
+// computed once per call into a 112-byte record. Rays whose sample depths never decrease, with a
+// quadrature window, are rendered from transmittance checkpoints (see far_prep_kernel and
+// forward_ckpt_kernel). The others sample by sample: the forward stages a ray's records in
 // shared memory and gives each thread one pixel of the ray, in list order (the reference's
 // multiplication order); it saves (T, sum I w, sum w) per pixel so the backward needs no
 // recompute pass. The backward gives each thread one (ray, Gaussian) instance, sweeps the
