@@ -38,21 +38,20 @@ BP, BG, BO, BD = 44, 44, 12, 12  # algorithmic bytes per Gaussian / pixel (param
 
 # Per-frame ncu figures of each stage's kernels, from one capture of a 4-frame launch of the
 # same scene (profiles/current_kernels.md), keyed by stage and by that stage's kernel variant
-# (0 one pixel per FP32 instruction, 1 packed FP32x2 pairs; the forward has the packed kernel only):
+# (0 one pixel per FP32 instruction, 1 packed FP32x2 pairs; the forward has one kernel, packed, under 0):
 #   traffic: dram__bytes_read.sum + dram__bytes_write.sum per frame (the backward stage is the
 #            shading adjoint + the per-Gaussian reduce_kernel), scaled to the launch's frames;
-#   inst:    (smsp__inst_executed.sum per frame, per launch) -- the reduction runs once per launch;
+#   inst:    (smsp__inst_executed.sum per frame, per launch); the reduction has a part per Gaussian, once per
+#            launch, and one per instance, which grows with the frames: 31.15M for 4 frames, 42.87M for 8;
 #   fma:     sm__pipe_fma_cycles_active share of the shading kernel.
 # A variant without a capture has no entry and reports no issue figure.
 NCU_STAGE = {
-    "ug_forward": {  # one kernel, whatever the variant
-        v: dict(traffic=(52.272128e6 + 3.503872e6) / 4, inst=(304468887 / 4, 0.0), fma=0.6566) for v in (0, 1)
-    },
+    "ug_forward": {0: dict(traffic=(52.272128e6 + 3.503872e6) / 4, inst=(304468887 / 4, 0.0), fma=0.6566)},
     "ug_backward": {
         0: dict(traffic=(100.244480e6 + 112.822016e6 + 156.032768e6 + 27.768320e6) / 4,
-                inst=(595110921 / 4, 21e6), fma=0.6863),
+                inst=(595110921 / 4 + 2.93e6, 19.44e6), fma=0.6863),
         1: dict(traffic=(98.460416e6 + 114.056192e6 + 156.032768e6 + 27.768320e6) / 4,
-                inst=(363441209 / 4, 21e6), fma=0.7284),
+                inst=(363441209 / 4 + 2.93e6, 19.44e6), fma=0.7284),
     },
 }
 SM_COUNT, SCHEDULERS_PER_SM = 148, 4
@@ -330,7 +329,7 @@ def run_b200(a):
     peaks = json.load(open(ROOT / "MEASURED_PEAKS.json")) if (ROOT / "MEASURED_PEAKS.json").exists() else {}
     peak = float(peaks.get("hbm_gbs", 6650.0))
     achieved = alg / (stage_avg_ms / 1e3) / 1e9
-    variants = {"ug_forward": launch_shape[3], "ug_backward": launch_shape[2]}
+    variants = {"ug_forward": 0, "ug_backward": launch_shape[2]}
     traffic = NCU_STAGE.get(dominant, {}).get(variants.get(dominant), {}).get("traffic")
     roofline = {"bound": "hbm", "kernel": dominant, "achieved": round(achieved, 2), "peak": peak, "unit": "GB/s",
                 "frac": round(achieved / peak, 4), "traffic": int(traffic * F) if traffic else None,
@@ -391,12 +390,12 @@ def issue_roofline(stage_ms, frames_per_launch, clocks, variants):
     """The bound the shading kernels actually meet: warp instructions issued per second
     against the GPU's issue ceiling (148 SMs x 4 schedulers x 1 warp instruction per clock at
     the median SM clock sampled during the timed region), per stage, from the instruction
-    counts of the committed ncu capture of the stage's kernel variant scaled to the launch's
+    counts of the committed ncu captures of the stage's kernel variant scaled to the launch's
     frames and this run's CUDA-event stage times."""
     mhz = clocks.get("sm_mhz") or clocks.get("sm_max_mhz") or 1965.0
     ceiling = SM_COUNT * SCHEDULERS_PER_SM * mhz * 1e6  # warp instructions / s
     out = {"bound": "instruction issue", "unit": "warp inst/s", "sm_mhz": mhz, "peak": ceiling,
-           "source": "smsp__inst_executed.sum per frame of a 4-frame ncu capture (profiles/) x frames per launch "
+           "source": "smsp__inst_executed.sum per frame of 4- and 8-frame ncu captures (profiles/) x frames per launch "
                      "/ CUDA-event stage time; peak = 148 SMs x 4 schedulers x median SM clock"}
     for stage, by_variant in NCU_STAGE.items():
         ms = stage_ms.get(stage)

@@ -38,6 +38,7 @@ constexpr int STABLE_THREADS = 512;
 // Elements with a depth key take this path from STABLE_MIN_KEYED on: below, the radix sort's twelve
 // launches cost more than sorting short buckets (20k surfels on 256 buckets 70 us against 44 us, 60k 60 us
 // against 133 us; scanlines of 40k Gaussians with short lists 50 against 45 us, with long ones 50 against 123 us).
+// GaussianPile draws its own line further up.
 constexpr int64_t STABLE_MIN_KEYED = 32768;
 static inline bool stable_bins(int64_t n, int64_t n_buckets, bool keyed) {
     return n_buckets <= STABLE_MAX_BUCKETS && (!keyed || n >= STABLE_MIN_KEYED);
